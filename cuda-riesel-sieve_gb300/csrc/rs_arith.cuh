@@ -116,13 +116,11 @@ __device__ __forceinline__ uint64_t shoup_mul(uint64_t x, uint64_t w, uint64_t w
 }
 
 // Shoup's product for a 32-bit x: c*w mod p with wq = floor(w * 2^64 / p).
-// The bound is the one above (x < 2^64), and the quotient estimate
-// floor(c * wq / 2^64) <= c*w/p < c fits 32 bits, so the high product is two
-// 32x32 multiply-adds and q*p one: about ten instructions against sixteen.
+// The high word h = floor(w * 2^32 / p) of wq is enough: q = floor(c*h / 2^32)
+// exceeds c*w/p - c/2^32 - 1, so r = c*w - q*p lies in [0, 2p) for every
+// c < 2^32, and the quotient is one 32x32 high product.
 __device__ __forceinline__ uint64_t shoup_mul32(uint32_t c, uint64_t w, uint64_t wq, uint64_t p) {
-  const uint64_t t = (uint64_t)c * (uint32_t)wq;
-  const uint64_t u = (uint64_t)c * (uint32_t)(wq >> 32) + (t >> 32);
-  const uint32_t q = (uint32_t)(u >> 32);
+  const uint32_t q = __umulhi(c, (uint32_t)(wq >> 32));
   const uint64_t r = (uint64_t)c * w + (uint64_t)q * (0 - p);
   const uint64_t s = r - p;
   return (int64_t)s < 0 ? r : s;

@@ -344,8 +344,8 @@ static void normalise(Seqs &s) {
 
 struct Plan {
   uint32_t Q = 0, nrows = 0, X = 0, x_lo = 0, x_hi = 0, m = 0, T = 0;
-  uint32_t tlanes = 0, rows_per_it = 0, steps_per_lane = 0, table_log2 = 0, jbits = 0, bucket_log2 = 0;
-  uint32_t nbuckets = 0;  // fast-path buckets (1 << bucket_log2 for the warp kernel; a multiple of 64 for a CTA)
+  uint32_t tlanes = 0, rows_per_it = 0, steps_per_lane = 0, table_log2 = 0, jbits = 0;
+  uint32_t nbuckets = 0;  // table size in units of eight 16-bit slots (CTA kernel: a multiple of 64)
   bool cta = false;  // one CTA of kCtaWarps warps per prime (bsgs_cta_kernel)
   uint32_t nmin = 0, nmax = 0, ncand = 0, words_per_row = 0;
   int64_t e0 = 0;
@@ -387,7 +387,7 @@ struct PlanChoice {
   uint32_t Q = 0, T = 0, m = 0;
   bool cta = false;
   double cost = 0;
-  uint32_t nb = 0;  // fast-path buckets
+  uint32_t nb = 0;  // table size, as Plan::nbuckets
 };
 
 // Plan a job.  With `force`, take exactly that choice (it must be feasible);
@@ -441,7 +441,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
       for (uint32_t e = 1; e < Q && c < (1ull << 32); e++) c *= s.base;
       ints_q = c < (1ull << 32);
     }
-    auto consider = [&](bool cta, uint64_t T, uint64_t m, uint32_t blog, uint32_t nb, uint32_t slog, double cost) {
+    auto consider = [&](bool cta, uint64_t T, uint64_t m, uint32_t nb, uint32_t slog, double cost) {
       if (ranked) ranked->push_back(PlanChoice{Q, (uint32_t)T, (uint32_t)m, cta, cost, nb});
       if (force) {
         if (force->Q != Q || force->T != T || force->m != m || force->cta != cta || force->nb != nb) return;
@@ -458,7 +458,6 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
         pl.rows_per_it = 32 / pl.tlanes;
         pl.steps_per_lane = (uint32_t)std::max<uint64_t>(1, T / 32);
         pl.table_log2 = slog;
-        pl.bucket_log2 = blog;
         pl.nbuckets = nb;
         pl.cta = cta;
         pl.cost = cost;
@@ -485,7 +484,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
           const double nb = (double)(1u << blog);
           // the kernel's shared memory per warp and per CTA (128-byte granules, 1 KB reserved)
           const uint64_t stage = kElV + ((rows + 1) & ~1u);
-          const uint64_t wsm = align_up((20u << blog) + 16 * (stage * 8 <= 2048 ? stage : kElV) + 16 * kMatchCap + 16, 16);
+          const uint64_t wsm = align_up((20u << blog) + 16 * (stage * 8 <= 2048 ? stage : kElV) + 256, 16);
           const double cta_bytes = (double)align_up(4 * wsm, 128) + 1024.0;
           const double warps = std::min(kFullWarps, 4.0 * std::floor(kSmemPerSm / cta_bytes));
           const double fp = ER * (double)T * ((double)m / nb) / 65536.0;  // expected tag matches per prime
@@ -494,7 +493,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
             const double cost = (std::ceil((double)m / 32.0) + kGiantWeight * std::ceil(ER / rpi) * spl +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
                                 std::sqrt(kFullWarps / warps);
-            consider(false, T, m, blog, 1u << blog, slog, cost);
+            consider(false, T, m, 1u << blog, slog, cost);
           }
         }
       }
@@ -524,7 +523,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
             const double cost = ((double)m / 32.0 + kGiantWeight * kCtaWarps * std::ceil(ER / kCtaWarps) * spl +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
                                 std::sqrt(kFullWarps / kCtaWarps) * kCtaStepCost;
-            consider(true, T, m, blog, nbk, slog, cost);
+            consider(true, T, m, nbk, slog, cost);
           }
         }
       }
@@ -658,6 +657,7 @@ struct Part {
   size_t dev_bytes = 0;   // their device size (with the character tables built on the device)
   HitBufs hb{};
   void *d_hits = nullptr;
+  uint32_t ctas = 0;  // warp kernel: CTAs per SM the shared memory is sized for
   int bsgs_grid = 0;
   int exact_grid = 0;
   // Quadratic-character tables (rs_options.char_tables): the odd parts k' with
@@ -839,6 +839,23 @@ static int build_char_tables(rs_job *j, Part &pt, double primes_more, bool all) 
   return RS_OK;
 }
 
+// Filter words of a warp with m baby steps, and the CTAs per SM (out) they are
+// sized for: the most CTAs that leave 1.25 words a baby step, up to 3.5 (more only
+// costs the clearing).  Fewer than 1.25 measured slower for the suspects
+// than one CTA fewer for its warps.  Just above 2048 the power of two is kept:
+// its keys have one guard bit more.
+static uint32_t warp_filter(uint32_t m, uint32_t fixed, uint32_t static_smem, uint32_t &ctas) {
+  uint32_t words = 0;
+  for (ctas = kWarpCtas;; ctas--) {
+    const uint32_t share = warp_kernel_share(ctas, static_smem);
+    words = share > fixed ? (share - fixed) / 16 * 4 : 0;
+    if (words >= 1.25 * m || ctas == 1) break;
+  }
+  words = std::min(words, std::max(64u, (7 * m / 2 + 3) & ~3u));
+  return words > 2048 && words < 2200 ? 2048 : words;
+}
+static uint32_t filter_shift(uint32_t words) { return std::max(11u, std::min(16u, 27 - ilog2_ceil(words))); }
+
 static int upload_part(rs_job *j, Part &pt) {
   const Plan &pl = pt.plan;
   const Seqs &s = pt.seqs;
@@ -968,7 +985,6 @@ static int upload_part(rs_job *j, Part &pt) {
   d.tlanes = pl.tlanes;
   d.rows_per_it = pl.rows_per_it;
   d.steps_per_lane = pl.steps_per_lane;
-  d.table_log2 = pl.bucket_log2;
   d.nbuckets = pl.nbuckets;
   d.exact_log2 = pl.table_log2;
   d.jbits = pl.jbits;
@@ -1017,10 +1033,12 @@ static int upload_part(rs_job *j, Part &pt) {
       d.ctab_smem = 1;
       d.warp_smem += ctab_bytes;
     }
-  } else  // bytes per warp: table, counts, two record stages, (V of a row mask,) match list
-    d.warp_smem = (uint32_t)align_up((20u << d.table_log2) + 16 * d.stage_elems + (d.row_mask ? 8 * kMaskRows : 0) +
-                                         kMatchCap * 16 + 16,
-                                     16);
+  } else {  // bytes per warp: the filter takes what the shared memory leaves (warp_filter)
+    const uint32_t fixed = warp_kernel_fixed(d.chain_len, d.stage_elems, d.row_mask != 0);
+    d.fwords = warp_filter(pl.m, fixed, 0, pt.ctas);
+    d.warp_smem = 4 * d.fwords + fixed;
+    d.fshift = filter_shift(d.fwords);
+  }
   d.row_r = (const uint32_t *)(b + o_rr);
   d.row_kidx = (const uint32_t *)(b + o_rk);
   d.row_c = (const uint32_t *)(b + o_rc);
@@ -1375,27 +1393,56 @@ int rs_job_destroy(rs_job *j) {
 
 static constexpr int kRetryHits = -1;
 
-// The baby-step product of a chunk [a, b] for one part (ChunkBufs::small_step).
-// The short product by the integer b^Q needs p > 2^33 and b^Q * p < 2^63 for
-// every p of the chunk; Shoup's product with a 32-bit constant needs
-// b^Q * 2^32 < p and exists only in the CTA-per-prime kernel; Shoup's full
-// product is always valid.  rs_options.baby_step may prefer a valid form over
-// the cheapest.
-static uint32_t chunk_step_form(const rs_job *j, const Part &pt, uint64_t a, uint64_t b) {
-  const uint64_t bq = pt.dev.bq_small;
-  const bool small_ok = bq != 0 && a > (1ull << 33) && (unsigned __int128)bq * b < ((unsigned __int128)1 << 63);
-  const bool high_ok = bq != 0 && pt.dev.cta_warps > 1 && (bq << 32) < a;
-  switch (j->opt.baby_step) {
-    case RS_BABY_SHOUP: return kStepShoup;
-    case RS_BABY_SHORT:
-      if (small_ok) return kStepSmall;
-      break;
-    case RS_BABY_HIGH:
-      if (high_ok) return kStepHigh;
-      break;
-    default: break;
+// Shift S of the short product by c for the primes of [a, b] (LazyShort): the
+// quotient falls short by less than 1 + k1 + R*k2 with k1 = c*2^S/a, k2 =
+// b/2^(32+S) and operands below R*p, so R = (1 + k1)/(1 - k2) bounds the
+// remainders too.  Valid for R <= 2; the best S balances k1 and k2.
+static bool short_step_valid(uint64_t c, uint64_t a, uint64_t b, uint32_t S) {
+  const double k1 = std::ldexp((double)c, (int)S) / (double)a, k2 = (double)b / std::ldexp(1.0, 32 + (int)S);
+  return c != 0 && k2 < 0.49 && 1.0 + k1 <= 1.999 * (1.0 - k2);
+}
+static bool short_step_shift(uint64_t c, uint64_t a, uint64_t b, uint32_t &S) {
+  if (c == 0) return false;
+  double best = 1e300;
+  for (uint32_t t = 0; t <= 32; t++) {
+    const double k1 = std::ldexp((double)c, (int)t) / (double)a, k2 = (double)b / std::ldexp(1.0, 32 + (int)t);
+    if (std::max(k1, k2) < best) {
+      best = std::max(k1, k2);
+      S = t;
+    }
   }
-  return small_ok ? kStepSmall : high_ok ? kStepHigh : kStepShoup;
+  return short_step_valid(c, a, b, S);
+}
+
+// The baby-step product of a chunk [a, b] for one part (ChunkBufs::small_step):
+// the short product by the integer b^Q where it is valid for every p of the
+// chunk, else Shoup's full product (always valid).  RS_BABY_HIGH is the short
+// product with shift 32, a 32-bit constant b^Q*2^64/p (CTA kernel only).
+// rs_options.baby_step may prefer a valid form over the cheapest.
+struct StepForm {
+  uint32_t form = kStepShoup, shift = 0, pair_ok = 0;
+};
+static StepForm chunk_step_form(const rs_job *j, const Part &pt, uint64_t a, uint64_t b) {
+  const uint64_t bq = pt.dev.bq_small;
+  StepForm f;
+  f.pair_ok = a > (1ull << 33) && (unsigned __int128)pt.dev.base * b < ((unsigned __int128)1 << 63) ? 1u : 0u;
+  if (pt.dev.cta_warps > 1) {
+    const bool small_ok = bq != 0 && a > (1ull << 33) && (unsigned __int128)bq * b < ((unsigned __int128)1 << 63);
+    const bool high_ok = bq != 0 && (bq << 32) < a;
+    f.form = small_ok ? kStepSmall : high_ok ? kStepHigh : kStepShoup;
+    if (j->opt.baby_step == RS_BABY_SHOUP) f.form = kStepShoup;
+    else if (j->opt.baby_step == RS_BABY_HIGH && high_ok) f.form = kStepHigh;
+    return f;
+  }
+  if (j->opt.baby_step != RS_BABY_SHOUP && short_step_shift(bq, a, b, f.shift)) f.form = kStepSmall;
+  else f.pair_ok = 0;
+  return f;
+}
+
+static void set_step(ChunkBufs &cb, const StepForm &f) {
+  cb.small_step = f.form;
+  cb.step_shift = f.shift;
+  cb.pair_ok = f.pair_ok;
 }
 
 // Chunks [a, b] of [lo, hi] (lo odd) with an expected prime count of ~0.8*C each.
@@ -1518,9 +1565,9 @@ static int sieve_range_impl(rs_job *j, uint64_t p0, uint64_t p1, rs_factor *out,
       st.launches += j->nsp > j->nsp_small ? 2 : 1;
       for (size_t q = 0; q < P && e == cudaSuccess; q++) {
         Part &pt = *j->parts[q];
-        const uint32_t form = chunk_step_form(j, pt, todo[c].a, todo[c].b);
-        forms[c * P + q] = form;
-        j->cb.small_step = form;
+        const StepForm form = chunk_step_form(j, pt, todo[c].a, todo[c].b);
+        forms[c * P + q] = form.form;
+        set_step(j->cb, form);
         if (ce) cudaEventRecord(ce[2 + 4 * q], j->st);
         e = launch_setup(pt.dev, j->cb, j->st);
         if (e == cudaSuccess) e = cudaMemsetAsync(j->cb.redo_count, 0, 4, j->st);
@@ -1819,6 +1866,12 @@ extern "C" int rs_batch_add(rs_batch *b, rs_job *job, uint64_t p0, uint64_t p1, 
   return RS_OK;
 }
 
+// Filter words an item has in a multi-job launch with this stage and warp share.
+static uint32_t batch_item_words(uint32_t warp_bytes, uint32_t stage_max, const JobDev &d) {
+  const uint32_t fixed = warp_kernel_fixed(d.chain_len, stage_max, d.row_mask != 0);
+  return warp_bytes > fixed ? (warp_bytes - fixed) / 16 * 4 : 0;
+}
+
 // Kernel variant of a warp-per-prime part: items of one multi-job launch share it.
 static uint32_t batch_variant(const JobDev &d) {
   const uint32_t rm = d.row_mask ? kRowsMask : d.row_ids_only ? kRowsIntId : d.int_rows ? kRowsIntV : kRowsV;
@@ -1842,7 +1895,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
     Part *pt;
     uint64_t lo, hi;
     std::vector<Chunk> chunks;
-    std::vector<uint32_t> forms;
+    std::vector<StepForm> forms;
     size_t count0 = 0;  // first slot of its chunks in the pinned count array
     bool own = false;   // BSGS through the job's own launch (CTA layout, or no batch kernel fits)
   };
@@ -1898,7 +1951,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
   // kBatchMaxItems runs each, and their launch shape; a group whose shape fits
   // no launch runs its jobs' own launches, as CTA-layout jobs do
   struct Group {
-    uint32_t variant, table_log2;
+    uint32_t variant, ctas;
     std::vector<size_t> runs;
     uint32_t stage_max = 0, warp_bytes = 0;
     int grid = 0;
@@ -1912,17 +1965,31 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
     }
     const uint32_t v = batch_variant(d);
     size_t g = 0;
-    for (; g < groups.size() && (groups[g].variant != v || groups[g].table_log2 != d.table_log2 ||
-                                 groups[g].runs.size() >= kBatchMaxItems);
+    const uint32_t ctas = runs[r].pt->ctas;
+    // every item of a group keeps at least 0.75 filter words a baby step beside the largest stage
+    auto fits = [&](const Group &G) {
+      const uint32_t share = warp_kernel_share(G.ctas, kBatchStaticSmem), stage = std::max(G.stage_max, d.stage_elems);
+      bool ok = 4 * batch_item_words(share, stage, d) >= 3 * d.m;
+      for (size_t x : G.runs) ok = ok && 4 * batch_item_words(share, stage, runs[x].pt->dev) >= 3 * runs[x].pt->dev.m;
+      return ok;
+    };
+    if (!fits(Group{v, ctas, {}})) {
+      runs[r].own = true;
+      continue;
+    }
+    for (; g < groups.size() && (groups[g].variant != v || groups[g].ctas != ctas ||
+                                 groups[g].runs.size() >= kBatchMaxItems || !fits(groups[g]));
          g++) {
     }
-    if (g == groups.size()) groups.push_back(Group{v, d.table_log2, {}});
+    if (g == groups.size()) groups.push_back(Group{v, ctas, {}});
     groups[g].runs.push_back(r);
     groups[g].stage_max = std::max(groups[g].stage_max, d.stage_elems);
   }
   for (size_t g = 0; g < groups.size();) {
     Group &G = groups[g];
-    G.warp_bytes = batch_warp_bytes(G.stage_max, G.table_log2, runs[G.runs[0]].pt->dev.row_mask != 0);
+    // a warp's share of the shared memory at the group's CTAs per SM; an item's
+    // filter gives way to the launch's stage and static shared memory (batch_item_words)
+    G.warp_bytes = warp_kernel_share(G.ctas, kBatchStaticSmem);
     if (batch_configure(runs[G.runs[0]].pt->dev, G.warp_bytes, B->device, &G.grid) == cudaSuccess) {
       g++;
       continue;
@@ -1943,8 +2010,9 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
         if (rd >= R.chunks.size()) continue;
         BatchItem x;
         x.J = R.pt->dev;
+        x.J.fwords = std::min(x.J.fwords, batch_item_words(groups[g].warp_bytes, groups[g].stage_max, x.J));
         x.cb = R.j->cb;
-        x.cb.small_step = R.forms[rd];
+        set_step(x.cb, R.forms[rd]);
         x.hb = R.pt->hb;
         hitems.push_back(x);
         gn[rd][g]++;
@@ -2015,7 +2083,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
                    j->cb.cap, s);
       cudaMemcpyAsync(&h_counts[R.count0 + rd], j->cb.count, 4, cudaMemcpyDeviceToHost, s);
       ChunkBufs cb = j->cb;
-      cb.small_step = R.forms[rd];
+      set_step(cb, R.forms[rd]);
       launch_setup(R.pt->dev, cb, s);
       cudaMemsetAsync(j->cb.redo_count, 0, 4, s);
       tot.launches += (j->nsp > j->nsp_small ? 2 : 1) + 1;
@@ -2034,7 +2102,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
         Run &R = runs[r];
         if (rd >= R.chunks.size()) continue;
         ChunkBufs cb = R.j->cb;
-        cb.small_step = R.forms[rd];
+        set_step(cb, R.forms[rd]);
         launch_bsgs_exact(R.pt->dev, cb, R.pt->hb, R.pt->exact_grid, s);
         tot.launches++;
       }
@@ -2043,7 +2111,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
       if (rd >= R.chunks.size() || !R.own) continue;
       const cudaStream_t s = B->side[br++ % kBatchBranches];
       ChunkBufs cb = R.j->cb;
-      cb.small_step = R.forms[rd];
+      set_step(cb, R.forms[rd]);
       launch_bsgs(R.pt->dev, cb, R.pt->hb, R.pt->bsgs_grid, s);
       launch_bsgs_exact(R.pt->dev, cb, R.pt->hb, R.pt->exact_grid, s);
       tot.launches += 2;
@@ -2111,7 +2179,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
         again.push_back(R.chunks[c]);
       } else {
         st.primes += n;
-        const uint32_t f = R.forms[c];
+        const uint32_t f = R.forms[c].form;
         st.primes_by_step[f == kStepShoup ? 0 : f == kStepSmall ? 1 : 2] += n;
       }
     }

@@ -10,10 +10,9 @@
 
 namespace rs {
 
-// BSGS fast path: per-prime hash of 16-bit tags, kBucket tags per 16-byte bucket.
+// CTA kernel: per-prime hash of 16-bit tags, kBucket tags per 16-byte bucket.
 constexpr int kBucket = 8;
-constexpr int kMatchCap = 15;       // deferred tag matches per prime before the exact path (15 keeps
-                                    // the benchmark job at five 4-warp CTAs per SM)
+constexpr int kMatchCap = 64;       // warp kernel: a prime with more suspects takes the exact path
 // BSGS exact path (rare primes): 32-bit entries (tag << jbits) | j, linear probing.
 // j <= m-1 <= 2^jbits - 2, so a real entry is never all ones.
 constexpr uint32_t kEmpty = 0xffffffffu;
@@ -80,6 +79,18 @@ struct __align__(16) KInfo {
   uint64_t k_rcp;
 };
 
+// Shared memory of the warp-per-prime kernels: an SM's, what a CTA reserves, its
+// allocation granule, and the CTAs of four warps that registers allow on an SM.
+constexpr uint32_t kSmemPerSm = 233472, kSmemReserved = 1024, kSmemGranule = 1024, kWarpCtas = 5;
+// Bytes a warp needs beside its filter: tags, two record stages, V of a row mask.
+inline uint32_t warp_kernel_fixed(uint32_t chain_len, uint32_t stage_elems, bool row_mask) {
+  return 128 * chain_len + 16 * stage_elems + (row_mask ? 4 * kMaskRows : 0);
+}
+// Bytes a warp may use with `ctas` CTAs (and `fixed_smem` static bytes each) on an SM.
+inline uint32_t warp_kernel_share(uint32_t ctas, uint32_t fixed_smem) {
+  return (((kSmemPerSm / ctas - kSmemReserved) / kSmemGranule * kSmemGranule - fixed_smem) / kWarpsPerBlock) & ~15u;
+}
+
 // Job constants, passed by value to every kernel (lives in the constant bank).
 struct JobDev {
   uint32_t base;
@@ -98,8 +109,9 @@ struct JobDev {
   uint32_t tlanes;       // min(T, 32): lanes sharing one row
   uint32_t rows_per_it;  // 32 / tlanes
   uint32_t steps_per_lane;  // max(1, T / 32)
-  uint32_t table_log2;   // warp kernel: fast-path buckets per prime = 1 << table_log2
-  uint32_t nbuckets;     // fast-path buckets per prime (the CTA kernel: any multiple of 64)
+  uint32_t fwords;       // warp kernel: 32-bit words of a prime's filter (a multiple of 4)
+  uint32_t fshift;       // low bits of a key that do not choose the filter word (11..16)
+  uint32_t nbuckets;     // CTA kernel: fast-path buckets per prime (any multiple of 64)
   uint32_t jbits;        // bits of j in an exact-path table entry
   uint32_t nrows, nk;
   int64_t e0;            // x = e0 + m*s - j for giant index s in [1, T]
@@ -150,11 +162,12 @@ struct ChunkBufs {
   uint32_t *redo_count; // [1]
   uint32_t *exact_tab;  // exact-kernel tables of jobs whose table exceeds shared memory (else null)
   uint32_t cap;
-  // The baby step of the chunk: kStepSmall if every prime p of the chunk has
-  // p > 2^33 and b^Q * p < 2^63 (the short product by the integer b^Q,
-  // mul_small), kStepHigh if b^Q < 2^32 and b^Q * 2^32 < p (Shoup's product
-  // with a 32-bit constant), else kStepShoup (Shoup's product).
+  // The baby step of the chunk: kStepSmall (the short product by the integer
+  // b^Q, with step_shift chosen for the chunk's primes: LazyShort), kStepHigh (the
+  // same with step_shift = 32) or kStepShoup (Shoup's product by a full-size constant).
   uint32_t small_step;
+  uint32_t step_shift;
+  uint32_t pair_ok;     // mul_small by the base is valid for every prime of the chunk
 };
 
 struct HitBufs {
@@ -178,6 +191,7 @@ struct BatchItem {
   HitBufs hb;
 };
 constexpr uint32_t kBatchMaxItems = 256;  // items of one multi-job launch
+constexpr uint32_t kBatchStaticSmem = 4 * (kBatchMaxItems + 1) + 12;  // its prefix sums, 16-byte aligned
 
 // Launchers (rs_kernels.cu).  All enqueue on `st` and return the launch status.
 // Odd primes of [lo, hi] (lo odd) appended to out[] (count may exceed cap).
@@ -198,10 +212,9 @@ int bsgs_exact_smem_bytes(const JobDev &job);
 uint64_t bsgs_exact_scratch_bytes(const JobDev &job, int exact_grid);
 cudaError_t bsgs_configure(const JobDev &job, int device, int *grid_out, int *exact_grid_out);
 // Multi-job launch over `nitems` items in device memory that share rep's kernel
-// variant (rep: any of them); stage_max and table_log2_max are the largest over
-// the items; row_mask: the variant builds V from an active-row mask.
-// batch_configure gives its per-warp shared memory and grid.
-uint32_t batch_warp_bytes(uint32_t stage_max, uint32_t table_log2_max, bool row_mask);
+// variant (rep: any of them); stage_max is the largest over the items, and
+// warp_bytes holds every item's warp_kernel_bytes with that stage.
+// batch_configure gives the grid.
 cudaError_t batch_configure(const JobDev &rep, uint32_t warp_bytes, int device, int *grid_out);
 cudaError_t launch_bsgs_batch(const JobDev &rep, const BatchItem *items, uint32_t nitems, uint32_t stage_max,
                               uint32_t warp_bytes, int grid, cudaStream_t st);

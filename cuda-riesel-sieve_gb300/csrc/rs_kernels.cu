@@ -31,6 +31,7 @@
 //                  path's list, with an exact (tag, j) table.
 //   verify_kernel  direct k*b^n check of every hit (kernel_v0.24.6.cu:1649-1671).
 #include <cstdio>
+#include <type_traits>
 
 #include "rs_arith.cuh"
 #include "rs_internal.h"
@@ -257,17 +258,20 @@ __global__ void __launch_bounds__(128) setup_kernel(JobDev J, ChunkBufs cb) {
   const uint64_t bq = shoup_const(bm, M.pinv);     // Shoup constant of b
   const uint64_t B = mont_pow(bm, J.Q, one, M);    // b^Q
   const uint64_t e = J.e0 >= 0 ? (uint64_t)J.e0 : (p - 1) - (uint64_t)(-J.e0) % (p - 1);
-  const uint64_t H = mont_pow(B, e, one, M);       // B^e0
+  // B^e0 times lambda.  Every baby step and giant value carries the factor
+  // lambda = 2^64 mod p: the filter's keys are fractions y/p, and without it the
+  // first baby steps 1, B, B^2, ... of a large p would all have keys near zero.
+  const uint64_t H = montmul(mont_pow(B, e, one, M), r2, M);
   const uint64_t G = mont_pow(B, J.m, one, M);     // B^m
   const uint64_t Bc = mont_pow(B, J.chain_len, one, M);  // B^chain_len
 
-  // Lane tables: B^(lane*chain_len) (baby chain starts) and G^(lane % tlanes + 1)
+  // Lane tables: lambda*B^(lane*chain_len) (baby chain starts) and G^(lane % tlanes + 1)
   // (giant multipliers), stepped with Shoup products by the fixed B^chain_len
   // and G, 16 values per round.
   uint64_t Bs, Gs = 0;
   {
     const uint64_t Bw = from_mont(Bc, p, M.pinv), Bq = shoup_const(Bc, M.pinv);
-    uint64_t v = one;
+    uint64_t v = r2;  // lambda * B^0
 #pragma unroll 1
     for (uint32_t h = 0; h < 2; h++) {
 #pragma unroll 4
@@ -278,14 +282,16 @@ __global__ void __launch_bounds__(128) setup_kernel(JobDev J, ChunkBufs cb) {
       }
       flush_table_round(S, cb.recs, J.rec_elems, i0, n, J.el_tab + 16 * h, lane);
     }
-    Bs = v;  // B^(32*chain_len)
+    Bs = Bc;  // B^(32*chain_len)
+#pragma unroll 1
+    for (uint32_t q = 0; q < 5; q++) Bs = montmul(Bs, Bs, M);
     // value t of the G table is G^(t % tlanes + 1): the chain restarts at G
     // whenever t % tlanes wraps to 0 (tlanes divides 32)
     const uint64_t Gw = from_mont(G, p, M.pinv), Gq = shoup_const(G, M.pinv);
-    // integer rows: the table holds Z_(t+1) = +-B^e0 * G^(t+1) times 2^128 instead
+    // integer rows: the table holds Z_(t+1) = +-lambda*B^e0 * G^(t+1) instead (times 2^128 for the CTA kernel)
     uint64_t g0 = G;
     if (J.int_rows) {
-      uint64_t h2 = montmul(H, r2, M);  // B^e0 times 2^128
+      uint64_t h2 = J.cta_warps > 1 ? montmul(H, r2, M) : H;
       if (J.sign > 0 && h2) h2 = p - h2;
       g0 = shoup_mul(h2, Gw, Gq, p);
     }
@@ -705,7 +711,6 @@ struct TableT {
     return hit;
   }
 };
-using WarpTable = TableT<false>;
 
 struct MatchList {
   Match *list;
@@ -765,86 +770,262 @@ __device__ __forceinline__ void baby_chains(const Table &W, const MatchList &ML,
   }
 }
 
-// Giant steps with one step per row slot: lane (lane_row) multiplies the V of
-// slots gi*RPI + lane_row and (gi+1)*RPI + lane_row by its G^(lane_t+1) and
-// tests the home buckets; bit gi/2 of hA (hB) records a hit or full bucket.
-// PAIRED (RPI == 1 only): slots gi, gi+1 hold a (k, 0), (k, 1) pair, so the
-// second value is the first times the integer b (the short product).
-// INT: integer rows with k*b^r in V (Shoup's product for a 32-bit operand).
-template <uint32_t RPI, bool PAIRED = false, bool INT = false>
-__device__ __forceinline__ void giant_home(const WarpTable &W, const uint64_t *__restrict__ Vs, uint32_t ngi,
-                                           uint32_t nact, uint32_t lane_row, uint64_t Glw, uint64_t Glq, uint64_t p,
-                                           uint32_t &hA, uint32_t &hB, uint32_t b = 0, uint32_t rc = 0) {
-#pragma unroll 2
-  for (uint32_t gi = 0; gi < ngi; gi += 2) {
-    uint64_t va, vb;
-    if (RPI == 1) {
-      // slots gi, gi+1 are adjacent: one 16-byte load (gi even, V 16-byte
-      // aligned).  Slot gi+1 may be past nact; its value (still inside the V
-      // area) is discarded after the loop.
-      const uint4 w = *reinterpret_cast<const uint4 *>(Vs + gi);
-      va = ((uint64_t)w.y << 32) | w.x;
-      vb = ((uint64_t)w.w << 32) | w.z;
-    } else {
-      const uint32_t sa = gi * RPI + lane_row;
-      va = Vs[min(sa, nact - 1)];
-      vb = Vs[min(sa + RPI, nact - 1)];
+// Fractions.  The filter's keys are fractions of residues: for a Montgomery-form
+// residue u of y (u = y*2^64 mod p), u * (-p^-1) mod 2^64 = floor(y*2^64/p), the
+// 64-bit fraction F64 of y/p.  Two properties make this the cheap key:
+//   - it needs no reduced u: u + p gives F64 - 1;
+//   - for an integer row c < 2^32 and W the F64 of the lane's multiplier Z,
+//     c*W mod 2^64 = F64(c*Z mod p) - floor(c*u_Z/p), less than c < 2^32 below
+//     the exact fraction: a giant step is one 32x32 high product and one
+//     multiply-add, without the quotient, the remainder and its correction.
+// So with F the high word of a value's exact F64, a giant step sees f in
+// {F - 1, F}: baby steps must be found from both.
+__device__ __forceinline__ uint64_t frac64(uint64_t u, uint64_t pinv) { return u * pinv; }
+
+// Products for the baby chain without the final correction: from x < 2p to the
+// product mod p plus 0 or p.
+struct LazyShoup {  // any p < 2^63, by a full-size constant
+  uint64_t w, wq, np;
+  __device__ __forceinline__ uint64_t operator()(uint64_t x) const { return x * w + __umul64hi(x, wq) * np; }
+};
+// The short product by the integer c = b^Q: q = floor(floor(x/2^S) * K / 2^32)
+// with K = floor(c * 2^(32+S) / p) < 2^32 is at most 1 + c*2^S/p + x/2^(32+S)
+// below c*x/p.  The host picks S with both terms small enough (chunk_step_form),
+// so that x < 2p gives a remainder below 2p again.
+struct LazyShort {
+  uint32_t c, K, S;
+  uint64_t np;
+  __device__ __forceinline__ uint64_t operator()(uint64_t x) const {
+    const uint32_t q = __umulhi(__funnelshift_rc((uint32_t)x, (uint32_t)(x >> 32), S), K);
+    return x * (uint64_t)c + (uint64_t)q * np;
+  }
+};
+
+// Membership filter of a prime's baby steps (a Bloom filter blocked by 32-bit
+// words) on the high words F of their fractions: bits sh1.. of F choose the
+// word (scaled to any number of words); five bits from sh1 on and five from sh2 =
+// sh1 - 5 on each rotate a fixed pattern whose bits are set in the word.  A giant
+// value whose bits are all set is a suspect: a match, or one of the false
+// positives (1.1e-3 at 0.56 values a word, 4e-4 at 0.3), which the scan of
+// the tag list below rejects.  A giant step may see F - 1 for a value's F; that
+// has another key only if the low sh2 bits of F are zero, and those values are
+// stored for F - 1 too.  Against buckets of eight 16-bit tags with insert counts an insert
+// is one atomic OR without a return value (no slot, no tag store, no full
+// buckets), and a probe is one 4-byte load instead of a 16-byte one, which
+// random addresses cost more than twice the shared-memory wavefronts.
+// The patterns are the best of a random search for few false positives.
+//
+// What bounds the kernel is the integer pipes: a 32x32 high or wide product takes
+// four cycles of a scheduler's multiply pipe, a low one two, an add, shift or
+// logic operation two of its ALU, and the two overlap to about 75%.  On the
+// benchmark job at 1e13 a baby step (short product, key, insert) takes 38 cycles
+// against 36 for the reduced product and a bucket insert, and a giant step
+// (key, probe) 28 against 50: 2.13 ns per prime against 2.82.
+constexpr uint32_t kFiltA = 0x22009u, kFiltB = 0x2100005u;
+__device__ __forceinline__ uint32_t rotl(uint32_t v, uint32_t s) { return __funnelshift_l(v, v, s); }
+
+struct Filter {
+  uint32_t *w;
+  uint32_t mul;  // words << sh1
+  uint32_t sh1, sh2;
+  __device__ __forceinline__ void add(uint32_t F) const {
+    const uint32_t u = F >> sh1;
+    atomicOr(&w[__umulhi(u, mul)], rotl(kFiltA, u) | rotl(kFiltB, F >> sh2));
+  }
+  __device__ __forceinline__ bool test(uint32_t f) const {
+    const uint32_t u = f >> sh1;
+    return (~w[__umulhi(u, mul)] & (rotl(kFiltA, u) | rotl(kFiltB, f >> sh2))) == 0;
+  }
+};
+
+// Baby steps of one lane: two chains of `len` steps from va and vb, of which
+// the first na (nb) count (all of them when FULL) and go into the filter.  The
+// low 16 bits of both values' keys of step t are kept in tags[t * stride] for
+// the suspects' scan.  zmask: the low sh2 bits of both halves.  The key is that
+// of F64 + 1, which is exact for the unreduced residue and differs from the
+// reduced one's only where the fraction's low word is all ones, where no giant
+// step sees F - 1.
+template <bool FULL, class Step>
+__device__ __forceinline__ void baby_filter(const Filter &F, uint32_t *tags, uint32_t stride, uint32_t zmask,
+                                            uint64_t va, uint64_t vb, uint32_t na, uint32_t nb, uint32_t len,
+                                            uint64_t pinv, const Step &step) {
+  const uint32_t low = zmask & 0xffffu;
+  auto group = [&](auto count, uint32_t t0) {
+    constexpr uint32_t N = decltype(count)::value;
+    uint32_t fa[N], fb[N], z = 0xffffffffu;
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) {
+      const uint32_t t = t0 + i;
+      fa[i] = (uint32_t)((frac64(va, pinv) + 1) >> 32);
+      fb[i] = (uint32_t)((frac64(vb, pinv) + 1) >> 32);
+      if (FULL || t < na) F.add(fa[i]);
+      if (FULL || t < nb) F.add(fb[i]);
+      const uint32_t tp = __byte_perm(fa[i], fb[i], 0x5410);
+      tags[t * stride] = tp;
+      z = __vminu2(z, tp & zmask);
+      va = step(va);
+      vb = step(vb);
     }
-    const uint64_t ya = INT ? shoup_mul32((uint32_t)va, Glw, Glq, p) : shoup_mul(va, Glw, Glq, p);
-    const uint64_t yb = PAIRED ? mul_small(ya, b, rc, p)
-                               : (INT ? shoup_mul32((uint32_t)vb, Glw, Glq, p) : shoup_mul(vb, Glw, Glq, p));
-    const uint32_t bit = 1u << (gi >> 1);
-    if (W.probe_home(ya)) hA |= bit;
-    if (W.probe_home(yb)) hB |= bit;
+    if (zero_half(z)) {  // rare: a key whose low bits are zero
+#pragma unroll
+      for (uint32_t i = 0; i < N; i++) {
+        if ((fa[i] & low) == 0) F.add(fa[i] - 1);
+        if ((fb[i] & low) == 0) F.add(fb[i] - 1);
+      }
+    }
+  };
+  uint32_t t = 0;
+#pragma unroll 1
+  for (; t + 6 <= len; t += 6) group(std::integral_constant<uint32_t, 6>{}, t);
+#pragma unroll 1
+  for (; t + 2 <= len; t += 2) group(std::integral_constant<uint32_t, 2>{}, t);
+  if (t < len) group(std::integral_constant<uint32_t, 1>{}, t);
+}
+
+// A lane's giant multiplier from its table entry e (Montgomery form): the
+// residue w in normal form and its Shoup constant wq = floor(w * 2^64 / p), which
+// is also w's 64-bit fraction.  Integer rows: w = Z, and c*w is the giant value
+// in normal form; V rows: w = G^s, and V*w its Montgomery form.
+struct GiantMul {
+  uint64_t wq;
+  uint64_t p;
+  __device__ __forceinline__ void set(uint64_t e, uint64_t mod, uint64_t pinv) {
+    wq = frac64(e, pinv);
+    p = mod;
+  }
+  __device__ __forceinline__ uint64_t w() const { return wq ? __umul64hi(wq, p) + 1 : 0; }  // from_mont(e)
+};
+
+// The start value of row slot sl: an integer k*b^r from the row ids (u16 into
+// ctab), an active-row mask's list (u32) or V (u64), or V's residue.
+template <int RM>
+__device__ __forceinline__ uint64_t giant_start(const void *src, const uint32_t *__restrict__ ctab, uint32_t sl) {
+  if constexpr (RM == kRowsIntId) return __ldg(ctab + reinterpret_cast<const uint16_t *>(src)[sl]);
+  else if constexpr (RM == kRowsMask) return reinterpret_cast<const uint32_t *>(src)[sl];
+  else if constexpr (RM == kRowsIntV) return (uint32_t) reinterpret_cast<const uint64_t *>(src)[sl];
+  else return reinterpret_cast<const uint64_t *>(src)[sl];
+}
+
+// The exact giant value from its start value.
+template <int RM>
+__device__ __forceinline__ uint64_t giant_exact(uint64_t v, const GiantMul &G) {
+  return RM == kRowsV ? shoup_mul(v, G.w(), G.wq, G.p) : shoup_mul32((uint32_t)v, G.w(), G.wq, G.p);
+}
+
+// The key of a giant value: F or F - 1 (see above).  w: G.w(), V rows only.
+template <int RM>
+__device__ __forceinline__ uint32_t giant_key(uint64_t v, const GiantMul &G, uint64_t w, uint64_t np, uint64_t pinv) {
+  if constexpr (RM == kRowsV)
+    return (uint32_t)(frac64(v * w + __umul64hi(v, G.wq) * np, pinv) >> 32);
+  else
+    return (uint32_t)v * (uint32_t)(G.wq >> 32) + __umulhi((uint32_t)v, (uint32_t)G.wq);
+}
+
+// The key F of an exact giant value y from the key f a giant step saw (F or F -
+// 1).  True if the fraction's low word may be all ones, where a baby step may be
+// stored under F + 1.
+template <int RM>
+__device__ __forceinline__ bool exact_key(uint64_t y, uint32_t f, uint64_t p, uint64_t pinv, uint32_t &F) {
+  if constexpr (RM == kRowsV) {  // y in Montgomery form
+    const uint64_t F64 = frac64(y, pinv);
+    F = (uint32_t)(F64 >> 32);
+    return (uint32_t)F64 == 0xffffffffu;
+  } else {  // y in normal form: y*2^32 = F*p + r, 0 <= r < p
+    if (f == 0xffffffffu && y < (p >> 1)) f = 0;  // F = 0, seen as -1
+    uint64_t r = (y << 32) - (uint64_t)f * p;     // in [0, 2p)
+    if (r >= p) {
+      r -= p;
+      f++;
+    }
+    F = f;
+    return r + (p >> 32) + 1 >= p;
   }
 }
 
-// The same for integer rows: slot gi holds a row id (16 bits), whose k*b^r is
-// read from the job's table (read-only cache) and multiplied by the lane's Z
-// with Shoup's product for a 32-bit operand.  A slot past nact (RPI == 1, nact
-// odd) repeats slot gi; its outcome is discarded after the loop.
-template <uint32_t RPI, bool PAIRED = false>
-__device__ __forceinline__ void giant_home_int(const WarpTable &W, const uint16_t *__restrict__ Rs,
-                                               const uint32_t *__restrict__ ctab, uint32_t ngi, uint32_t nact,
-                                               uint32_t lane_row, uint64_t Glw, uint64_t Glq, uint64_t p, uint32_t &hA,
-                                               uint32_t &hB, uint32_t b = 0, uint32_t rc = 0) {
-#pragma unroll 2
-  for (uint32_t gi = 0; gi < ngi; gi += 2) {
-    uint32_t ra, rb;
-    if (RPI == 1) {
-      const uint32_t rr = *reinterpret_cast<const uint32_t *>(Rs + gi);  // slots gi, gi+1 (gi even)
-      ra = rr & 0xffffu;
-      rb = gi + 1 < nact ? rr >> 16 : ra;
+// One giant step of the row slots of passes [g0, g1), two passes at a time:
+// lane (lane_row) takes the start values of slots g*RPI + lane_row and
+// (g+1)*RPI + lane_row.  Outcomes: bit i of hA (passes g0 + 2i) and hB (g0 +
+// 2i + 1); at most 64 passes a call.  Slots past nact (RPI > 1) repeat a value;
+// the caller drops their outcomes.
+// PAIRED (RPI == 1, V rows): slots g, g+1 hold a (k, 0), (k, 1) pair, so the
+// second value is the first times the integer b (the short product).
+template <uint32_t RPI, int RM, bool PAIRED = false>
+__device__ __forceinline__ void giant_test(const Filter &F, const void *src, const uint32_t *__restrict__ ctab,
+                                           uint32_t g0, uint32_t g1, uint32_t nact, uint32_t lane_row,
+                                           const GiantMul &G, uint64_t np, uint64_t pinv, uint32_t &hA, uint32_t &hB,
+                                           uint32_t b = 0, uint32_t rc = 0) {
+  const uint64_t w = RM == kRowsV ? G.w() : 0;
+  auto pass = [&](uint32_t g, uint32_t bit, auto both, uint32_t &ha, uint32_t &hb) {
+    constexpr bool BOTH = decltype(both)::value;
+    uint64_t va, vb = 0;
+    if constexpr (RPI == 1 && RM == kRowsMask) {
+      const uint2 c = *reinterpret_cast<const uint2 *>(reinterpret_cast<const uint32_t *>(src) + g);
+      va = c.x;
+      vb = c.y;
+    } else if constexpr (RPI == 1 && RM == kRowsIntId) {
+      const uint32_t rr = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const uint16_t *>(src) + g);
+      va = __ldg(ctab + (rr & 0xffffu));
+      if (BOTH) vb = __ldg(ctab + (rr >> 16));
+    } else if constexpr (RPI == 1) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint64_t *>(src) + g);
+      va = ((uint64_t)v.y << 32) | v.x;
+      vb = ((uint64_t)v.w << 32) | v.z;
     } else {
-      const uint32_t sa = gi * RPI + lane_row;
-      ra = Rs[min(sa, nact - 1)];
-      rb = Rs[min(sa + RPI, nact - 1)];
+      const uint32_t sa = g * RPI + lane_row;
+      va = giant_start<RM>(src, ctab, min(sa, nact - 1));
+      if (BOTH) vb = giant_start<RM>(src, ctab, min(sa + RPI, nact - 1));
     }
-    const uint64_t ya = shoup_mul32(__ldg(ctab + ra), Glw, Glq, p);
-    const uint64_t yb = PAIRED ? mul_small(ya, b, rc, p) : shoup_mul32(__ldg(ctab + rb), Glw, Glq, p);
-    const uint32_t bit = 1u << (gi >> 1);
-    if (W.probe_home(ya)) hA |= bit;
-    if (W.probe_home(yb)) hB |= bit;
+    uint32_t fa, fb;
+    if constexpr (PAIRED && RM == kRowsV) {
+      const uint64_t ya = shoup_mul(va, w, G.wq, G.p);
+      fa = (uint32_t)(frac64(ya, pinv) >> 32);
+      fb = (uint32_t)(frac64(mul_small(ya, b, rc, G.p), pinv) >> 32);
+    } else {
+      fa = giant_key<RM>(va, G, w, np, pinv);
+      if (BOTH) fb = giant_key<RM>(vb, G, w, np, pinv);
+    }
+    if (F.test(fa)) ha |= bit;
+    if (BOTH && F.test(fb)) hb |= bit;
+  };
+  // Two iterations of constant outcome bits at a time, then what is left.
+  constexpr std::true_type two{};
+  uint32_t g = g0, sh = 0;
+#pragma unroll 1
+  for (; g + 4 <= g1; g += 4, sh += 2) {
+    uint32_t ha = 0, hb = 0;
+    pass(g, 1, two, ha, hb);
+    pass(g + 2, 2, two, ha, hb);
+    hA |= ha << sh;
+    hB |= hb << sh;
   }
+  uint32_t ha = 0, hb = 0;
+  if (g + 2 <= g1) {
+    pass(g, 1, two, ha, hb);
+    if (g + 2 < g1) pass(g + 2, 2, std::false_type{}, ha, hb);
+  } else if (g < g1) {
+    pass(g, 1, std::false_type{}, ha, hb);
+  }
+  hA |= ha << sh;
+  hB |= hb << sh;
 }
 
 // The work of one prime in the warp-per-prime layout, the whole warp together:
-// baby steps into the table, giant steps with home-bucket tests, deferred
-// probes, and the exact resolution of tag matches.  cur is the prime's staged
-// record (header, and V or the row mask; nact != 0), Bl and Glm the lane's two
-// table entries, c_lo / c_hi (row_mask) the lane's row constants; npaired
-// counts the primes that took the row-pair path.  Shared by the single-job
-// kernel and the multi-job kernel below.
+// baby steps into the filter, giant steps tested against it, and the exact
+// resolution of the suspects.  cur is the prime's staged record (header, and V
+// or the row mask; nact != 0), Bl and Glm the lane's two table entries, c_lo /
+// c_hi (row_mask) the lane's row constants, tags the lane's column of the tag
+// list; npaired counts the primes that took the row-pair path.  Shared by the
+// single-job kernel and the multi-job kernel below.
 template <int TL, int RM>
-__device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb, const HitBufs &hb,
-                                           const WarpTable &W, const MatchList &ML, uint64_t *vbuf,
+__device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb, const HitBufs &hb, uint32_t *fwords,
+                                           uint32_t nw, uint32_t *tags, uint32_t *vbuf,
                                            const uint64_t *cur, uint32_t i, uint32_t nact, uint64_t Bl,
                                            uint64_t Glm, uint32_t lane, uint32_t c_lo, uint32_t c_hi,
                                            uint32_t &npaired) {
   constexpr uint32_t RPI = 32 / TL;  // row slots per lane-group pass
   const uint32_t lane_t = lane & (TL - 1);
   const uint32_t lane_row = lane / TL;
-  const uint32_t spl = J.steps_per_lane;
+  const uint32_t spl = TL == 32 ? J.steps_per_lane : 1;
   if constexpr (RM == kRowsMask) {  // V from the active-row mask
     const uint64_t am = cur[kElV];
     const uint32_t lo = (uint32_t)am, hi = (uint32_t)(am >> 32), below = (1u << lane) - 1u;
@@ -855,175 +1036,146 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
   // Multipliers in normal form with their Shoup constants; the values
   // they multiply stay in Montgomery form, so products stay comparable.
   const uint64_t Stw = cur[kElStw], Stq = cur[kElStq];
-  const uint64_t Gw = cur[kElGw], Gq = cur[kElGq];
-  const uint64_t Glw = from_mont(Glm, p, pinv), Glq = shoup_const(Glm, pinv);
+  const uint64_t np = 0 - p;
+  Filter F;
+  F.w = fwords;
+  F.sh1 = J.fshift;
+  F.sh2 = J.fshift - 5;
+  F.mul = nw << J.fshift;
+  const uint32_t zmask = 0x10001u * ((1u << (J.fshift - 5)) - 1u);
   // chain starts B^(lane*CL) and B^((lane+32)*CL); valid steps na, nb (j < m)
   const uint32_t CL = J.chain_len;
   const uint32_t ja0 = lane * CL, jb0 = ja0 + 32 * CL;
   const uint32_t na = J.m > ja0 ? min(CL, J.m - ja0) : 0;
   const uint32_t nb = J.m > jb0 ? min(CL, J.m - jb0) : 0;
   const uint64_t Blb = shoup_mul(Bl, cur[kElOfw], cur[kElOfq], p);
-  // clear the table (tags and counts)
   const uint4 z4 = make_uint4(0, 0, 0, 0);
 #pragma unroll 4
-  for (uint32_t q = lane; q < W.nb + W.nb / 4; q += 32) W.tab4[q] = z4;
-  if (lane == 0) *ML.count = 0;
+  for (uint32_t q = lane; q < nw / 4; q += 32) reinterpret_cast<uint4 *>(fwords)[q] = z4;
   __syncwarp();
 
-  // Baby steps: chain A owns j = ja0 + t, chain B j = jb0 + t.  Values whose
-  // home bucket is full go to a short list (the match list's space, unused
-  // until the giant steps) and are inserted after the loop.
-  uint64_t *ovf = reinterpret_cast<uint64_t *>(ML.list);
-  if (J.m == 64 * CL) {  // every chain full (the planner's usual choice of m)
-    // (kStepHigh chunks take Shoup's product here: a third baby loop in this
-    // kernel measured slower on the short-product path)
-    if (cb.small_step == kStepSmall)
-      baby_chains<true>(W, ML, ovf, Bl, Blb, na, nb, CL, StepSmall{J.bq_small, (uint32_t)cur[kElRcp], p});
+  // Baby steps: chain A owns j = ja0 + t, chain B j = jb0 + t.
+  auto baby = [&](auto step) {
+    if (J.m == 64 * CL)  // every chain full (the planner's usual choice of m)
+      baby_filter<true>(F, tags, 32, zmask, Bl, Blb, na, nb, CL, pinv, step);
     else
-      baby_chains<true>(W, ML, ovf, Bl, Blb, na, nb, CL, StepShoup{Stw, Stq, p});
-  } else {
-    if (cb.small_step == kStepSmall)
-      baby_chains<false>(W, ML, ovf, Bl, Blb, na, nb, CL, StepSmall{J.bq_small, (uint32_t)cur[kElRcp], p});
-    else
-      baby_chains<false>(W, ML, ovf, Bl, Blb, na, nb, CL, StepShoup{Stw, Stq, p});
-  }
+      baby_filter<false>(F, tags, 32, zmask, Bl, Blb, na, nb, CL, pinv, step);
+  };
+  if (cb.small_step == kStepShoup) baby(LazyShoup{Stw, Stq, np});
+  else baby(LazyShort{J.bq_small, (uint32_t)(Stq >> (32 - cb.step_shift)), cb.step_shift, np});
   __syncwarp();
-  const uint32_t novf = *ML.count;
-  if (novf > 2 * ML.cap) {  // pathological table: leave the prime to the exact path
-    if (lane == 0) {
-      const uint32_t r = atomicAdd(cb.redo_count, 1u);
-      if (r < cb.cap) cb.redo[r] = i;
-    }
-    __syncwarp();
-    return;
-  }
-  if (novf) {
-    const uint64_t v = lane < novf ? ovf[lane] : 0;
-    __syncwarp();
-    if (lane == 0) *ML.count = 0;
-    if (lane < novf) W.insert_after(v, W.home((uint32_t)v));
-    __syncwarp();
-  }
 
   // Giant steps: lane (lane_row, lane_t) takes row slots g*RPI + lane_row for
-  // two consecutive passes g at a time, giant indices s = lane_t + 1 (+32).
+  // two consecutive passes g at a time, giant indices s = lane_t + 1 + 32u.
   const uint32_t ngi = (nact + RPI - 1) / RPI;
-  const uint64_t *Vs = J.stage_full ? cur + kElV : cb.recs + (size_t)i * J.rec_elems + kElV;
-  // integer rows: the row ids (16 bits) of the staged or global record
-  const uint16_t *Rs = reinterpret_cast<const uint16_t *>(
-      J.stage_full ? cur + J.el_row : cb.recs + (size_t)i * J.rec_elems + J.el_row);
-  // the giant value of slot sl (the general and the integer-row form)
-  auto giant_val = [&](uint32_t sl) -> uint64_t {
-    if constexpr (RM == kRowsIntId) return shoup_mul32(__ldg(J.row_c + Rs[sl]), Glw, Glq, p);
-    else if constexpr (RM == kRowsIntV) return shoup_mul32((uint32_t)Vs[sl], Glw, Glq, p);
-    else if constexpr (RM == kRowsMask) return shoup_mul32((uint32_t)vbuf[sl], Glw, Glq, p);
-    else return shoup_mul(Vs[sl], Glw, Glq, p);
+  // the start values (or row ids): built by the warp, staged, or in the record
+  const void *src_s = RM == kRowsMask ? (const void *)vbuf
+                                      : RM == kRowsIntId ? (const void *)(cur + J.el_row) : (const void *)(cur + kElV);
+  const void *src_g = cb.recs + (size_t)i * J.rec_elems + (RM == kRowsIntId ? J.el_row : kElV);
+  const bool staged = RM == kRowsMask || J.stage_full;
+  // (k, 0), (k, 1) row pairs; V rows form the second value by the short product
+  // by b (p > 2^33, b*p < 2^63: mul_small)
+  const bool paired = RPI == 1 && cb.pair_ok && (cur[kElNact] >> 32);
+  npaired += paired && staged && spl == 1;
+  // A lane's further steps (T > 32): advance the multiplier once and go through
+  // the rows again; in blocks of at most 64 tests a lane, after which the block's
+  // suspects are settled.
+  uint64_t E = Glm;  // the lane's multiplier as stored, advanced by G^32 per step u
+  GiantMul G;
+  G.set(E, p, pinv);
+  auto start = [&](uint32_t sl) {
+    return staged ? giant_start<RM>(src_s, J.row_c, sl) : giant_start<RM>(src_g, J.row_c, sl);
   };
-  if (spl == 1 && ngi <= 64) {
-    // One giant step per slot.  The loop only tests each value's home
-    // bucket and collects the outcome as bits (pass gi of chain A or B ->
-    // bit gi/2); tag hits and full home buckets are finished after it.
+  uint32_t u = 0, at = 0, suspects = 0;  // step, the block's first pass, suspects so far
+#pragma unroll 1
+  while (true) {
+    const uint32_t g1 = min(ngi, at + 64);
+    uint32_t hA = 0, hB = 0;
     // Separate calls for staged and global V keep each load's address
     // space known to the compiler.
-    uint32_t hA = 0, hB = 0;
-    const bool paired = RPI == 1 && cb.small_step == kStepSmall && (cur[kElNact] >> 32);
-    npaired += paired && J.stage_full;
-    if constexpr (RM == kRowsIntId) {
-      const uint16_t *Rst = reinterpret_cast<const uint16_t *>(cur + J.el_row);
-      if (paired && J.stage_full)
-        giant_home_int<RPI, RPI == 1>(W, Rst, J.row_c, ngi, nact, lane_row, Glw, Glq, p, hA, hB, J.base,
-                                      (uint32_t)cur[kElRcp]);
-      else if (J.stage_full)
-        giant_home_int<RPI>(W, Rst, J.row_c, ngi, nact, lane_row, Glw, Glq, p, hA, hB);
-      else
-        giant_home_int<RPI>(W, Rs, J.row_c, ngi, nact, lane_row, Glw, Glq, p, hA, hB);
-    } else {
-      constexpr bool INT = RM == kRowsIntV || RM == kRowsMask;
-      const uint64_t *Vst = RM == kRowsMask ? vbuf : cur + kElV;  // V in shared memory
-      if (paired && J.stage_full)
-        giant_home<RPI, RPI == 1, INT>(W, Vst, ngi, nact, lane_row, Glw, Glq, p, hA, hB, J.base,
-                                       (uint32_t)cur[kElRcp]);
-      else if (J.stage_full)
-        giant_home<RPI, false, INT>(W, Vst, ngi, nact, lane_row, Glw, Glq, p, hA, hB);
-      else
-        giant_home<RPI, false, INT>(W, Vs, ngi, nact, lane_row, Glw, Glq, p, hA, hB);
-    }
-    if (hA | hB) {
+    if (RM == kRowsV && paired && staged)
+      giant_test<RPI, RM, RPI == 1>(F, src_s, J.row_c, at, g1, nact, lane_row, G, np, pinv, hA, hB, J.base,
+                                    (uint32_t)cur[kElRcp]);
+    else if (staged)
+      giant_test<RPI, RM>(F, src_s, J.row_c, at, g1, nact, lane_row, G, np, pinv, hA, hB);
+    else
+      giant_test<RPI, RM>(F, src_g, J.row_c, at, g1, nact, lane_row, G, np, pinv, hA, hB);
+    // Suspects: every lane forms the exact value and key of its next one, then
+    // the warp takes them in turn: each lane scans its own tags (its two chains,
+    // 16 bits of each value's key), and a tag match is settled by walking the
+    // two chains again in the exact values' form.
+    uint64_t bits = ((uint64_t)hB << 32) | hA;
 #pragma unroll 1
-      for (uint32_t h = 0; h < 2; h++) {
-        uint32_t bits = h ? hB : hA;
-        while (bits) {
-          const uint32_t g = 2 * (__ffs(bits) - 1) + h;
-          bits &= bits - 1;
-          const uint32_t sl = g * RPI + lane_row;
-          if (sl < nact) {
-            const uint64_t y = giant_val(sl);
-            if (W.probe(y)) ML.push(y, sl, lane_t + 1);
-          }
+    while (uint32_t any = __ballot_sync(0xffffffffu, bits != 0)) {
+      const uint32_t bit = bits ? __ffsll((long long)bits) - 1 : 0;
+      const uint32_t sl = (at + 2 * (bit & 31) + (bit >> 5)) * RPI + lane_row;
+      const bool mine = bits != 0 && sl < nact;
+      bits &= bits - 1;
+      any = __ballot_sync(0xffffffffu, mine);
+      suspects += __popc(any);
+      if (suspects > (uint32_t)kMatchCap) {  // the exact path takes the prime
+        if (lane == 0) {
+          const uint32_t r = atomicAdd(cb.redo_count, 1u);
+          if (r < cb.cap) cb.redo[r] = i;
         }
+        return;
       }
-    }
-  } else {
-#pragma unroll 1
-    for (uint32_t gi = 0; gi < ngi; gi += 2) {
-      const uint32_t sa = gi * RPI + lane_row, sb = sa + RPI;
-      const bool aa = sa < nact, ab = sb < nact;
-      uint64_t ya = giant_val(min(sa, nact - 1));
-      uint64_t yb = giant_val(min(sb, nact - 1));
-      uint32_t s = lane_t + 1;
-#pragma unroll 1
-      for (uint32_t u = 0;; u++) {
-        if (W.probe(ya) && aa) ML.push(ya, sa, s);
-        if (W.probe(yb) && ab) ML.push(yb, sb, s);
-        if (u + 1 >= spl) break;
-        ya = shoup_mul(ya, Gw, Gq, p);
-        yb = shoup_mul(yb, Gw, Gq, p);
-        s += 32;
+      uint64_t y = 0;
+      uint32_t f = 0;
+      bool edge = false;
+      if (mine) {
+        const uint64_t v = start(sl);
+        y = giant_exact<RM>(v, G);
+        edge = exact_key<RM>(y, giant_key<RM>(v, G, RM == kRowsV ? G.w() : 0, np, pinv), p, pinv, f);
       }
-    }
-  }
-  __syncwarp();
-
-  // Tag matches: recompute the baby steps and compare full 64-bit values.
-  const uint32_t mc = *ML.count;
-  if (mc > (uint32_t)kMatchCap) {
-    if (lane == 0) {
-      const uint32_t r = atomicAdd(cb.redo_count, 1u);
-      if (r < cb.cap) cb.redo[r] = i;
-    }
-  } else if (mc > 0) {
-    uint64_t va = Bl, vb = Blb;
-#pragma unroll 1
-    for (uint32_t t = 0; t < CL; t++) {
+      const uint32_t both = __ballot_sync(0xffffffffu, edge);  // these could be stored under F + 1 too
 #pragma unroll 1
       for (uint32_t h = 0; h < 2; h++) {
-        const uint64_t v = h ? vb : va;
-        if (t < (h ? nb : na)) {
 #pragma unroll 1
-          for (uint32_t q = 0; q < mc; q++) {
-            const Match mt = ML.list[q];
-            if (mt.y == v) {
+        for (uint32_t left = h ? both : any; left; left &= left - 1) {
+          const int src = __ffs(left) - 1;
+          const uint32_t T = __byte_perm(__shfl_sync(0xffffffffu, f, src) + h, 0, 0x1010);
+          uint32_t z = 0xffffffffu;
+#pragma unroll 6
+          for (uint32_t t = 0; t < CL; t++) z = __vminu2(z, tags[t * 32] ^ T);
+          if (!__any_sync(0xffffffffu, zero_half(z))) continue;
+          const uint64_t ys = __shfl_sync(0xffffffffu, y, src);
+          const uint32_t slot = __shfl_sync(0xffffffffu, sl, src);
+          uint64_t va = RM == kRowsV ? Bl : from_mont(Bl, p, pinv);
+          uint64_t vb = RM == kRowsV ? Blb : from_mont(Blb, p, pinv);
+#pragma unroll 1
+          for (uint32_t t = 0; t < CL; t++) {
+            const bool ma = va == ys && t < na, mb = vb == ys && t < nb;
+            if (ma || mb) {
+              const uint32_t s = ((uint32_t)src & (TL - 1)) + 1 + 32 * u;
               uint32_t row;
               if constexpr (RM == kRowsMask) {
-                row = nth_row(cur[kElV], mt.slot);
+                row = nth_row(cur[kElV], slot);
               } else {
-                const uint64_t pk = rec_el(J, cb, J.el_row + (mt.slot >> 2), i);
-                row = (uint32_t)(pk >> (16 * (mt.slot & 3))) & 0xffffu;
+                const uint64_t pk = rec_el(J, cb, J.el_row + (slot >> 2), i);
+                row = (uint32_t)(pk >> (16 * (slot & 3))) & 0xffffu;
               }
-              record_hit(J, hb, p, row, mt.s, (h ? jb0 : ja0) + t);
+              if (ma) record_hit(J, hb, p, row, s, ja0 + t);
+              if (mb) record_hit(J, hb, p, row, s, jb0 + t);
             }
+            va = shoup_mul(va, Stw, Stq, p);
+            vb = shoup_mul(vb, Stw, Stq, p);
           }
         }
       }
-      va = shoup_mul(va, Stw, Stq, p);
-      vb = shoup_mul(vb, Stw, Stq, p);
     }
+    at = g1;
+    if (at < ngi) continue;
+    if (++u >= spl) break;
+    at = 0;
+    E = shoup_mul(E, cur[kElGw], cur[kElGq], p);
+    G.set(E, p, pinv);
   }
 }
 
 // Per-warp shared memory of the fast kernel:
-//   [NB buckets x 16 B][NB counts x 4 B][2 stages x stage_elems x 8 B]
-//   ([kMaskRows V x 8 B], row_mask only)[kMatchCap matches][count, 16 B]
+//   [filter, fwords x 4 B][tags, chain_len x 32 x 4 B][2 stages x stage_elems x 8 B]
+//   ([kMaskRows V x 4 B], row_mask only)
 // The stages hold a record's header and V (double-buffered with cp.async); each
 // lane's B^lane and G^(lane+1) entries are loaded into registers one prime ahead.
 // With row_mask the stage holds the header and the active-row mask, and the
@@ -1041,20 +1193,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 4)
 bsgs_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
   extern __shared__ uint4 smem4[];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t NB = 1u << J.table_log2;
   uint8_t *base = reinterpret_cast<uint8_t *>(smem4) + (size_t)warp * J.warp_smem;
-  WarpTable W;
-  W.tab4 = reinterpret_cast<uint4 *>(base);
-  W.tab16 = reinterpret_cast<uint16_t *>(base);
-  W.cnt32 = reinterpret_cast<uint32_t *>(base + NB * 16);
-  W.nb = NB;
-  W.bmask = NB - 1;
-  uint64_t *stage0 = reinterpret_cast<uint64_t *>(base + NB * 20);
-  uint64_t *vbuf = stage0 + 2 * J.stage_elems;  // row_mask: V of the current prime
-  MatchList ML;
-  ML.list = reinterpret_cast<Match *>(vbuf + (RM == kRowsMask ? kMaskRows : 0));
-  ML.count = reinterpret_cast<uint32_t *>(ML.list + kMatchCap);
-  ML.cap = kMatchCap;
+  uint32_t *fwords = reinterpret_cast<uint32_t *>(base);
+  uint32_t *tags = fwords + J.fwords + lane;
+  uint64_t *stage0 = reinterpret_cast<uint64_t *>(fwords + J.fwords + 32 * J.chain_len);
+  uint32_t *vbuf = reinterpret_cast<uint32_t *>(stage0 + 2 * J.stage_elems);  // row_mask: V of the current prime
   const uint32_t total = *cb.count;
   const uint32_t n = total < cb.cap ? total : cb.cap;
   const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
@@ -1093,7 +1236,8 @@ bsgs_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
     stage_wait_prev();
     __syncwarp();
     const uint32_t nact = (uint32_t)cur[kElNact];
-    if (nact != 0) bsgs_prime<TL, RM>(J, cb, hb, W, ML, vbuf, cur, i, nact, Bl, Glm, lane, c_lo, c_hi, npaired);
+    if (nact != 0)
+      bsgs_prime<TL, RM>(J, cb, hb, fwords, J.fwords, tags, vbuf, cur, i, nact, Bl, Glm, lane, c_lo, c_hi, npaired);
     __syncwarp();
   }
   stage_wait_all();
@@ -1108,12 +1252,12 @@ bsgs_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
 // and baby-step product; all items share the template's giant lanes TL and
 // start-value form RM.  Per-warp shared memory, in fixed places whatever the
 // item:
-//   [2 stages x stage_max x 8 B]([kMaskRows V x 8 B], RM = kRowsMask)[kMatchCap matches][count, 16 B]
-//   [the item's table: NB buckets x 16 B, NB counts x 4 B]
+//   [2 stages x stage_max x 8 B]([kMaskRows V x 4 B], RM = kRowsMask)
+//   [the item's filter, fwords x 4 B, and tags, chain_len x 32 x 4 B]
 // The record of the warp's next prime (possibly another item's) is staged by
 // cp.async while the current one runs, as in bsgs_kernel.
 template <int TL, int RM>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 4)
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, kWarpCtas)
 bsgs_batch_kernel(const BatchItem *__restrict__ items, uint32_t nitems, uint32_t warp_bytes, uint32_t stage_max) {
   extern __shared__ uint4 smem4[];
   __shared__ uint32_t start[kBatchMaxItems + 1];  // prefix sums of the items' prime counts
@@ -1132,12 +1276,8 @@ bsgs_batch_kernel(const BatchItem *__restrict__ items, uint32_t nitems, uint32_t
   const uint32_t total = start[nitems];
   uint8_t *base = reinterpret_cast<uint8_t *>(smem4) + (size_t)warp * warp_bytes;
   uint64_t *stage0 = reinterpret_cast<uint64_t *>(base);
-  uint64_t *vbuf = stage0 + 2 * stage_max;
-  MatchList ML;
-  ML.list = reinterpret_cast<Match *>(vbuf + (RM == kRowsMask ? kMaskRows : 0));
-  ML.count = reinterpret_cast<uint32_t *>(ML.list + kMatchCap);
-  ML.cap = kMatchCap;
-  uint8_t *tbase = reinterpret_cast<uint8_t *>(ML.count) + 16;
+  uint32_t *vbuf = reinterpret_cast<uint32_t *>(stage0 + 2 * stage_max);
+  uint32_t *fwords = vbuf + (RM == kRowsMask ? kMaskRows : 0);
   const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
   const uint32_t first = blockIdx.x * kWarpsPerBlock + warp;
   // the item of global index g, from the item of an earlier (smaller) index
@@ -1187,16 +1327,9 @@ bsgs_batch_kernel(const BatchItem *__restrict__ items, uint32_t nitems, uint32_t
     stage_wait_prev();
     __syncwarp();
     const uint32_t nact = (uint32_t)cur[kElNact];
-    if (nact != 0) {
-      const uint32_t NB = 1u << X.J.table_log2;
-      WarpTable W;
-      W.tab4 = reinterpret_cast<uint4 *>(tbase);
-      W.tab16 = reinterpret_cast<uint16_t *>(tbase);
-      W.cnt32 = reinterpret_cast<uint32_t *>(tbase + NB * 16);
-      W.nb = NB;
-      W.bmask = NB - 1;
-      bsgs_prime<TL, RM>(X.J, X.cb, X.hb, W, ML, vbuf, cur, i, nact, Bl, Glm, lane, c_lo, c_hi, npaired);
-    }
+    if (nact != 0)
+      bsgs_prime<TL, RM>(X.J, X.cb, X.hb, fwords, X.J.fwords, fwords + X.J.fwords + lane, vbuf, cur, i, nact, Bl,
+                         Glm, lane, c_lo, c_hi, npaired);
     __syncwarp();
   }
   stage_wait_all();
@@ -1535,6 +1668,8 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
     for (uint32_t c = 0; c < 2; c++) {
       const uint32_t j0 = (gt + G * c) * J.chain_len;
       uint64_t v = c ? shoup_mul(Bl, rec_el(J, cb, kElOfw, i), rec_el(J, cb, kElOfq, i), p) : Bl;
+      // integer rows of the warp layout: giant values (below) come in normal form
+      if (WG == 1 && J.int_rows) v = from_mont(v, p, pinv);
 #pragma unroll 1
       for (uint32_t j = j0; j < J.m && j < j0 + J.chain_len; j++) {
         uint32_t h = (uint32_t)v & tmask;
@@ -1558,7 +1693,8 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
         const uint32_t row = J.row_mask ? nth_row(rec_el(J, cb, J.el_v, i), slot)
                                         : (uint32_t)(rec_el(J, cb, J.el_row + (slot >> 2), i) >> (16 * (slot & 3))) &
                                               0xffffu;
-        // integer rows: montmul(k*b^r, Z * 2^128) is the Montgomery form of the giant value
+        // integer rows: montmul(k*b^r, Z * 2^128) is the Montgomery form of the giant
+        // value (CTA layout); with Z's Montgomery form (warp layout) its normal form
         uint64_t y = montmul(J.row_ids_only || J.row_mask ? (uint64_t)__ldg(J.row_c + row)
                                                           : rec_el(J, cb, J.el_v + slot, i),
                              Gl, p, pinv);
@@ -1676,10 +1812,6 @@ static BatchFn batch_fn(const JobDev &rep) {
   }
 }
 
-uint32_t batch_warp_bytes(uint32_t stage_max, uint32_t table_log2_max, bool row_mask) {
-  const uint32_t b = 16 * stage_max + (row_mask ? 8 * kMaskRows : 0) + 16 * kMatchCap + 16 + (20u << table_log2_max);
-  return (b + 15) & ~15u;
-}
 
 cudaError_t batch_configure(const JobDev &rep, uint32_t warp_bytes, int device, int *grid_out) {
   return configure_one((const void *)batch_fn(rep), kWarpsPerBlock * (int)warp_bytes, 32 * kWarpsPerBlock, device,
