@@ -700,6 +700,11 @@ struct rs_job {
   uint32_t chunk_cap = 0;
   uint32_t chunk_rec_elems = 0;  // record elements the chunk buffers were sized for
   uint64_t chunk_exact_bytes = 0;  // exact-kernel scratch they hold
+  bool has_cta() const {
+    for (auto &pt : parts)
+      if (pt->dev.cta_warps > 1) return true;
+    return false;
+  }
   uint32_t max_rec_elems() const {
     uint32_t r = 0;
     for (auto &pt : parts) r = std::max(r, pt->dev.rec_elems);
@@ -762,7 +767,8 @@ static uint32_t plan_row_form(const Plan &pl, const Seqs &s, std::vector<uint32_
 // First element of the lane tables in a record (el_tab; a record has el_tab + 64
 // elements), from the plan and the row form, as upload_part lays it out.
 static uint32_t record_el_tab(const Plan &pl, uint32_t form) {
-  const uint32_t el_v = pl.cta ? kElWoff + 2 * kCtaWarps : kElV;
+  const uint32_t el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : kElV;
+  if (pl.cta) form = kRowsIntId;  // CTA records hold row ids only
   if (form == kRowsMask) return el_v + 2;
   const uint32_t max_act = std::max<uint32_t>(1, pl.nrows);
   const uint32_t el_row = el_v + (form == kRowsIntId ? 0u : ((max_act + 1) & ~1u));
@@ -773,7 +779,7 @@ static uint32_t record_el_tab(const Plan &pl, uint32_t form) {
 // character tables included), from a plan made without the bitmap.
 static uint64_t part_array_bytes(const Plan &pl, const Seqs &s, bool datless) {
   const uint64_t nk = s.k.size(), nr = pl.nrows;
-  uint64_t b = 3 * nr * 4 + nk * (4 + 4 + 4 + 8 + 4 + sizeof(KInfo)) + (nk + 1) * 4;
+  uint64_t b = 6 * nr * 4 + 4ull * pl.Q + nk * (4 + 4 + 4 + 8 + 4 + sizeof(KInfo)) + (nk + 1) * 4;
   b += datless ? 4 : nr * (uint64_t)pl.words_per_row * 4;
   std::vector<uint32_t> odd;
   for (uint32_t k : s.k) {
@@ -788,7 +794,7 @@ static uint64_t part_array_bytes(const Plan &pl, const Seqs &s, bool datless) {
   uint64_t words = 0;
   for (uint32_t k : odd) words += (k + 31) / 32;
   if (words <= (256ull << 20)) b += words * 4 + odd.size() * 8;
-  return b + 20 * 256;  // section alignment
+  return b + 23 * 256;  // section alignment
 }
 
 // Primes in [a, b], estimated (b - a + 1) / ln b.
@@ -881,6 +887,25 @@ static int upload_part(rs_job *j, Part &pt) {
   };
   std::vector<uint32_t> row_c;
   const uint32_t form = plan_row_form(pl, s, &row_c);
+  // the residues' row lists of the CTA kernel, each from a multiple of 4 slots
+  std::vector<uint32_t> row_k(pl.row_r.size()), row_base(pl.Q, 0);
+  uint32_t row_slots = 0;
+  {
+    std::vector<uint32_t> per(pl.Q, 0);
+    for (size_t r = 0; r < pl.row_r.size(); r++) {
+      row_k[r] = s.k[pl.row_kidx[r]];
+      per[pl.row_r[r]]++;
+    }
+    for (uint32_t r = 0; r < pl.Q; r++) {
+      row_base[r] = row_slots;
+      row_slots += (per[r] + 3) & ~3u;
+    }
+    row_slots = (row_slots + 7) & ~7u;
+  }
+  std::vector<uint64_t> row_kr(pl.row_r.size());
+  for (size_t r = 0; r < row_kr.size(); r++)
+    row_kr[r] = row_k[r] | (uint64_t)(pl.row_r[r] | row_base[pl.row_r[r]] << 12) << 32;
+  const size_t o_rw = sec(row_k.size() * 4), o_rb = sec(row_base.size() * 4), o_rx = sec(row_kr.size() * 8);
   const size_t o_rr = sec(pl.row_r.size() * 4), o_rk = sec(pl.row_kidx.size() * 4), o_rc = sec(row_c.size() * 4);
   const size_t o_kv = sec(nk * 4), o_ko = sec(nk * 4), o_ke = sec(nk * 4), o_kr = sec(nk * 8);
   const size_t o_k0 = sec((nk + 1) * 4), o_bm = sec(pl.bitmap.size() * 4);
@@ -926,6 +951,9 @@ static int upload_part(rs_job *j, Part &pt) {
   const size_t o_jb = sec(twords * 4);
   pt.job_bytes = o_jb;  // bytes uploaded (the character tables are built on the device)
   std::vector<uint8_t> host(o_jb, 0);
+  memcpy(host.data() + o_rw, row_k.data(), row_k.size() * 4);
+  memcpy(host.data() + o_rb, row_base.data(), row_base.size() * 4);
+  memcpy(host.data() + o_rx, row_kr.data(), row_kr.size() * 8);
   memcpy(host.data() + o_rr, pl.row_r.data(), pl.row_r.size() * 4);
   memcpy(host.data() + o_rk, pl.row_kidx.data(), pl.row_kidx.size() * 4);
   memcpy(host.data() + o_rc, row_c.data(), row_c.size() * 4);
@@ -985,7 +1013,6 @@ static int upload_part(rs_job *j, Part &pt) {
   d.tlanes = pl.tlanes;
   d.rows_per_it = pl.rows_per_it;
   d.steps_per_lane = pl.steps_per_lane;
-  d.nbuckets = pl.nbuckets;
   d.exact_log2 = pl.table_log2;
   d.jbits = pl.jbits;
   d.nrows = pl.nrows;
@@ -998,10 +1025,12 @@ static int upload_part(rs_job *j, Part &pt) {
   d.words_per_row = pl.words_per_row;
   d.datless = j->opt.datless ? 1u : 0u;
   d.max_act = std::max<uint32_t>(1, pl.nrows);
-  d.int_rows = form != kRowsV ? 1u : 0u;
-  d.row_ids_only = form == kRowsIntId ? 1u : 0u;  // no V in the record
-  d.row_mask = form == kRowsMask ? 1u : 0u;       // neither V nor row ids: an active-row mask
-  d.el_v = d.cta_warps > 1 ? kElWoff + 2 * d.cta_warps : kElV;
+  // CTA layout: every row is the integer k (the kernel multiplies by b^r), its
+  // records hold row ids only
+  d.int_rows = pl.cta || form != kRowsV ? 1u : 0u;
+  d.row_ids_only = pl.cta || form == kRowsIntId ? 1u : 0u;  // no V in the record
+  d.row_mask = !pl.cta && form == kRowsMask ? 1u : 0u;      // neither V nor row ids: an active-row mask
+  d.el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : kElV;
   if (d.row_mask) {
     d.el_row = d.el_v;
     d.el_tab = d.el_v + 2;
@@ -1021,18 +1050,22 @@ static int upload_part(rs_job *j, Part &pt) {
     d.stage_elems = d.el_v;
   }
   d.ctab_smem = 0;
-  if (d.cta_warps > 1) {  // bytes per CTA: table, counts, V (or row ids), match list (, row table)
-    d.warp_smem = (uint32_t)align_up(20u * d.nbuckets +
-                                         (d.row_ids_only ? 16 * ((d.max_act + 7) / 8) : 8 * ((d.max_act + 1) & ~1u)) +
-                                         kCtaMatchCap * 16 + 16,
-                                     16);
-    // row ids: the kernel reads k*b^r of each row from a shared-memory copy of
-    // the job's row table when it fits beside the rest
-    const uint32_t ctab_bytes = (uint32_t)align_up(4ull * d.nrows, 16);
-    if (d.row_ids_only && d.warp_smem + ctab_bytes <= kCtaSmemMax) {
-      d.ctab_smem = 1;
-      d.warp_smem += ctab_bytes;
-    }
+  if (d.cta_warps > 1) {
+    // bytes per CTA: tags, the rows' ids and (when 1.5 filter words a baby step
+    // still fit) their k, suspects and keys, counts; the filter takes the rest up
+    // to 3.5 words a baby step
+    d.row_slots = row_slots;
+    const uint64_t fixed = align_up(2ull * pl.m + 2ull * row_slots + 20ull * kCtaMatchCap + 4ull * pl.Q + 16, 16);
+    d.ctab_smem = fixed + 4ull * row_slots + 6ull * pl.m <= kCtaSmemMax ? 1u : 0u;
+    const uint64_t used = fixed + (d.ctab_smem ? 4ull * row_slots : 0);
+    const uint64_t left = used < kCtaSmemMax ? (kCtaSmemMax - used) / 16 * 4 : 0;
+    d.fwords = (uint32_t)std::min<uint64_t>({left, 65532, std::max<uint64_t>(1024, (7ull * pl.m / 2 + 3) & ~3ull)});
+    if (d.fwords < 256) return fail(RS_ERR_INVALID, "a CTA plan's rows leave no shared memory for its filter");
+    d.fshift = filter_shift(d.fwords);
+    d.warp_smem = (uint32_t)(4ull * d.fwords + used);
+    uint64_t kmax = 0;
+    for (uint32_t k : s.k) kmax = std::max<uint64_t>(kmax, k);
+    d.edge_lim = (uint32_t)std::min<uint64_t>(0xffffffffu, ((kmax + 1) >> (d.fshift - 10)) + 1);
   } else {  // bytes per warp: the filter takes what the shared memory leaves (warp_filter)
     const uint32_t fixed = warp_kernel_fixed(d.chain_len, d.stage_elems, d.row_mask != 0);
     d.fwords = warp_filter(pl.m, fixed, 0, pt.ctas);
@@ -1042,6 +1075,9 @@ static int upload_part(rs_job *j, Part &pt) {
   d.row_r = (const uint32_t *)(b + o_rr);
   d.row_kidx = (const uint32_t *)(b + o_rk);
   d.row_c = (const uint32_t *)(b + o_rc);
+  d.row_k = (const uint32_t *)(b + o_rw);
+  d.row_base = (const uint32_t *)(b + o_rb);
+  d.row_kr = (const uint2 *)(b + o_rx);
   d.k_val = (const uint32_t *)(b + o_kv);
   d.k_odd = (const uint32_t *)(b + o_ko);
   d.k_e2 = (const uint32_t *)(b + o_ke);
@@ -1125,7 +1161,9 @@ static int ensure_gbits(rs_job *j, uint64_t words) {
   return RS_OK;
 }
 
-static size_t chunk_bytes_per_prime(const rs_job *j) { return 8 + 4 + 8 * (size_t)j->max_rec_elems(); }
+static size_t chunk_bytes_per_prime(const rs_job *j) {
+  return 8 + 4 + 8 * (size_t)j->max_rec_elems() + (j->has_cta() ? kCandPerPrime * sizeof(Candidate) : 0);
+}
 
 static uint64_t exact_scratch_bytes(const rs_job *j) {
   uint64_t b = 0;
@@ -1136,7 +1174,9 @@ static uint64_t exact_scratch_bytes(const rs_job *j) {
 static int ensure_chunk_buffers(rs_job *j, uint32_t cap) {
   const uint32_t rec = j->max_rec_elems();
   const uint64_t xs = exact_scratch_bytes(j);
-  if (j->d_chunk && j->chunk_cap >= cap && j->chunk_rec_elems >= rec && j->chunk_exact_bytes >= xs) return RS_OK;
+  const uint32_t ncand = j->has_cta() ? (uint32_t)std::min<uint64_t>((uint64_t)cap * kCandPerPrime, 1u << 30) : 0;
+  if (j->d_chunk && j->chunk_cap >= cap && j->chunk_rec_elems >= rec && j->chunk_exact_bytes >= xs && j->cb.cand_cap >= ncand)
+    return RS_OK;
   if (j->d_chunk) cudaFreeAsync(j->d_chunk, j->st);
   j->d_chunk = nullptr;
   size_t off = 0;
@@ -1146,7 +1186,7 @@ static int ensure_chunk_buffers(rs_job *j, uint32_t cap) {
     return o;
   };
   const size_t o_pr = sec((size_t)cap * 8), o_ct = sec(16), o_rec = sec((size_t)cap * 8 * rec);
-  const size_t o_rd = sec((size_t)cap * 4), o_rc = sec(16), o_xt = sec(xs);
+  const size_t o_rd = sec((size_t)cap * 4), o_rc = sec(16), o_xt = sec(xs), o_cd = sec((size_t)ncand * sizeof(Candidate));
   CUDA_TRY(cudaMallocAsync(&j->d_chunk, off, j->st));
   uint8_t *b = (uint8_t *)j->d_chunk;
   j->cb.primes = (uint64_t *)(b + o_pr);
@@ -1155,6 +1195,8 @@ static int ensure_chunk_buffers(rs_job *j, uint32_t cap) {
   j->cb.redo = (uint32_t *)(b + o_rd);
   j->cb.redo_count = (uint32_t *)(b + o_rc);
   j->cb.exact_tab = xs ? (uint32_t *)(b + o_xt) : nullptr;
+  j->cb.cand = ncand ? (Candidate *)(b + o_cd) : nullptr;
+  j->cb.cand_cap = ncand;
   j->cb.cap = cap;
   j->chunk_cap = cap;
   j->chunk_rec_elems = rec;
@@ -1426,12 +1468,9 @@ static StepForm chunk_step_form(const rs_job *j, const Part &pt, uint64_t a, uin
   const uint64_t bq = pt.dev.bq_small;
   StepForm f;
   f.pair_ok = a > (1ull << 33) && (unsigned __int128)pt.dev.base * b < ((unsigned __int128)1 << 63) ? 1u : 0u;
-  if (pt.dev.cta_warps > 1) {
-    const bool small_ok = bq != 0 && a > (1ull << 33) && (unsigned __int128)bq * b < ((unsigned __int128)1 << 63);
-    const bool high_ok = bq != 0 && (bq << 32) < a;
-    f.form = small_ok ? kStepSmall : high_ok ? kStepHigh : kStepShoup;
-    if (j->opt.baby_step == RS_BABY_SHOUP) f.form = kStepShoup;
-    else if (j->opt.baby_step == RS_BABY_HIGH && high_ok) f.form = kStepHigh;
+  if (j->opt.baby_step == RS_BABY_HIGH && pt.dev.cta_warps > 1 && short_step_valid(bq, a, b, 32)) {
+    f.form = kStepHigh;
+    f.shift = 32;
     return f;
   }
   if (j->opt.baby_step != RS_BABY_SHOUP && short_step_shift(bq, a, b, f.shift)) f.form = kStepSmall;
@@ -1570,13 +1609,13 @@ static int sieve_range_impl(rs_job *j, uint64_t p0, uint64_t p1, rs_factor *out,
         set_step(j->cb, form);
         if (ce) cudaEventRecord(ce[2 + 4 * q], j->st);
         e = launch_setup(pt.dev, j->cb, j->st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(j->cb.redo_count, 0, 4, j->st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(j->cb.redo_count, 0, 8, j->st);
         if (ce) cudaEventRecord(ce[3 + 4 * q], j->st);
         if (e == cudaSuccess) e = launch_bsgs(pt.dev, j->cb, pt.hb, pt.bsgs_grid, j->st);
         if (ce) cudaEventRecord(ce[4 + 4 * q], j->st);
         if (e == cudaSuccess) e = launch_bsgs_exact(pt.dev, j->cb, pt.hb, pt.exact_grid, j->st);
         if (ce) cudaEventRecord(ce[5 + 4 * q], j->st);
-        st.launches += 3;
+        st.launches += pt.dev.cta_warps > 1 ? 4 : 3;
         st.bsgs_launches += 1;
       }
       if (e != cudaSuccess) {
@@ -2085,7 +2124,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
       ChunkBufs cb = j->cb;
       set_step(cb, R.forms[rd]);
       launch_setup(R.pt->dev, cb, s);
-      cudaMemsetAsync(j->cb.redo_count, 0, 4, s);
+      cudaMemsetAsync(j->cb.redo_count, 0, 8, s);
       tot.launches += (j->nsp > j->nsp_small ? 2 : 1) + 1;
     }
     join(0);
@@ -2114,7 +2153,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
       set_step(cb, R.forms[rd]);
       launch_bsgs(R.pt->dev, cb, R.pt->hb, R.pt->bsgs_grid, s);
       launch_bsgs_exact(R.pt->dev, cb, R.pt->hb, R.pt->exact_grid, s);
-      tot.launches += 2;
+      tot.launches += R.pt->dev.cta_warps > 1 ? 3 : 2;
       tot.bsgs_launches++;
     }
     join(1);
@@ -2494,6 +2533,7 @@ int rs::job_footprint(const char *text, size_t len, const rs_options &opt, JobFo
   *fp = JobFootprint{};
   fp->parts = (uint32_t)groups.size();
   uint32_t rec = 0;
+  bool cta = false;
   for (Seqs &g : groups) {
     normalise(g);
     Plan pl;
@@ -2501,8 +2541,9 @@ int rs::job_footprint(const char *text, size_t len, const rs_options &opt, JobFo
     if (rc) return rc;
     fp->arrays += part_array_bytes(pl, g, opt.datless != 0);
     rec = std::max(rec, record_el_tab(pl, plan_row_form(pl, g, nullptr)) + 64);
+    cta = cta || pl.cta;
   }
-  fp->per_prime = 8 + 4 + 8 * (uint64_t)rec;
+  fp->per_prime = 8 + 4 + 8 * (uint64_t)rec + (cta ? kCandPerPrime * sizeof(Candidate) : 0);
   return RS_OK;
 }
 

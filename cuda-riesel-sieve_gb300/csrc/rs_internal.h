@@ -10,8 +10,7 @@
 
 namespace rs {
 
-// CTA kernel: per-prime hash of 16-bit tags, kBucket tags per 16-byte bucket.
-constexpr int kBucket = 8;
+constexpr int kBucket = 8;          // 16-bit table slots in the planner's unit of table size
 constexpr int kMatchCap = 64;       // warp kernel: a prime with more suspects takes the exact path
 // BSGS exact path (rare primes): 32-bit entries (tag << jbits) | j, linear probing.
 // j <= m-1 <= 2^jbits - 2, so a real entry is never all ones.
@@ -37,6 +36,7 @@ constexpr uint32_t kNoTable = 0xffffffffu;  // no quadratic-character table for 
 //   6,7 B in normal form and its Shoup constant (the chain step),
 //   8,9 B^(32W*chain_len) likewise (chain t -> chain t+32W), 10,11 G^32 likewise,
 //   W > 1 only: 12.. B^(32w*chain_len) for w < W likewise (pairs; warp w's offset),
+//   then b likewise,
 //   el_v.. V[max_act] (giant-step start per active row), el_row.. row ids (u16,
 //   4 per element), el_tab.. B^(lane*chain_len) (32 elements, the chain starts
 //   of warp 0), el_tab+32.. G^(lane % tlanes + 1) (32 elements).
@@ -69,7 +69,7 @@ constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3;
 constexpr uint32_t kMaskRows = 64;  // rows a row_mask record can describe
 constexpr int kCtaWarps = 16;      // warps sharing one prime in the CTA-per-prime kernel
 constexpr uint32_t kCtaSmemMax = 232448;  // shared memory a CTA may opt into (227 KB)
-constexpr int kCtaMatchCap = 64;   // deferred tag matches per prime there
+constexpr int kCtaMatchCap = 64;   // suspects per prime there; a prime with more takes the exact path
 
 // Per-k data of the setup kernel's row loop, 32 bytes: odd part of k, its 2-adic
 // valuation, the offset of its character table (kNoTable if none), k, its first
@@ -109,9 +109,10 @@ struct JobDev {
   uint32_t tlanes;       // min(T, 32): lanes sharing one row
   uint32_t rows_per_it;  // 32 / tlanes
   uint32_t steps_per_lane;  // max(1, T / 32)
-  uint32_t fwords;       // warp kernel: 32-bit words of a prime's filter (a multiple of 4)
+  uint32_t fwords;       // 32-bit words of a prime's filter (a multiple of 4)
   uint32_t fshift;       // low bits of a key that do not choose the filter word (11..16)
-  uint32_t nbuckets;     // CTA kernel: fast-path buckets per prime (any multiple of 64)
+  uint32_t edge_lim;     // CTA kernel: keys this close above a field's multiple are stored twice (baby_filter)
+  uint32_t row_slots;    // CTA kernel: slots of the residues' row lists (a multiple of 8)
   uint32_t jbits;        // bits of j in an exact-path table entry
   uint32_t nrows, nk;
   int64_t e0;            // x = e0 + m*s - j for giant index s in [1, T]
@@ -128,11 +129,14 @@ struct JobDev {
   uint32_t warp_smem;    // shared-memory bytes per warp (bsgs_kernel) or per CTA (bsgs_cta_kernel)
   uint32_t exact_log2;   // slots of the exact kernel's table = 1 << exact_log2
   uint32_t exact_global; // that table exceeds shared memory: it lives in ChunkBufs::exact_tab
-  uint32_t ctab_smem;    // CTA kernel, row ids: the table k*b^r of every row is copied into shared memory
+  uint32_t ctab_smem;    // CTA kernel: the k of the active rows are kept in shared memory beside their ids
   // device arrays
   const uint32_t *row_r;     // [nrows] n mod Q of each row
   const uint32_t *row_kidx;  // [nrows] index of the row's k
-  const uint32_t *row_c;     // [nrows] k*b^r (meaningful when int_rows)
+  const uint32_t *row_c;     // [nrows] k*b^r (warp layout, meaningful when int_rows)
+  const uint32_t *row_k;     // [nrows] k of each row
+  const uint32_t *row_base;  // [Q] first slot of each residue's row list (multiples of 4)
+  const uint2 *row_kr;       // [nrows] k, and residue r (12 bits) | first slot of its list << 12 (CTA layout)
   const uint32_t *k_val;     // [nk]
   const uint32_t *k_odd;     // [nk] odd part of k
   const uint32_t *k_e2;      // [nk] 2-adic valuation of k
@@ -153,13 +157,23 @@ struct Hit {
   uint32_t n;
 };
 
+// A tag match of the CTA kernel: giant value y (normal form), the prime's index,
+// row and giant index, and the thread whose chains hold the tag.
+struct Candidate {
+  uint64_t y;
+  uint32_t i, row, s, thread;
+};
+constexpr uint32_t kCandPerPrime = 8;  // room per prime of a chunk (about 3 are used on the wide job)
+
 // Buffers of one chunk of primes.
 struct ChunkBufs {
   uint64_t *primes;     // [cap]
   uint32_t *count;      // [1] primes found by the sieve (may exceed cap)
   uint64_t *recs;       // [cap * rec_elems] records
   uint32_t *redo;       // [cap] primes handed to the exact BSGS kernel
-  uint32_t *redo_count; // [1]
+  uint32_t *redo_count; // [2] redo entries, candidates
+  Candidate *cand;      // [cand_cap] CTA layout: tag matches for settle_kernel (else null)
+  uint32_t cand_cap;
   uint32_t *exact_tab;  // exact-kernel tables of jobs whose table exceeds shared memory (else null)
   uint32_t cap;
   // The baby step of the chunk: kStepSmall (the short product by the integer

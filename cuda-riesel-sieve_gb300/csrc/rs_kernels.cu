@@ -288,10 +288,10 @@ __global__ void __launch_bounds__(128) setup_kernel(JobDev J, ChunkBufs cb) {
     // value t of the G table is G^(t % tlanes + 1): the chain restarts at G
     // whenever t % tlanes wraps to 0 (tlanes divides 32)
     const uint64_t Gw = from_mont(G, p, M.pinv), Gq = shoup_const(G, M.pinv);
-    // integer rows: the table holds Z_(t+1) = +-lambda*B^e0 * G^(t+1) instead (times 2^128 for the CTA kernel)
+    // integer rows: the table holds Z_(t+1) = +-lambda*B^e0 * G^(t+1) instead
     uint64_t g0 = G;
     if (J.int_rows) {
-      uint64_t h2 = J.cta_warps > 1 ? montmul(H, r2, M) : H;
+      uint64_t h2 = H;
       if (J.sign > 0 && h2) h2 = p - h2;
       g0 = shoup_mul(h2, Gw, Gq, p);
     }
@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(128) setup_kernel(JobDev J, ChunkBufs cb) {
       o = montmul(o, Bs, M);
     }
     off = o;  // B^(32W*c)
+    rec_st2(rec, kElWoff + 2 * J.cta_warps, bmod, bq);  // b and its Shoup constant
   }
   rec_st2(rec, kElOfw, from_mont(off, p, M.pinv), shoup_const(off, M.pinv));
 }
@@ -588,187 +589,15 @@ __device__ __forceinline__ uint32_t nth_row(uint64_t mask, uint32_t n) {
 }
 
 struct __align__(16) Match {
-  uint64_t y;     // giant-step value whose tag matched
-  uint32_t slot;  // active-row slot
+  uint64_t y;     // giant value (normal form)
+  uint32_t row;   // its row
   uint32_t s;     // giant index
 };
-
-// 16-bit tag of a residue: the high half of its low word (the bucket index
-// uses the low log2(NB) <= 16 bits), raised to 1 if 0 (0 marks an empty slot).
-// tag_pair gives it in both halves, t*0x10001: the high half copied to both
-// halves, each raised to at least 1; its low half is the tag itself.
-__device__ __forceinline__ uint32_t tag_pair(uint32_t lo) { return __vmaxu2(__byte_perm(lo, 0, 0x3232), 0x00010001u); }
 
 // Nonzero iff some 16-bit half of x is zero: (x - 0x10001) & ~x sets bit 15 of
 // the low half iff it is zero, and bit 15 of the high half iff it is zero or
 // the low half borrowed (which only happens when the low half is zero).
 __device__ __forceinline__ uint32_t zero_half(uint32_t x) { return (x - 0x00010001u) & ~x & 0x80008000u; }
-
-// Bucket layout: 16 bytes = eight 16-bit tags (0 = empty).  True iff one of
-// the 8 tags equals the tag pair T = t*0x10001.
-__device__ __forceinline__ bool bucket_has(const uint4 &q, uint32_t T) {
-  return zero_half(__vminu2(__vminu2(q.x ^ T, q.y ^ T), __vminu2(q.z ^ T, q.w ^ T))) != 0;
-}
-
-constexpr uint32_t kSlots = 8;  // tag slots per bucket
-
-// Hash-table view of a prime's shared memory: NB buckets of tags and NB 32-bit
-// insert counts, kept apart from the buckets so that the counts of a warp's 32
-// random buckets spread over all 32 banks.  An insert takes slot c of its
-// bucket from an atomic add on the bucket's count and writes its tag there with
-// a plain 16-bit store.  Slots fill in order, so a bucket is full iff its slot 7
-// holds a tag, and an entry overflows into the next bucket only when its bucket
-// is full: a probe scans from the home bucket to the first bucket that is not
-// full.  The home bucket comes from the low 16 bits of a residue's low word and
-// the tag from the high 16 bits: the low bits masked when NB is a power of two
-// (MUL false), else scaled, (lo16 * NB) >> 16 (MUL true; any NB <= 65536), which
-// lets a CTA size its table to its shared memory instead of to a power of two.
-//
-// SIG: the bucket's count word also holds a 16-bit signature of its entries:
-// the count in bits 0-15 (a bucket sees at most one increment per baby step,
-// and the planner keeps CTA plans below 2^16 baby steps, so it never carries
-// out), and bit 16 + sig(v) set (atomic OR) for every entry v
-// stored there, sig(v) a 4-bit hash of v's high word.  A tag match counts only
-// if the bucket holding the tag has the signature bit of the probed value, so
-// with ~2 entries a bucket ~88% of the false 16-bit matches are rejected
-// before they cost a pass over the baby steps; a true match always has its bit.
-template <bool MUL, bool SIG = false>
-struct TableT {
-  uint4 *tab4;
-  uint16_t *tab16;
-  uint32_t *cnt32;
-  uint32_t nb;     // buckets
-  uint32_t bmask;  // nb - 1 (MUL false)
-
-  __device__ __forceinline__ uint32_t home(uint32_t lo) const {
-    return MUL ? (uint32_t)(((lo & 0xffffu) * nb) >> 16) : (lo & bmask);
-  }
-  __device__ __forceinline__ uint32_t next(uint32_t b) const {
-    return MUL ? (b + 1 == nb ? 0u : b + 1) : ((b + 1) & bmask);
-  }
-  __device__ __forceinline__ static uint32_t sig_bit(uint64_t v) {
-    return 1u << (16 + ((uint32_t)(v >> 32) * 0x9E3779B1u >> 28));
-  }
-
-  __device__ __forceinline__ uint32_t take(uint32_t b) const {
-    const uint32_t c = atomicAdd(&cnt32[b], 1u);
-    return SIG ? c & 0xffffu : c;
-  }
-  __device__ __forceinline__ void store(uint64_t v, uint32_t b, uint32_t c) const {
-    tab16[b * kSlots + c] = (uint16_t)tag_pair((uint32_t)v);
-    if (SIG) atomicOr(&cnt32[b], sig_bit(v));
-  }
-
-  // Insert continuing after bucket b, whose slots are all taken.
-  __device__ __forceinline__ void insert_after(uint64_t v, uint32_t b) const {
-    uint32_t c = kSlots;
-#pragma unroll 1
-    for (uint32_t g = 0; c >= kSlots && g + 1 < nb; g++) {
-      b = next(b);
-      c = take(b);
-    }
-    if (c < kSlots) store(v, b, c);
-  }
-
-  // Insert into the home bucket; false if it was full (the caller finishes the
-  // insert later with insert_after, keeping the rare overflow off the hot loop).
-  __device__ __forceinline__ bool insert_home(uint64_t v) const {
-    const uint32_t b = home((uint32_t)v);
-    const uint32_t c = take(b);
-    if (c < kSlots) store(v, b, c);
-    return c < kSlots;
-  }
-
-  // Home-bucket test: true if the tag of y is in y's home bucket or that bucket
-  // is full (then only probe() can tell).
-  __device__ __forceinline__ bool probe_home(uint64_t y) const {
-    const uint32_t lo = (uint32_t)y;
-    const uint4 q = tab4[home(lo)];
-    const uint32_t T = tag_pair(lo);
-    const uint32_t m = __vminu2(__vminu2(q.x ^ T, q.y ^ T), __vminu2(q.z ^ T, q.w ^ T));
-    return (zero_half(m) | (q.w & 0xffff0000u)) != 0;  // a tag match, or slot 7 taken
-  }
-
-  // True iff some entry with the tag of y (and, SIG, the signature bit of y)
-  // lies in y's probe sequence.
-  __device__ __forceinline__ bool probe(uint64_t y) const {
-    const uint32_t lo = (uint32_t)y;
-    uint32_t b = home(lo);
-    const uint32_t T = tag_pair(lo);
-    const uint32_t sb = SIG ? sig_bit(y) : 0u;
-    auto has = [&](const uint4 &q, uint32_t bk) { return bucket_has(q, T) && (!SIG || (cnt32[bk] & sb)); };
-    uint4 q = tab4[b];
-    bool hit = has(q, b);
-    if (q.w >= 0x10000u) {  // the home bucket is full, continue scanning
-#pragma unroll 1
-      for (uint32_t g = 0; g + 1 < nb; g++) {
-        b = next(b);
-        q = tab4[b];
-        hit |= has(q, b);
-        if (q.w < 0x10000u) break;
-      }
-    }
-    return hit;
-  }
-};
-
-struct MatchList {
-  Match *list;
-  uint32_t *count;
-  uint32_t cap;  // matches the list holds; the baby phase's overflow values use the same space (2*cap)
-  // Baby-phase use of the same space: up to 2*cap values to insert late.
-  __device__ __forceinline__ void append(uint64_t *ovf, uint64_t v) const {
-    const uint32_t idx = atomicAdd(count, 1u);
-    if (idx < 2 * cap) ovf[idx] = v;
-  }
-  __device__ __forceinline__ void push(uint64_t y, uint32_t slot, uint32_t s) const {
-    const uint32_t idx = atomicAdd(count, 1u);
-    if (idx < cap) {
-      Match mt;
-      mt.y = y;
-      mt.slot = slot;
-      mt.s = s;
-      list[idx] = mt;
-    }
-  }
-};
-
-// One chain step: the product by B, as Shoup's product by the full-size
-// constant or, when the chunk allows it, as the short product by the integer b^Q.
-struct StepShoup {
-  uint64_t w, wq, p;
-  __device__ __forceinline__ uint64_t operator()(uint64_t x) const { return shoup_mul(x, w, wq, p); }
-};
-struct StepSmall {
-  uint32_t c, rc;
-  uint64_t p;
-  __device__ __forceinline__ uint64_t operator()(uint64_t x) const { return mul_small(x, c, rc, p); }
-};
-// b^Q * 2^32 < p (large primes): Shoup's product with a 32-bit constant.
-struct StepHigh {
-  uint32_t w, wq;
-  uint64_t p;
-  __device__ __forceinline__ uint64_t operator()(uint64_t x) const { return shoup_mul_w32(x, w, wq, p); }
-};
-
-// Baby steps of one lane: two chains of `len` steps from va and vb, of which
-// the first na (nb) are inserted (all of them when FULL).  A value whose home bucket is full is
-// appended to ovf and inserted after the loop.
-template <bool FULL, class Step, class Table>
-__device__ __forceinline__ void baby_chains(const Table &W, const MatchList &ML, uint64_t *ovf, uint64_t va,
-                                            uint64_t vb, uint32_t na, uint32_t nb, uint32_t len, const Step &step) {
-#pragma unroll 4
-  for (uint32_t t = 0; t < len; t++) {
-    const bool fa = (!FULL && t >= na) || W.insert_home(va);
-    const bool fb = (!FULL && t >= nb) || W.insert_home(vb);
-    if (!(fa && fb)) {
-      if (!fa) ML.append(ovf, va);
-      if (!fb) ML.append(ovf, vb);
-    }
-    va = step(va);
-    vb = step(vb);
-  }
-}
 
 // Fractions.  The filter's keys are fractions of residues: for a Montgomery-form
 // residue u of y (u = y*2^64 mod p), u * (-p^-1) mod 2^64 = floor(y*2^64/p), the
@@ -821,62 +650,82 @@ struct LazyShort {
 // benchmark job at 1e13 a baby step (short product, key, insert) takes 38 cycles
 // against 36 for the reduced product and a bucket insert, and a giant step
 // (key, probe) 28 against 50: 2.13 ns per prime against 2.82.
-constexpr uint32_t kFiltA = 0x22009u, kFiltB = 0x2100005u;
+constexpr uint32_t kFilt2A = 0x22009u, kFilt2B = 0x2100005u;
+// The CTA kernel probes ~64,000 values a prime: three five-bit fields (sh1, sh1 -
+// 5, sh1 - 10) and rotations, 1.6e-4 false positives at 0.35 values a word.
+constexpr uint32_t kFilt3A = 0x800081u, kFilt3B = 0x80005u, kFilt3C = 0x40041u;
 __device__ __forceinline__ uint32_t rotl(uint32_t v, uint32_t s) { return __funnelshift_l(v, v, s); }
 
+template <int K>
 struct Filter {
   uint32_t *w;
   uint32_t mul;  // words << sh1
-  uint32_t sh1, sh2;
+  uint32_t sh1;
+  __device__ __forceinline__ uint32_t low() const { return sh1 - 5 * (K - 1); }  // bits below the last field
+  __device__ __forceinline__ uint32_t bits(uint32_t u, uint32_t F) const {
+    return K == 2 ? rotl(kFilt2A, u) | rotl(kFilt2B, F >> (sh1 - 5))
+                  : rotl(kFilt3A, u) | rotl(kFilt3B, F >> (sh1 - 5)) | rotl(kFilt3C, F >> (sh1 - 10));
+  }
   __device__ __forceinline__ void add(uint32_t F) const {
     const uint32_t u = F >> sh1;
-    atomicOr(&w[__umulhi(u, mul)], rotl(kFiltA, u) | rotl(kFiltB, F >> sh2));
+    atomicOr(&w[__umulhi(u, mul)], bits(u, F));
   }
   __device__ __forceinline__ bool test(uint32_t f) const {
     const uint32_t u = f >> sh1;
-    return (~w[__umulhi(u, mul)] & (rotl(kFiltA, u) | rotl(kFiltB, f >> sh2))) == 0;
+    return (~w[__umulhi(u, mul)] & bits(u, f)) == 0;
   }
 };
 
 // Baby steps of one lane: two chains of `len` steps from va and vb, of which
 // the first na (nb) count (all of them when FULL) and go into the filter.  The
 // low 16 bits of both values' keys of step t are kept in tags[t * stride] for
-// the suspects' scan.  zmask: the low sh2 bits of both halves.  The key is that
-// of F64 + 1, which is exact for the unreduced residue and differs from the
-// reduced one's only where the fraction's low word is all ones, where no giant
-// step sees F - 1.
-template <bool FULL, class Step>
-__device__ __forceinline__ void baby_filter(const Filter &F, uint32_t *tags, uint32_t stride, uint32_t zmask,
+// the suspects' scan.  The key is that of F64 + 1, which is exact for the
+// unreduced residue and differs from the reduced one's only where the fraction's
+// low word is all ones, where no giant step sees F - 1.
+// A giant step sees F - 1 under another key only if F64 is less than cmax (the
+// largest integer row) above a multiple of 2^(32 + low()): those are stored
+// for F - 1 too.  With many low bits (EDGE false) it is enough to look at them:
+// lim has them in both halves; else (EDGE) lim is the bound for F64's 32 bits
+// below the last field.  The test is made for groups of N steps, since a branch
+// a step costs a fifth of the loop.
+template <bool FULL, bool EDGE, uint32_t N, int K, class Step>
+__device__ __forceinline__ void baby_filter(const Filter<K> &F, uint32_t *tags, uint32_t stride, uint32_t lim,
                                             uint64_t va, uint64_t vb, uint32_t na, uint32_t nb, uint32_t len,
                                             uint64_t pinv, const Step &step) {
-  const uint32_t low = zmask & 0xffffu;
   auto group = [&](auto count, uint32_t t0) {
-    constexpr uint32_t N = decltype(count)::value;
-    uint32_t fa[N], fb[N], z = 0xffffffffu;
+    constexpr uint32_t M = decltype(count)::value;
+    uint32_t fa[M], fb[M], ga[M], gb[M], z = 0xffffffffu;
 #pragma unroll
-    for (uint32_t i = 0; i < N; i++) {
+    for (uint32_t i = 0; i < M; i++) {
       const uint32_t t = t0 + i;
-      fa[i] = (uint32_t)((frac64(va, pinv) + 1) >> 32);
-      fb[i] = (uint32_t)((frac64(vb, pinv) + 1) >> 32);
+      const uint64_t xa = frac64(va, pinv) + 1, xb = frac64(vb, pinv) + 1;
+      fa[i] = (uint32_t)(xa >> 32);
+      fb[i] = (uint32_t)(xb >> 32);
       if (FULL || t < na) F.add(fa[i]);
       if (FULL || t < nb) F.add(fb[i]);
       const uint32_t tp = __byte_perm(fa[i], fb[i], 0x5410);
       tags[t * stride] = tp;
-      z = __vminu2(z, tp & zmask);
+      if (EDGE) {
+        ga[i] = __funnelshift_l((uint32_t)xa, fa[i], 32 - F.low());
+        gb[i] = __funnelshift_l((uint32_t)xb, fb[i], 32 - F.low());
+        z = min(z, min(ga[i], gb[i]));
+      } else {
+        z = __vminu2(z, tp & lim);
+      }
       va = step(va);
       vb = step(vb);
     }
-    if (zero_half(z)) {  // rare: a key whose low bits are zero
+    if (EDGE ? z < lim : zero_half(z) != 0) {  // rare
 #pragma unroll
-      for (uint32_t i = 0; i < N; i++) {
-        if ((fa[i] & low) == 0) F.add(fa[i] - 1);
-        if ((fb[i] & low) == 0) F.add(fb[i] - 1);
+      for (uint32_t i = 0; i < M; i++) {
+        if (EDGE ? ga[i] < lim : (fa[i] & lim & 0xffffu) == 0) F.add(fa[i] - 1);
+        if (EDGE ? gb[i] < lim : (fb[i] & lim & 0xffffu) == 0) F.add(fb[i] - 1);
       }
     }
   };
   uint32_t t = 0;
 #pragma unroll 1
-  for (; t + 6 <= len; t += 6) group(std::integral_constant<uint32_t, 6>{}, t);
+  for (; t + N <= len; t += N) group(std::integral_constant<uint32_t, N>{}, t);
 #pragma unroll 1
   for (; t + 2 <= len; t += 2) group(std::integral_constant<uint32_t, 2>{}, t);
   if (t < len) group(std::integral_constant<uint32_t, 1>{}, t);
@@ -950,7 +799,7 @@ __device__ __forceinline__ bool exact_key(uint64_t y, uint32_t f, uint64_t p, ui
 // PAIRED (RPI == 1, V rows): slots g, g+1 hold a (k, 0), (k, 1) pair, so the
 // second value is the first times the integer b (the short product).
 template <uint32_t RPI, int RM, bool PAIRED = false>
-__device__ __forceinline__ void giant_test(const Filter &F, const void *src, const uint32_t *__restrict__ ctab,
+__device__ __forceinline__ void giant_test(const Filter<2> &F, const void *src, const uint32_t *__restrict__ ctab,
                                            uint32_t g0, uint32_t g1, uint32_t nact, uint32_t lane_row,
                                            const GiantMul &G, uint64_t np, uint64_t pinv, uint32_t &hA, uint32_t &hB,
                                            uint32_t b = 0, uint32_t rc = 0) {
@@ -1037,12 +886,11 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
   // they multiply stay in Montgomery form, so products stay comparable.
   const uint64_t Stw = cur[kElStw], Stq = cur[kElStq];
   const uint64_t np = 0 - p;
-  Filter F;
+  Filter<2> F;
   F.w = fwords;
   F.sh1 = J.fshift;
-  F.sh2 = J.fshift - 5;
   F.mul = nw << J.fshift;
-  const uint32_t zmask = 0x10001u * ((1u << (J.fshift - 5)) - 1u);
+  const uint32_t lim = 0x10001u * ((1u << F.low()) - 1u);
   // chain starts B^(lane*CL) and B^((lane+32)*CL); valid steps na, nb (j < m)
   const uint32_t CL = J.chain_len;
   const uint32_t ja0 = lane * CL, jb0 = ja0 + 32 * CL;
@@ -1057,9 +905,9 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
   // Baby steps: chain A owns j = ja0 + t, chain B j = jb0 + t.
   auto baby = [&](auto step) {
     if (J.m == 64 * CL)  // every chain full (the planner's usual choice of m)
-      baby_filter<true>(F, tags, 32, zmask, Bl, Blb, na, nb, CL, pinv, step);
+      baby_filter<true, false, 6>(F, tags, 32, lim, Bl, Blb, na, nb, CL, pinv, step);
     else
-      baby_filter<false>(F, tags, 32, zmask, Bl, Blb, na, nb, CL, pinv, step);
+      baby_filter<false, false, 6>(F, tags, 32, lim, Bl, Blb, na, nb, CL, pinv, step);
   };
   if (cb.small_step == kStepShoup) baby(LazyShoup{Stw, Stq, np});
   else baby(LazyShort{J.bq_small, (uint32_t)(Stq >> (32 - cb.step_shift)), cb.step_shift, np});
@@ -1382,243 +1230,262 @@ int bsgs_smem_bytes(const JobDev &job) {
   return job.cta_warps > 1 ? (int)job.warp_smem : kWarpsPerBlock * (int)job.warp_smem;
 }
 
-// Giant steps of the CTA kernel: warp w takes row slots w, w + W, ..., four at
-// a time (four independent product chains per lane).  The loop tests home
-// buckets only and records the outcome as bits (step u of slot k -> bit 4u + k,
-// spl <= 8); tag hits and full buckets are finished after each pass.  RM: vst
-// holds V (kRowsV), the integers k*b^r (kRowsIntV) or 16-bit row ids whose
-// k*b^r come from the job's table ctab (kRowsIntId; CS: ctab is the CTA's
-// shared-memory copy of it).  TWO (integer rows, spl == 2): the
-// second value of a slot is also c times a lane multiplier, Z advanced by G^32
-// (Glw2, Glq2), so both products are independent short ones.
-template <int RM, bool TWO, bool CS, class Table>
-__device__ __forceinline__ void cta_giants(const Table &W, const MatchList &ML, const uint64_t *vst, uint32_t nact,
-                                           uint32_t warp, uint32_t lane, uint32_t spl, uint64_t Glw, uint64_t Glq,
-                                           uint64_t Gw, uint64_t Gq, uint64_t p, const uint32_t *__restrict__ ctab,
-                                           uint64_t Glw2 = 0, uint64_t Glq2 = 0) {
-  const uint16_t *rid = reinterpret_cast<const uint16_t *>(vst);
-  auto row_c = [&](uint32_t r) -> uint32_t { return CS ? ctab[r] : __ldg(ctab + r); };
+// Giant steps of the CTA kernel for one residue r: warp w takes groups w, w + W,
+// ... of four of the n active rows (ks: their k, or rid and the job's row_k),
+// multiplied by the lane's Z*b^r for one or two steps u (G0, G1).  Suspects are
+// listed as they are found.
+template <bool KS, bool TWO>
+__device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint32_t *keys, uint32_t *count,
+                                           const uint32_t *ks, const uint16_t *rid, const uint32_t *__restrict__ row_k,
+                                           uint32_t n, uint32_t warp, const GiantMul &G0, const GiantMul &G1,
+                                           uint32_t s0) {
 #pragma unroll 1
-  for (uint32_t s0 = warp; s0 < nact; s0 += 4 * kCtaWarps) {
-    uint64_t y[4];
+  for (uint32_t g = 4 * warp; g < n; g += 4 * kCtaWarps) {
     uint32_t c[4];
-    uint32_t valid = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < 4; k++) {
-      const uint32_t sl = s0 + k * kCtaWarps;
-      valid |= (sl < nact ? 0x11111111u : 0u) << k;
-      if (RM == kRowsIntId) {
-        c[k] = row_c(rid[sl < nact ? sl : s0]);
-        y[k] = shoup_mul32(c[k], Glw, Glq, p);
-      } else if (RM == kRowsIntV) {
-        c[k] = (uint32_t)vst[sl < nact ? sl : s0];
-        y[k] = shoup_mul32(c[k], Glw, Glq, p);
-      } else {
-        y[k] = shoup_mul(vst[sl < nact ? sl : s0], Glw, Glq, p);
-      }
-    }
-    uint32_t bits = 0;
-    if (TWO) {
-      uint64_t z[4];
-#pragma unroll
-      for (uint32_t k = 0; k < 4; k++) z[k] = shoup_mul32(c[k], Glw2, Glq2, p);
-#pragma unroll
-      for (uint32_t k = 0; k < 4; k++) {
-        if (W.probe_home(y[k])) bits |= 1u << k;
-        if (W.probe_home(z[k])) bits |= 1u << (4 + k);
-      }
+    if (KS) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(ks + g);
+      c[0] = v.x, c[1] = v.y, c[2] = v.z, c[3] = v.w;
     } else {
-#pragma unroll 1
-      for (uint32_t u = 0;; u++) {
 #pragma unroll
-        for (uint32_t k = 0; k < 4; k++)
-          if (W.probe_home(y[k])) bits |= 1u << (4 * u + k);
-        if (u + 1 >= spl) break;
-#pragma unroll
-        for (uint32_t k = 0; k < 4; k++) y[k] = shoup_mul(y[k], Gw, Gq, p);
-      }
+      for (uint32_t i = 0; i < 4; i++) c[i] = __ldg(row_k + rid[min(g + i, n - 1)]);
     }
-    bits &= valid;
-    while (bits) {  // rare
-      const uint32_t b = __ffs(bits) - 1;
-      bits &= bits - 1;
-      const uint32_t k = b & 3, u = b >> 2, sl = s0 + k * kCtaWarps;
-      uint64_t v = RM == kRowsIntId  ? shoup_mul32(row_c(rid[sl]), Glw, Glq, p)
-                   : RM == kRowsIntV ? shoup_mul32((uint32_t)vst[sl], Glw, Glq, p)
-                                     : shoup_mul(vst[sl], Glw, Glq, p);
+    uint32_t hit = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+      if (F.test(giant_key<kRowsIntV>(c[i], G0, 0, 0, 0))) hit |= 1u << i;
+      if (TWO && F.test(giant_key<kRowsIntV>(c[i], G1, 0, 0, 0))) hit |= 16u << i;
+    }
+    if (hit) {  // rare
 #pragma unroll 1
-      for (uint32_t q = 0; q < u; q++) v = shoup_mul(v, Gw, Gq, p);
-      if (W.probe(v)) ML.push(v, sl, lane + 1 + 32 * u);
+      for (uint32_t i = 0; i < 8; i++) {
+        const uint32_t sl = g + (i & 3);
+        if (!((hit >> i) & 1u) || sl >= n) continue;
+        const GiantMul &G = i & 4 ? G1 : G0;
+        const uint32_t k = KS ? ks[sl] : __ldg(row_k + rid[sl]);
+        const uint64_t y = giant_exact<kRowsIntV>(k, G);
+        uint32_t f;
+        const bool edge = exact_key<kRowsIntV>(y, giant_key<kRowsIntV>(k, G, 0, 0, 0), G.p, 0, f);
+        // (edge: a baby step may be stored under the next key)
+        const uint32_t idx = atomicAdd(count, edge ? 2u : 1u);
+        for (uint32_t e = 0; e <= (uint32_t)edge; e++)
+          if (idx + e < (uint32_t)kCtaMatchCap) {
+            list[idx + e] = Match{y, rid[sl], s0 + (i & 4 ? 32 : 0)};
+            keys[idx + e] = f + e;
+          }
+      }
     }
   }
 }
 
-// The CTA-per-prime kernel, for jobs whose best baby-step count needs a table
+// The CTA-per-prime kernel, for jobs whose best baby-step count needs a filter
 // larger than a warp's share of shared memory (many k, wide n ranges).  All
 // kCtaWarps warps of a CTA work on one prime: thread t runs baby chains t and
-// t + 32W into one table that fills most of the SM's shared memory, and warp w
-// takes the giant steps of row slots w, w + W, ... (32 lanes per row, T/32
-// steps per lane).  Shared memory:
-//   [NB buckets x 16 B][NB count words x 4 B: insert count, entries' signature]
-//   [V, max_act x 8 B][kCtaMatchCap matches][count, 16 B]([row table, nrows x 4 B])
-// The row table (row ids only, when it fits) is copied once per launch.
-// V is staged with cp.async during the baby steps.  Table operations, the
-// deferred overflow inserts and the exact tag-match resolution are those of
-// bsgs_kernel; hits are pushed where they are found (tag matches are rare).
-template <int RM, bool MUL>
+// t + 32W into one filter that fills most of the SM's shared memory; the active
+// rows are sorted by their residue r, and for each r the warps share the rows
+// (32 lanes per row, T/32 steps per lane) with the lane's multiplier Z*b^r, so
+// that every row is the integer k.  Shared memory:
+//   [filter, fwords x 4 B][tags, 32W x chain_len x 4 B][k of the active rows,
+//   row_slots x 4 B (when it fits: KS)][their row ids, row_slots x 2 B]
+//   [kCtaMatchCap suspects][their keys][rows per residue, Q x 4 B][count, 16 B]
+// What bounds it is the integer pipes, as the warp kernel, at four warps a
+// scheduler.  On the wide job (1000 k, T = 64) it takes 103 ns per prime against 156
+// with buckets of eight 16-bit tags, counts and signatures: giant steps 49 (one
+// high product, one multiply-add and a 4-byte probe instead of a 32-bit Shoup
+// product and a 16-byte probe), baby steps 19, suspects 18 (about 12 a prime),
+// clearing and row lists 17 (25 before the next prime's loads were moved
+// under the giant steps).
+template <bool KS>
 __global__ void __launch_bounds__(32 * kCtaWarps, 1) bsgs_cta_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
   extern __shared__ uint4 smem4[];
-  constexpr uint32_t G = 32 * kCtaWarps;
+  constexpr uint32_t T = 32 * kCtaWarps;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t NB = J.nbuckets;
-  uint8_t *base = reinterpret_cast<uint8_t *>(smem4);
-  TableT<MUL, true> W;
-  W.tab4 = reinterpret_cast<uint4 *>(base);
-  W.tab16 = reinterpret_cast<uint16_t *>(base);
-  W.cnt32 = reinterpret_cast<uint32_t *>(base + NB * 16);
-  W.nb = NB;
-  W.bmask = NB - 1;
-  uint64_t *vst = reinterpret_cast<uint64_t *>(base + NB * 20);
-  const uint32_t vst_elems = RM == kRowsIntId ? 2 * ((J.max_act + 7) / 8) : (J.max_act + 1) & ~1u;
-  MatchList ML;
-  ML.list = reinterpret_cast<Match *>(vst + vst_elems);
-  ML.count = reinterpret_cast<uint32_t *>(ML.list + kCtaMatchCap);
-  ML.cap = kCtaMatchCap;
-  uint64_t *ovf = reinterpret_cast<uint64_t *>(ML.list);
+  const uint32_t CL = J.chain_len, spl = J.steps_per_lane;
+  uint32_t *fwords = reinterpret_cast<uint32_t *>(smem4);
+  uint32_t *tags = fwords + J.fwords;
+  uint32_t *ks = tags + T * CL;
+  uint16_t *rid = reinterpret_cast<uint16_t *>(ks + (KS ? J.row_slots : 0));
+  Match *list = reinterpret_cast<Match *>(rid + J.row_slots);
+  uint32_t *keys = reinterpret_cast<uint32_t *>(list + kCtaMatchCap);
+  uint32_t *nrow = keys + kCtaMatchCap;
+  uint32_t *count = nrow + J.Q;
+  Filter<3> F;
+  F.w = fwords;
+  F.sh1 = J.fshift;
+  F.mul = J.fwords << J.fshift;
   const uint32_t total = *cb.count;
   const uint32_t n = total < cb.cap ? total : cb.cap;
-  const uint32_t CL = J.chain_len, spl = J.steps_per_lane;
-  const uint32_t ja0 = tid * CL, jb0 = (tid + G) * CL;  // the thread's chains; m == 2*G*CL
-  const uint32_t vdst = (uint32_t)__cvta_generic_to_shared(vst);
-  // the row table, copied once per launch (row ids, when it fits); the first
-  // barrier of the prime loop orders these stores before any read
-  uint32_t *cts = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(ML.count) + 16);
-  if (RM == kRowsIntId && J.ctab_smem)
-    for (uint32_t r = tid; r < J.nrows; r += G) cts[r] = __ldg(J.row_c + r);
+  const uint32_t ja0 = tid * CL, jb0 = (tid + T) * CL;  // the thread's chains; m == 2*T*CL
 
+  // What a prime needs first is loaded during the giant steps of the one before
+  // it: its header and the thread's first two row ids with their k and slots.
+  uint64_t np_ = 0, npinv = 0, nBl = 0;
+  uint32_t nn = 0, nid[2] = {0, 0};
+  uint2 nkr[2] = {};
+  auto fetch = [&](uint32_t i) {
+    const uint64_t *rec = cb.recs + (size_t)i * J.rec_elems;
+    nn = (uint32_t)rec[kElNact];
+    np_ = rec[kElP];
+    npinv = rec[kElPinv];
+    nBl = rec[J.el_tab + lane];
+    const uint16_t *ids = reinterpret_cast<const uint16_t *>(rec + J.el_row);
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) {
+      nid[h] = tid + h * T < nn ? ids[tid + h * T] : 0;
+      nkr[h] = __ldg(J.row_kr + nid[h]);
+    }
+  };
+  if (blockIdx.x < n) fetch(blockIdx.x);
 #pragma unroll 1
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint64_t *rec = cb.recs + (size_t)i * J.rec_elems;
-    const uint32_t nact = (uint32_t)rec[kElNact];
-    if (nact == 0) continue;
-    const uint64_t p = rec[kElP], pinv = rec[kElPinv];
-    __syncthreads();  // the previous prime is done with the table, V and the list
-    // V of the active rows (integer rows: their 16-bit row ids) into shared
-    // memory, 16 bytes per copy
-    constexpr bool IDS = RM == kRowsIntId;
-    const uint32_t vn = IDS ? 2 * ((nact + 7) / 8) : (nact + 1) & ~1u;
-    const uint64_t *vsrc = rec + (IDS ? J.el_row : J.el_v);
-#pragma unroll 1
-    for (uint32_t e = 2 * tid; e < vn; e += 2 * G)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(vdst + 8 * e), "l"(vsrc + e)
-                   : "memory");
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const uint32_t nact = nn;
+    if (nact == 0) {
+      if (i + gridDim.x < n) fetch(i + gridDim.x);
+      continue;
+    }
+    const uint64_t p = np_, pinv = npinv, np = 0 - p;
+    uint64_t Bl = nBl;
+    const uint64_t Stw = rec[kElStw], Stq = rec[kElStq];
+    const uint64_t ofw = rec[kElOfw], ofq = rec[kElOfq];
+    const uint64_t ww = rec[kElWoff + 2 * warp], wq = rec[kElWoff + 2 * warp + 1];
+    if (i + gridDim.x < n && 16 * tid < J.rec_elems)  // the next prime's record into L2
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + (size_t)gridDim.x * J.rec_elems + 16 * tid));
+    __syncthreads();  // the previous prime is done with shared memory
     const uint4 z4 = make_uint4(0, 0, 0, 0);
 #pragma unroll 4
-    for (uint32_t q = tid; q < NB + NB / 4; q += G) W.tab4[q] = z4;
-    if (tid == 0) *ML.count = 0;
+    for (uint32_t q = tid; q < J.fwords / 4; q += T) smem4[q] = z4;
+    for (uint32_t q = tid; q <= J.Q; q += T) nrow[q] = 0;  // and count
     __syncthreads();
+    // the active rows into their residues' lists (in any order): x the k, y the residue's first slot and r
+    auto place = [&](bool on, uint32_t id, uint2 kr) {
+      const uint32_t r = on ? kr.y & 0xfffu : 0xffffffffu;
+      const uint32_t same = __match_any_sync(0xffffffffu, r);
+      const int lead = __ffs(same) - 1;
+      uint32_t at = 0;
+      if (on && (int)lane == lead) at = atomicAdd(&nrow[r], __popc(same));
+      at = __shfl_sync(0xffffffffu, at, lead) + __popc(same & ((1u << lane) - 1u)) + (kr.y >> 12);
+      if (!on) return;
+      rid[at] = (uint16_t)id;
+      if (KS) ks[at] = kr.x;
+    };
+    if (32 * warp < nact) place(tid < nact, nid[0], nkr[0]);
+    if (32 * warp + T < nact) place(tid + T < nact, nid[1], nkr[1]);
+#pragma unroll 1
+    for (uint32_t a = tid + 2 * T; a < ((nact + 31) & ~31u); a += T) {
+      const uint32_t id = a < nact ? reinterpret_cast<const uint16_t *>(rec + J.el_row)[a] : 0;
+      place(a < nact, id, __ldg(J.row_kr + id));
+    }
 
     // Baby steps: chain starts B^(lane*c) times the warp's offset B^(32w*c)
-    uint64_t Bl = rec[J.el_tab + lane];
-    if (warp) Bl = shoup_mul(Bl, rec[kElWoff + 2 * warp], rec[kElWoff + 2 * warp + 1], p);
-    const uint64_t Blb = shoup_mul(Bl, rec[kElOfw], rec[kElOfq], p);
-    if (cb.small_step == kStepSmall)
-      baby_chains<true>(W, ML, ovf, Bl, Blb, CL, CL, CL, StepSmall{J.bq_small, (uint32_t)rec[kElRcp], p});
-    else if (cb.small_step == kStepHigh)
-      baby_chains<true>(W, ML, ovf, Bl, Blb, CL, CL, CL, StepHigh{J.bq_small, (uint32_t)rec[kElStq], p});
+    if (warp) Bl = shoup_mul(Bl, ww, wq, p);
+    const uint64_t Blb = shoup_mul(Bl, ofw, ofq, p);
+    if (cb.small_step == kStepShoup)
+      baby_filter<true, true, 4>(F, tags + tid, T, J.edge_lim, Bl, Blb, CL, CL, CL, pinv, LazyShoup{Stw, Stq, np});
     else
-      baby_chains<true>(W, ML, ovf, Bl, Blb, CL, CL, CL, StepShoup{rec[kElStw], rec[kElStq], p});
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      baby_filter<true, true, 4>(F, tags + tid, T, J.edge_lim, Bl, Blb, CL, CL, CL, pinv,
+                                 LazyShort{J.bq_small, (uint32_t)(Stq >> (32 - cb.step_shift)), cb.step_shift, np});
     __syncthreads();
-    const uint32_t novf = *ML.count;
-    if (novf > 2 * ML.cap) {  // pathological table: leave the prime to the exact path
+
+    // Giant steps, residue by residue: the multiplier's stored form E = Z*b^r
+    {
+      const uint64_t bw = rec[kElWoff + 2 * kCtaWarps], bq = rec[kElWoff + 2 * kCtaWarps + 1];
+      const uint64_t Gw = rec[kElGw], Gq = rec[kElGq];
+      uint64_t Er = rec[J.el_tab + 32 + lane];
+      if (i + gridDim.x < n) fetch(i + gridDim.x);
+#pragma unroll 1
+      for (uint32_t r = 0; r < J.Q; r++) {
+        const uint32_t nr = nrow[r];
+        if (nr) {
+          const uint32_t at = __ldg(J.row_base + r);
+          const uint32_t w = (warp + 5 * r) % kCtaWarps;  // uneven shares of several residues fall on different warps
+          uint64_t E = Er;
+#pragma unroll 1
+          for (uint32_t u = 0; u < spl; u += 2) {
+            GiantMul G0, G1;
+            G0.set(E, p, pinv);
+            G1 = G0;
+            if (u + 1 < spl) {
+              E = shoup_mul(E, Gw, Gq, p);
+              G1.set(E, p, pinv);
+              cta_giants<KS, true>(F, list, keys, count, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
+              if (u + 2 < spl) E = shoup_mul(E, Gw, Gq, p);
+            } else {
+              cta_giants<KS, false>(F, list, keys, count, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
+            }
+          }
+        }
+        if (r + 1 < J.Q) Er = shoup_mul(Er, bw, bq, p);
+      }
+    }
+    __syncthreads();
+
+    // Suspects, eight at a time: each thread scans its own tags (its two chains,
+    // 16 bits of each value's key) for their exact keys.  Tag matches (about three
+    // a prime on the wide job, nearly all false) go to settle_kernel: a thread that
+    // walked its chains here kept the whole CTA waiting, 17 of 117 ns per prime.
+    const uint32_t mc = *count;
+    if (mc > (uint32_t)kCtaMatchCap) {
       if (tid == 0) {
         const uint32_t r = atomicAdd(cb.redo_count, 1u);
         if (r < cb.cap) cb.redo[r] = i;
       }
       continue;
     }
-    if (novf) {
-      const uint64_t v = tid < novf ? ovf[tid] : 0;
-      __syncthreads();
-      if (tid == 0) *ML.count = 0;
-      if (tid < novf) W.insert_after(v, W.home((uint32_t)v));
-      __syncthreads();
-    }
-
-    // Giant steps (cta_giants)
-    const uint64_t Glm = rec[J.el_tab + 32 + lane];
-    const uint64_t Glw = from_mont(Glm, p, pinv), Glq = shoup_const(Glm, pinv);
-    const uint64_t Gw = rec[kElGw], Gq = rec[kElGq];
-    if constexpr (RM == kRowsIntId) {
-      if (spl == 2) {
-        const uint64_t E2 = shoup_mul(Glm, Gw, Gq, p);  // Z advanced by G^32, times 2^128
-        const uint64_t E2w = from_mont(E2, p, pinv), E2q = shoup_const(E2, pinv);
-        if (J.ctab_smem)
-          cta_giants<RM, true, true>(W, ML, vst, nact, warp, lane, spl, Glw, Glq, Gw, Gq, p, cts, E2w, E2q);
-        else
-          cta_giants<RM, true, false>(W, ML, vst, nact, warp, lane, spl, Glw, Glq, Gw, Gq, p, J.row_c, E2w, E2q);
-      } else if (J.ctab_smem) {
-        cta_giants<RM, false, true>(W, ML, vst, nact, warp, lane, spl, Glw, Glq, Gw, Gq, p, cts);
-      } else {
-        cta_giants<RM, false, false>(W, ML, vst, nact, warp, lane, spl, Glw, Glq, Gw, Gq, p, J.row_c);
-      }
-    } else if constexpr (RM == kRowsIntV) {
-      if (spl == 2) {
-        const uint64_t E2 = shoup_mul(Glm, Gw, Gq, p);  // Z advanced by G^32, times 2^128
-        cta_giants<RM, true, false>(W, ML, vst, nact, warp, lane, spl, Glw, Glq, Gw, Gq, p, J.row_c,
-                                    from_mont(E2, p, pinv), shoup_const(E2, pinv));
-      } else {
-        cta_giants<RM, false, false>(W, ML, vst, nact, warp, lane, spl, Glw, Glq, Gw, Gq, p, J.row_c);
-      }
-    } else {
-      cta_giants<kRowsV, false, false>(W, ML, vst, nact, warp, lane, spl, Glw, Glq, Gw, Gq, p, J.row_c);
-    }
-    __syncthreads();
-
-    // Tag matches: recompute the baby steps and compare full 64-bit values.
-    const uint32_t mc = *ML.count;
-    if (mc > ML.cap) {
-      if (tid == 0) {
-        const uint32_t r = atomicAdd(cb.redo_count, 1u);
-        if (r < cb.cap) cb.redo[r] = i;
-      }
-    } else if (mc > 0) {
-      // The first four matched values stay in registers (most primes have one
-      // or two false tag matches); only a step whose value equals one of them
-      // (or every step, with more than four matches) scans the list.
-      const uint64_t y0 = ML.list[0].y;
-      const uint64_t y1 = mc > 1 ? ML.list[1].y : y0;
-      const uint64_t y2 = mc > 2 ? ML.list[2].y : y0;
-      const uint64_t y3 = mc > 3 ? ML.list[3].y : y0;
-      auto pass = [&](auto step) {
-        uint64_t va = Bl, vb = Blb;
-#pragma unroll 2
-        for (uint32_t t = 0; t < CL; t++) {
-          const bool in_a = va == y0 || va == y1 || va == y2 || va == y3;
-          const bool in_b = vb == y0 || vb == y1 || vb == y2 || vb == y3;
-          if (in_a || in_b || mc > 4) {
 #pragma unroll 1
-            for (uint32_t q = 0; q < mc; q++) {
-              const Match mt = ML.list[q];
-              if (mt.y == va || mt.y == vb) {  // both when B has a small order
-                const uint64_t pk = rec_el(J, cb, J.el_row + (mt.slot >> 2), i);
-                const uint32_t row = (uint32_t)(pk >> (16 * (mt.slot & 3))) & 0xffffu;
-                if (mt.y == va) record_hit(J, hb, p, row, mt.s, ja0 + t);
-                if (mt.y == vb) record_hit(J, hb, p, row, mt.s, jb0 + t);
-              }
-            }
-          }
-          va = step(va);
-          vb = step(vb);
+    for (uint32_t q0 = 0; q0 < mc; q0 += 8) {
+      uint32_t tag[8], z[8];
+#pragma unroll
+      for (uint32_t q = 0; q < 8; q++) {
+        tag[q] = __byte_perm(keys[min(q0 + q, mc - 1)], 0, 0x1010);
+        z[q] = 0xffffffffu;
+      }
+#pragma unroll 4
+      for (uint32_t t = 0; t < CL; t++) {
+        const uint32_t tp = tags[t * T + tid];
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) z[q] = __vminu2(z[q], tp ^ tag[q]);
+      }
+      uint32_t hit = 0;
+#pragma unroll
+      for (uint32_t q = 0; q < 8; q++) hit |= zero_half(z[q]) && q0 + q < mc ? 1u << q : 0u;
+#pragma unroll 1
+      for (; hit; hit &= hit - 1) {
+        const Match mt = list[q0 + __ffs(hit) - 1];
+        const uint32_t idx = atomicAdd(cb.redo_count + 1, 1u);
+        if (idx < cb.cand_cap) {
+          cb.cand[idx] = Candidate{mt.y, i, mt.row, mt.s, tid};
+        } else {  // no room: the exact path takes the prime
+          const uint32_t r = atomicAdd(cb.redo_count, 1u);
+          if (r < cb.cap) cb.redo[r] = i;
         }
-      };
-      if (cb.small_step == kStepSmall) pass(StepSmall{J.bq_small, (uint32_t)rec[kElRcp], p});
-      else pass(StepShoup{rec[kElStw], rec[kElStq], p});
+      }
     }
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// The tag matches of a CTA launch: one thread per candidate walks the two baby
+// chains of the thread that found it and compares the values themselves.
+__global__ void __launch_bounds__(128) settle_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
+  const uint32_t cnt = cb.redo_count[1], n = cnt < cb.cand_cap ? cnt : cb.cand_cap;
+  const uint32_t T = 32 * J.cta_warps, CL = J.chain_len;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+    const Candidate x = cb.cand[c];
+    const uint64_t *rec = cb.recs + (size_t)x.i * J.rec_elems;
+    const uint64_t p = rec[kElP], pinv = rec[kElPinv], Stw = rec[kElStw], Stq = rec[kElStq];
+    const uint32_t w = x.thread >> 5;
+    uint64_t va = rec[J.el_tab + (x.thread & 31)];
+    if (w) va = shoup_mul(va, rec[kElWoff + 2 * w], rec[kElWoff + 2 * w + 1], p);
+    uint64_t vb = shoup_mul(va, rec[kElOfw], rec[kElOfq], p);
+    va = from_mont(va, p, pinv);
+    vb = from_mont(vb, p, pinv);
+#pragma unroll 1
+    for (uint32_t t = 0; t < CL; t++) {
+      if (va == x.y) record_hit(J, hb, p, x.row, x.s, x.thread * CL + t);
+      if (vb == x.y) record_hit(J, hb, p, x.row, x.s, (x.thread + T) * CL + t);
+      va = shoup_mul(va, Stw, Stq, p);
+      vb = shoup_mul(vb, Stw, Stq, p);
+    }
+  }
 }
 
 // The exact path: a table of (tag << jbits) | j entries with linear probing per
@@ -1646,12 +1513,13 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
   const uint32_t lane_row = lane / J.tlanes;
   const uint32_t rows_pass = J.rows_per_it * WG;  // row slots per pass of the group
   const uint32_t rc = *cb.redo_count;
-  const uint32_t nr = rc < cb.cap ? rc : cb.cap;
+  const bool all = rc > cb.cap;  // more entries than the list holds: every prime of the chunk
+  const uint32_t nr = !all ? rc : *cb.count < cb.cap ? *cb.count : cb.cap;
   const uint32_t ngroups = gridDim.x * NG;
   if (blockIdx.x == 0 && threadIdx.x == 0 && nr) atomicAdd(&hb.stat[kStatExact], (unsigned long long)nr);
 #pragma unroll 1
   for (uint32_t r = blockIdx.x * NG + grp; r < nr; r += ngroups) {
-    const uint32_t i = cb.redo[r];
+    const uint32_t i = all ? r : cb.redo[r];
     const uint64_t p = rec_el(J, cb, kElP, i), pinv = rec_el(J, cb, kElPinv, i);
     const uint32_t nact = (uint32_t)rec_el(J, cb, kElNact, i);
     const uint64_t Gs = rec_el(J, cb, kElGs, i);
@@ -1668,8 +1536,7 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
     for (uint32_t c = 0; c < 2; c++) {
       const uint32_t j0 = (gt + G * c) * J.chain_len;
       uint64_t v = c ? shoup_mul(Bl, rec_el(J, cb, kElOfw, i), rec_el(J, cb, kElOfq, i), p) : Bl;
-      // integer rows of the warp layout: giant values (below) come in normal form
-      if (WG == 1 && J.int_rows) v = from_mont(v, p, pinv);
+      if (J.int_rows) v = from_mont(v, p, pinv);  // giant values (below) come in normal form
 #pragma unroll 1
       for (uint32_t j = j0; j < J.m && j < j0 + J.chain_len; j++) {
         uint32_t h = (uint32_t)v & tmask;
@@ -1693,11 +1560,18 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
         const uint32_t row = J.row_mask ? nth_row(rec_el(J, cb, J.el_v, i), slot)
                                         : (uint32_t)(rec_el(J, cb, J.el_row + (slot >> 2), i) >> (16 * (slot & 3))) &
                                               0xffffu;
-        // integer rows: montmul(k*b^r, Z * 2^128) is the Montgomery form of the giant
-        // value (CTA layout); with Z's Montgomery form (warp layout) its normal form
-        uint64_t y = montmul(J.row_ids_only || J.row_mask ? (uint64_t)__ldg(J.row_c + row)
-                                                          : rec_el(J, cb, J.el_v + slot, i),
-                             Gl, p, pinv);
+        // integer rows: the normal form of k*b^r*Z from Z's Montgomery form (the CTA
+        // layout, whose k*b^r may exceed 32 bits: k*Z, times b per residue step)
+        uint64_t y;
+        if (WG > 1) {
+          y = montmul((uint64_t)__ldg(J.row_k + row), Gl, p, pinv);
+          const uint64_t bw = rec_el(J, cb, kElWoff + 2 * WG, i), bq = rec_el(J, cb, kElWoff + 2 * WG + 1, i);
+#pragma unroll 1
+          for (uint32_t q = __ldg(J.row_r + row); q; q--) y = shoup_mul(y, bw, bq, p);
+        } else {
+          y = montmul(J.row_ids_only || J.row_mask ? (uint64_t)__ldg(J.row_c + row) : rec_el(J, cb, J.el_v + slot, i), Gl,
+                      p, pinv);
+        }
         uint32_t s = lane_t + 1;
 #pragma unroll 1
         for (uint32_t u = 0; u < J.steps_per_lane; u++) {
@@ -1758,18 +1632,8 @@ static cudaError_t configure_one(const void *fn, int smem, int threads, int devi
 
 static int bsgs_threads(const JobDev &job) { return job.cta_warps > 1 ? 32 * kCtaWarps : 32 * kWarpsPerBlock; }
 
-template <bool MUL>
-static BsgsFn bsgs_cta_fn_t(const JobDev &job) {
-  switch (row_mode(job)) {
-    case kRowsIntId: return bsgs_cta_kernel<kRowsIntId, MUL>;
-    case kRowsIntV: return bsgs_cta_kernel<kRowsIntV, MUL>;
-    default: return bsgs_cta_kernel<kRowsV, MUL>;
-  }
-}
-
 static BsgsFn bsgs_cta_fn(const JobDev &job) {
-  const bool pow2 = (job.nbuckets & (job.nbuckets - 1)) == 0;
-  return pow2 ? bsgs_cta_fn_t<false>(job) : bsgs_cta_fn_t<true>(job);
+  return job.ctab_smem ? bsgs_cta_kernel<true> : bsgs_cta_kernel<false>;
 }
 
 static const void *bsgs_fast_fn(const JobDev &job) {
@@ -1797,8 +1661,10 @@ cudaError_t bsgs_configure(const JobDev &job, int device, int *grid_out, int *ex
 cudaError_t launch_bsgs(const JobDev &job, const ChunkBufs &cb, const HitBufs &hb, int grid,
                         cudaStream_t st) {
   if (job.cta_warps > 1)
+  {
     bsgs_cta_fn(job)<<<grid, 32 * kCtaWarps, bsgs_smem_bytes(job), st>>>(job, cb, hb);
-  else
+    settle_kernel<<<grid, 128, 0, st>>>(job, cb, hb);
+  } else
     bsgs_fn(job)<<<grid, 32 * kWarpsPerBlock, bsgs_smem_bytes(job), st>>>(job, cb, hb);
   return cudaGetLastError();
 }
