@@ -214,7 +214,14 @@ constexpr uint32_t kBatchStaticSmem = 4 * (kBatchMaxItems + 1) + 12;  // its pre
 uint64_t sieve_bitmap_words(uint64_t lo, uint64_t hi);
 cudaError_t launch_sieve(uint64_t lo, uint64_t hi, const uint32_t *sp, const uint64_t *sp_rcp, uint32_t nsp,
                          uint32_t nsmall, uint32_t *gbits, uint64_t *out, uint32_t *count, uint32_t cap,
-                         cudaStream_t st);
+                         cudaStream_t st, uint32_t *seg = nullptr);
+// Ordered form: with seg (sieve_segments(lo, hi) words) launch_sieve leaves the
+// primes as bits in gbits, their prefix sums per segment in seg and the total in
+// count; launch_emit writes the first cap of them in ascending order, as 64-bit
+// values (out) or as sieving primes with floor(2^64 / q) (out32, rcp).
+uint32_t sieve_segments(uint64_t lo, uint64_t hi);
+cudaError_t launch_emit(uint64_t lo, uint64_t hi, const uint32_t *gbits, const uint32_t *seg, uint32_t cap, uint64_t *out,
+                        uint32_t *out32, uint64_t *rcp, cudaStream_t st);
 cudaError_t launch_setup(const JobDev &job, const ChunkBufs &cb, cudaStream_t st);
 cudaError_t launch_bsgs(const JobDev &job, const ChunkBufs &cb, const HitBufs &hb, int grid,
                         cudaStream_t st);

@@ -62,10 +62,13 @@ __global__ void __launch_bounds__(256) sieve_large_kernel(uint64_t lo, uint64_t 
   for (uint64_t x = (f - lo) >> 1; x < nodd; x += q) atomicOr(&gbits[x >> 5], 1u << (x & 31));
 }
 
+// ORDERED: the segment's primes go back to gbits as bits and their number to
+// seg_count, for the ordered compaction below.
+template <bool ORDERED>
 __global__ void __launch_bounds__(kSieveThreads)
 sieve_small_kernel(uint64_t lo, uint64_t hi, const uint32_t *__restrict__ sp, const uint64_t *__restrict__ sp_rcp,
-                   uint32_t nsmall, const uint32_t *__restrict__ gbits, uint64_t *__restrict__ out,
-                   uint32_t *__restrict__ count, uint32_t cap) {
+                   uint32_t nsmall, uint32_t *gbits, uint64_t *__restrict__ out, uint32_t *__restrict__ count,
+                   uint32_t cap, uint32_t *__restrict__ seg_count) {
   __shared__ uint32_t bits[kSieveOdds / 32];
   __shared__ uint32_t warp_tot[kSieveThreads / 32];
   __shared__ uint32_t block_base;
@@ -76,7 +79,7 @@ sieve_small_kernel(uint64_t lo, uint64_t hi, const uint32_t *__restrict__ sp, co
   const uint64_t last = base + 2ull * (nodd - 1);
   const uint32_t tid = threadIdx.x;
   const uint32_t nwords = (nodd + 31) / 32;
-  const uint32_t *gseg = gbits + (size_t)blockIdx.x * (kSieveOdds / 32);
+  uint32_t *gseg = gbits + (size_t)blockIdx.x * (kSieveOdds / 32);
 
   for (uint32_t w = tid; w < kSieveOdds / 32; w += kSieveThreads) bits[w] = w < nwords ? gseg[w] : 0u;
   __syncthreads();
@@ -144,7 +147,15 @@ sieve_small_kernel(uint64_t lo, uint64_t hi, const uint32_t *__restrict__ sp, co
       if (lane >= (uint32_t)d) s += y;
     }
     if (lane < kSieveThreads / 32) warp_tot[lane] = s - v;  // exclusive
-    if (lane == kSieveThreads / 32 - 1) block_base = atomicAdd(count, s);
+    if (lane == kSieveThreads / 32 - 1) {
+      if (ORDERED) seg_count[blockIdx.x] = s;
+      else block_base = atomicAdd(count, s);
+    }
+  }
+  if (ORDERED) {
+#pragma unroll
+    for (uint32_t i = 0; i < WPT; i++) gseg[tid * WPT + i] = wv[i];
+    return;
   }
   __syncthreads();
   uint32_t pos = block_base + warp_tot[warp] + incl - mine;
@@ -161,24 +172,120 @@ sieve_small_kernel(uint64_t lo, uint64_t hi, const uint32_t *__restrict__ sp, co
   }
 }
 
+// Exclusive prefix sums of the segments' prime counts, in place; the total to *count.
+__global__ void __launch_bounds__(1024) segment_scan_kernel(uint32_t *seg, uint32_t n, uint32_t *count) {
+  __shared__ uint32_t warp_tot[32];
+  __shared__ uint32_t carry;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) carry = 0;
+  __syncthreads();
+  for (uint32_t b = 0; b < n; b += 1024) {
+    const uint32_t v = b + tid < n ? seg[b + tid] : 0;
+    uint32_t incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= (uint32_t)d) incl += y;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t t = warp_tot[lane];
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, t, d);
+        if (lane >= (uint32_t)d) t += y;
+      }
+      warp_tot[lane] = t;  // inclusive
+    }
+    __syncthreads();
+    const uint32_t base = carry + (warp ? warp_tot[warp - 1] : 0) + incl - v;
+    if (b + tid < n) seg[b + tid] = base;
+    __syncthreads();
+    if (tid == 1023) carry += warp_tot[31];
+    __syncthreads();
+  }
+  if (tid == 0) *count = carry;
+}
+
+// The primes of every segment's bits in ascending order, each segment from its
+// prefix sum on: as 64-bit values, or (rcp given) as sieving primes, 32-bit with
+// floor(2^64 / q).
+__global__ void __launch_bounds__(kSieveThreads)
+segment_emit_kernel(uint64_t lo, const uint32_t *__restrict__ gbits, const uint32_t *__restrict__ seg, uint32_t cap,
+                    uint64_t *__restrict__ out, uint32_t *__restrict__ out32, uint64_t *__restrict__ rcp) {
+  constexpr uint32_t WPT = kSieveOdds / 32 / kSieveThreads;
+  __shared__ uint32_t warp_tot[kSieveThreads / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t *g = gbits + (size_t)blockIdx.x * (kSieveOdds / 32) + tid * WPT;
+  uint32_t wv[WPT], mine = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < WPT; i++) {
+    wv[i] = g[i];
+    mine += __popc(wv[i]);
+  }
+  uint32_t incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= (uint32_t)d) incl += y;
+  }
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  uint32_t pos = seg[blockIdx.x] + incl - mine;
+  for (uint32_t w = 0; w < warp; w++) pos += warp_tot[w];
+  const uint64_t base = lo + 2ull * kSieveOdds * blockIdx.x;
+#pragma unroll
+  for (uint32_t i = 0; i < WPT; i++) {
+    uint32_t m = wv[i];
+    const uint64_t wbase = base + 64ull * (tid * WPT + i);
+    while (m) {
+      const uint64_t q = wbase + 2ull * (uint32_t)(__ffs(m) - 1);
+      m &= m - 1;
+      if (pos < cap) {
+        if (rcp) {
+          out32[pos] = (uint32_t)q;
+          rcp[pos] = ~0ull / q;  // floor(2^64 / q) for odd q > 1
+        } else {
+          out[pos] = q;
+        }
+      }
+      pos++;
+    }
+  }
+}
+
 uint64_t sieve_bitmap_words(uint64_t lo, uint64_t hi) {
   const uint64_t nodd = (hi - lo) / 2 + 1;
   const uint64_t segs = (nodd + kSieveOdds - 1) / kSieveOdds;
   return segs * (kSieveOdds / 32);
 }
+uint32_t sieve_segments(uint64_t lo, uint64_t hi) { return (uint32_t)(sieve_bitmap_words(lo, hi) / (kSieveOdds / 32)); }
 
 cudaError_t launch_sieve(uint64_t lo, uint64_t hi, const uint32_t *sp, const uint64_t *sp_rcp, uint32_t nsp,
                          uint32_t nsmall, uint32_t *gbits, uint64_t *out, uint32_t *count, uint32_t cap,
-                         cudaStream_t st) {
+                         cudaStream_t st, uint32_t *seg) {
   const uint64_t nodd = (hi - lo) / 2 + 1;
-  const uint64_t blocks = (nodd + kSieveOdds - 1) / kSieveOdds;
+  const uint32_t blocks = sieve_segments(lo, hi);
   cudaError_t e = cudaMemsetAsync(gbits, 0, sieve_bitmap_words(lo, hi) * 4, st);
   if (e != cudaSuccess) return e;
   if (nsp > nsmall) {
     const uint32_t nl = nsp - nsmall;
     sieve_large_kernel<<<(nl + 255) / 256, 256, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, nsp, gbits, nodd);
   }
-  sieve_small_kernel<<<(unsigned)blocks, kSieveThreads, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, gbits, out, count, cap);
+  if (!seg) {
+    sieve_small_kernel<false>
+        <<<blocks, kSieveThreads, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, gbits, out, count, cap, nullptr);
+  } else {
+    sieve_small_kernel<true><<<blocks, kSieveThreads, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, gbits, nullptr, nullptr, 0, seg);
+    segment_scan_kernel<<<1, 1024, 0, st>>>(seg, blocks, count);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_emit(uint64_t lo, uint64_t hi, const uint32_t *gbits, const uint32_t *seg, uint32_t cap, uint64_t *out,
+                        uint32_t *out32, uint64_t *rcp, cudaStream_t st) {
+  segment_emit_kernel<<<sieve_segments(lo, hi), kSieveThreads, 0, st>>>(lo, gbits, seg, cap, out, out32, rcp);
   return cudaGetLastError();
 }
 
