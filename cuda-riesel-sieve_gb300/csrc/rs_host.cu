@@ -764,11 +764,17 @@ static uint32_t plan_row_form(const Plan &pl, const Seqs &s, std::vector<uint32_
   return ids ? kRowsIntId : kRowsIntV;
 }
 
+// Rows of the warp layout handled by residue (JobDev::by_res).
+static bool row_by_res(const Plan &pl, uint32_t form, size_t nk) {
+  return form == kRowsV && !pl.cta && pl.Q <= kResMax && nk >= 4 && pl.nrows <= 512;
+}
+
 // First element of the lane tables in a record (el_tab; a record has el_tab + 64
 // elements), from the plan and the row form, as upload_part lays it out.
-static uint32_t record_el_tab(const Plan &pl, uint32_t form) {
-  const uint32_t el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : kElV;
-  if (pl.cta) form = kRowsIntId;  // CTA records hold row ids only
+static uint32_t record_el_tab(const Plan &pl, uint32_t form, size_t nk) {
+  const bool res = row_by_res(pl, form, nk);
+  const uint32_t el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : res ? kElV + 2 : kElV;
+  if (pl.cta || res) form = kRowsIntId;  // these records hold row ids only
   if (form == kRowsMask) return el_v + 2;
   const uint32_t max_act = std::max<uint32_t>(1, pl.nrows);
   const uint32_t el_row = el_v + (form == kRowsIntId ? 0u : ((max_act + 1) & ~1u));
@@ -1026,11 +1032,16 @@ static int upload_part(rs_job *j, Part &pt) {
   d.datless = j->opt.datless ? 1u : 0u;
   d.max_act = std::max<uint32_t>(1, pl.nrows);
   // CTA layout: every row is the integer k (the kernel multiplies by b^r), its
-  // records hold row ids only
-  d.int_rows = pl.cta || form != kRowsV ? 1u : 0u;
-  d.row_ids_only = pl.cta || form == kRowsIntId ? 1u : 0u;  // no V in the record
+  // records hold row ids only.  So are rows whose k*b^r exceeds 32 bits in the warp
+  // layout, when the residues have rows to share a multiplier (four k or more, Q
+  // up to 8) and the ids can be staged: a residue costs its multiplier (about 90
+  // cycles), a row 28 cycles instead of 70 and no V product in the setup kernel.
+  d.by_res = row_by_res(pl, form, nk) ? 1u : 0u;
+  d.row_slots = row_slots;
+  d.int_rows = pl.cta || d.by_res || form != kRowsV ? 1u : 0u;
+  d.row_ids_only = pl.cta || d.by_res || form == kRowsIntId ? 1u : 0u;  // no V in the record
   d.row_mask = !pl.cta && form == kRowsMask ? 1u : 0u;      // neither V nor row ids: an active-row mask
-  d.el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : kElV;
+  d.el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : d.by_res ? kElV + 2 : kElV;
   if (d.row_mask) {
     d.el_row = d.el_v;
     d.el_tab = d.el_v + 2;
@@ -1054,7 +1065,6 @@ static int upload_part(rs_job *j, Part &pt) {
     // bytes per CTA: tags, the rows' ids and (when 1.5 filter words a baby step
     // still fit) their k, suspects and keys, counts; the filter takes the rest up
     // to 3.5 words a baby step
-    d.row_slots = row_slots;
     const uint64_t fixed = align_up(2ull * pl.m + 2ull * row_slots + 20ull * kCtaMatchCap + 4ull * pl.Q + 16, 16);
     d.ctab_smem = fixed + 4ull * row_slots + 6ull * pl.m <= kCtaSmemMax ? 1u : 0u;
     const uint64_t used = fixed + (d.ctab_smem ? 4ull * row_slots : 0);
@@ -1067,7 +1077,7 @@ static int upload_part(rs_job *j, Part &pt) {
     for (uint32_t k : s.k) kmax = std::max<uint64_t>(kmax, k);
     d.edge_lim = (uint32_t)std::min<uint64_t>(0xffffffffu, ((kmax + 1) >> (d.fshift - 10)) + 1);
   } else {  // bytes per warp: the filter takes what the shared memory leaves (warp_filter)
-    const uint32_t fixed = warp_kernel_fixed(d.chain_len, d.stage_elems, d.row_mask != 0);
+    const uint32_t fixed = warp_kernel_fixed(d.chain_len, d.stage_elems, d.row_mask != 0, d.by_res != 0, d.row_slots);
     d.fwords = warp_filter(pl.m, fixed, 0, pt.ctas);
     d.warp_smem = 4 * d.fwords + fixed;
     d.fshift = filter_shift(d.fwords);
@@ -1945,14 +1955,14 @@ extern "C" int rs_batch_add(rs_batch *b, rs_job *job, uint64_t p0, uint64_t p1, 
 }
 
 // Filter words an item has in a multi-job launch with this stage and warp share.
-static uint32_t batch_item_words(uint32_t warp_bytes, uint32_t stage_max, const JobDev &d) {
-  const uint32_t fixed = warp_kernel_fixed(d.chain_len, stage_max, d.row_mask != 0);
+static uint32_t batch_item_words(uint32_t warp_bytes, uint32_t stage_max, uint32_t slots_max, const JobDev &d) {
+  const uint32_t fixed = warp_kernel_fixed(d.chain_len, stage_max, d.row_mask != 0, d.by_res != 0, slots_max);
   return warp_bytes > fixed ? (warp_bytes - fixed) / 16 * 4 : 0;
 }
 
 // Kernel variant of a warp-per-prime part: items of one multi-job launch share it.
 static uint32_t batch_variant(const JobDev &d) {
-  const uint32_t rm = d.row_mask ? kRowsMask : d.row_ids_only ? kRowsIntId : d.int_rows ? kRowsIntV : kRowsV;
+  const uint32_t rm = d.by_res ? kRowsRes : d.row_mask ? kRowsMask : d.row_ids_only ? kRowsIntId : d.int_rows ? kRowsIntV : kRowsV;
   return d.tlanes * 8 + rm;
 }
 
@@ -2031,7 +2041,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
   struct Group {
     uint32_t variant, ctas;
     std::vector<size_t> runs;
-    uint32_t stage_max = 0, warp_bytes = 0;
+    uint32_t stage_max = 0, slots_max = 0, warp_bytes = 0;
     int grid = 0;
   };
   std::vector<Group> groups;
@@ -2046,9 +2056,10 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
     const uint32_t ctas = runs[r].pt->ctas;
     // every item of a group keeps at least 0.75 filter words a baby step beside the largest stage
     auto fits = [&](const Group &G) {
-      const uint32_t share = warp_kernel_share(G.ctas, kBatchStaticSmem), stage = std::max(G.stage_max, d.stage_elems);
-      bool ok = 4 * batch_item_words(share, stage, d) >= 3 * d.m;
-      for (size_t x : G.runs) ok = ok && 4 * batch_item_words(share, stage, runs[x].pt->dev) >= 3 * runs[x].pt->dev.m;
+      const uint32_t share = warp_kernel_share(G.ctas, kBatchStaticSmem), stage = std::max(G.stage_max, d.stage_elems),
+                     slots = std::max(G.slots_max, d.row_slots);
+      bool ok = 4 * batch_item_words(share, stage, slots, d) >= 3 * d.m;
+      for (size_t x : G.runs) ok = ok && 4 * batch_item_words(share, stage, slots, runs[x].pt->dev) >= 3 * runs[x].pt->dev.m;
       return ok;
     };
     if (!fits(Group{v, ctas, {}})) {
@@ -2062,6 +2073,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
     if (g == groups.size()) groups.push_back(Group{v, ctas, {}});
     groups[g].runs.push_back(r);
     groups[g].stage_max = std::max(groups[g].stage_max, d.stage_elems);
+    groups[g].slots_max = std::max(groups[g].slots_max, d.row_slots);
   }
   for (size_t g = 0; g < groups.size();) {
     Group &G = groups[g];
@@ -2088,7 +2100,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
         if (rd >= R.chunks.size()) continue;
         BatchItem x;
         x.J = R.pt->dev;
-        x.J.fwords = std::min(x.J.fwords, batch_item_words(groups[g].warp_bytes, groups[g].stage_max, x.J));
+        x.J.fwords = std::min(x.J.fwords, batch_item_words(groups[g].warp_bytes, groups[g].stage_max, groups[g].slots_max, x.J));
         x.cb = R.j->cb;
         set_step(x.cb, R.forms[rd]);
         x.hb = R.pt->hb;
@@ -2173,7 +2185,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
       if (!gn[rd][g]) continue;
       const cudaStream_t s = B->side[br++ % kBatchBranches];
       launch_bsgs_batch(runs[groups[g].runs[0]].pt->dev, d_items + goff[rd][g], gn[rd][g], groups[g].stage_max,
-                        groups[g].warp_bytes, groups[g].grid, s);
+                        groups[g].slots_max, groups[g].warp_bytes, groups[g].grid, s);
       tot.launches++;
       tot.bsgs_launches++;
       for (size_t r : groups[g].runs) {
@@ -2574,7 +2586,7 @@ int rs::job_footprint(const char *text, size_t len, const rs_options &opt, JobFo
     rc = make_plan(g, opt, pl, false);
     if (rc) return rc;
     fp->arrays += part_array_bytes(pl, g, opt.datless != 0);
-    rec = std::max(rec, record_el_tab(pl, plan_row_form(pl, g, nullptr)) + 64);
+    rec = std::max(rec, record_el_tab(pl, plan_row_form(pl, g, nullptr), g.k.size()) + 64);
     cta = cta || pl.cta;
   }
   fp->per_prime = 8 + 4 + 8 * (uint64_t)rec + (cta ? kCandPerPrime * sizeof(Candidate) : 0);

@@ -65,7 +65,8 @@ constexpr uint32_t kStepShoup = 0, kStepSmall = 1, kStepHigh = 2;  // ChunkBufs:
 // Giant-step start values of the fast kernels (template argument): V in
 // Montgomery form, the integers k*b^r in V, k*b^r read by row id, or k*b^r of
 // the rows of an active-row mask.
-constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3;
+constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3, kRowsRes = 4;
+constexpr uint32_t kResMax = 8;    // residues (Q) of a by_res job at most
 constexpr uint32_t kMaskRows = 64;  // rows a row_mask record can describe
 constexpr int kCtaWarps = 16;      // warps sharing one prime in the CTA-per-prime kernel
 constexpr uint32_t kCtaSmemMax = 232448;  // shared memory a CTA may opt into (227 KB)
@@ -82,9 +83,10 @@ struct __align__(16) KInfo {
 // Shared memory of the warp-per-prime kernels: an SM's, what a CTA reserves, its
 // allocation granule, and the CTAs of four warps that registers allow on an SM.
 constexpr uint32_t kSmemPerSm = 233472, kSmemReserved = 1024, kSmemGranule = 1024, kWarpCtas = 5;
-// Bytes a warp needs beside its filter: tags, two record stages, V of a row mask.
-inline uint32_t warp_kernel_fixed(uint32_t chain_len, uint32_t stage_elems, bool row_mask) {
-  return 128 * chain_len + 16 * stage_elems + (row_mask ? 4 * kMaskRows : 0);
+// Bytes a warp needs beside its filter: tags, two record stages, V of a row mask or the residues' row lists.
+inline uint32_t warp_kernel_fixed(uint32_t chain_len, uint32_t stage_elems, bool row_mask, bool by_res,
+                                  uint32_t row_slots) {
+  return 128 * chain_len + 16 * stage_elems + (row_mask ? 4 * kMaskRows : by_res ? 4 * kResMax + 6 * row_slots : 0);
 }
 // Bytes a warp may use with `ctas` CTAs (and `fixed_smem` static bytes each) on an SM.
 inline uint32_t warp_kernel_share(uint32_t ctas, uint32_t fixed_smem) {
@@ -105,6 +107,7 @@ struct JobDev {
   uint32_t int_rows;     // every row's k*b^r < 2^32: V holds these integers (see the record layout)
   uint32_t row_ids_only; // integer rows whose records keep no V: the kernels read k*b^r by row id
   uint32_t row_mask;     // integer rows whose records keep only a mask of the active rows (see above)
+  uint32_t by_res;       // warp layout, k*b^r too large for integer rows: the rows are the integers k, one list per residue
   uint32_t T;            // giant steps per row
   uint32_t tlanes;       // min(T, 32): lanes sharing one row
   uint32_t rows_per_it;  // 32 / tlanes
@@ -112,7 +115,7 @@ struct JobDev {
   uint32_t fwords;       // 32-bit words of a prime's filter (a multiple of 4)
   uint32_t fshift;       // low bits of a key that do not choose the filter word (11..16)
   uint32_t edge_lim;     // CTA kernel: keys this close above a field's multiple are stored twice (baby_filter)
-  uint32_t row_slots;    // CTA kernel: slots of the residues' row lists (a multiple of 8)
+  uint32_t row_slots;    // CTA kernel and by_res: slots of the residues' row lists (a multiple of 8)
   uint32_t jbits;        // bits of j in an exact-path table entry
   uint32_t nrows, nk;
   int64_t e0;            // x = e0 + m*s - j for giant index s in [1, T]
@@ -233,12 +236,12 @@ int bsgs_exact_smem_bytes(const JobDev &job);
 uint64_t bsgs_exact_scratch_bytes(const JobDev &job, int exact_grid);
 cudaError_t bsgs_configure(const JobDev &job, int device, int *grid_out, int *exact_grid_out);
 // Multi-job launch over `nitems` items in device memory that share rep's kernel
-// variant (rep: any of them); stage_max is the largest over the items, and
+// variant (rep: any of them); stage_max and row_slots_max are the largest over the items, and
 // warp_bytes holds every item's warp_kernel_bytes with that stage.
 // batch_configure gives the grid.
 cudaError_t batch_configure(const JobDev &rep, uint32_t warp_bytes, int device, int *grid_out);
 cudaError_t launch_bsgs_batch(const JobDev &rep, const BatchItem *items, uint32_t nitems, uint32_t stage_max,
-                              uint32_t warp_bytes, int grid, cudaStream_t st);
+                              uint32_t row_slots_max, uint32_t warp_bytes, int grid, cudaStream_t st);
 
 // Build the character tables sel[0..nsel) of a job's list (odd parts kodd[],
 // word offsets word_off[] into bits); first[] are the running word counts of

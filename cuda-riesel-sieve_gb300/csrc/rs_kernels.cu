@@ -603,6 +603,7 @@ __global__ void __launch_bounds__(128) setup_kernel(JobDev J, ChunkBufs cb) {
     rec_st2(rec, kElWoff + 2 * J.cta_warps, bmod, bq);  // b and its Shoup constant
   }
   rec_st2(rec, kElOfw, from_mont(off, p, M.pinv), shoup_const(off, M.pinv));
+  if (J.by_res) rec_st2(rec, kElV, bmod, bq);
 }
 
 // Quadratic-character tables: word w of the table of odd k' holds bit t =
@@ -988,6 +989,32 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
     if ((lo >> lane) & 1u) vbuf[__popc(lo & below)] = c_lo;
     if ((hi >> lane) & 1u) vbuf[__popc(lo) + __popc(hi & below)] = c_hi;
   }
+  // By residue: the active rows' k (ks) and ids (rid) in one list per residue r,
+  // from slot J.row_base[r] on, in any order; their numbers in vbuf[0..Q).
+  uint32_t *ks = vbuf + kResMax;
+  uint16_t *rid = reinterpret_cast<uint16_t *>(ks + J.row_slots);
+  if constexpr (RM == kRowsRes) {
+    if (lane < kResMax) vbuf[lane] = 0;
+    __syncwarp();
+    const uint16_t *ids = reinterpret_cast<const uint16_t *>(cur + J.el_row);
+#pragma unroll 1
+    for (uint32_t a = lane; a < ((nact + 31) & ~31u); a += 32) {
+      const bool on = a < nact;
+      const uint32_t id = on ? ids[a] : 0;
+      const uint2 kr = __ldg(J.row_kr + id);
+      const uint32_t r = on ? kr.y & 0xfffu : 0xffffffffu;
+      const uint32_t same = __match_any_sync(0xffffffffu, r);
+      const uint32_t have = on ? vbuf[r] : 0;
+      __syncwarp();
+      const uint32_t at = have + __popc(same & ((1u << lane) - 1u));
+      if (on) {
+        ks[at + (kr.y >> 12)] = kr.x;
+        rid[at + (kr.y >> 12)] = (uint16_t)id;
+        if ((same >> lane) == 1u) vbuf[r] = at + 1;  // the last of its residue
+      }
+      __syncwarp();
+    }
+  }
   const uint64_t p = cur[kElP], pinv = cur[kElPinv];
   // Multipliers in normal form with their Shoup constants; the values
   // they multiply stay in Montgomery form, so products stay comparable.
@@ -1022,12 +1049,24 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
 
   // Giant steps: lane (lane_row, lane_t) takes row slots g*RPI + lane_row for
   // two consecutive passes g at a time, giant indices s = lane_t + 1 + 32u.
-  const uint32_t ngi = (nact + RPI - 1) / RPI;
+  constexpr int GM = RM == kRowsRes ? kRowsMask : RM;  // the lists hold integers, as a mask's
+  uint32_t n = nact;  // the rows gone through: all active ones, or those of residue r
+  uint32_t r = 0, base = 0;
+  uint64_t E = Glm;  // the lane's multiplier as stored, advanced by G^32 per step u
+  uint64_t Er = Glm; // ... for u = 0
+  if constexpr (RM == kRowsRes) {
+    for (; vbuf[r] == 0; r++) Er = shoup_mul(Er, cur[kElV], cur[kElV + 1], p);
+    n = vbuf[r];
+    base = __ldg(J.row_base + r);
+    E = Er;
+  }
+  uint32_t ngi = (n + RPI - 1) / RPI;
   // the start values (or row ids): built by the warp, staged, or in the record
-  const void *src_s = RM == kRowsMask ? (const void *)vbuf
-                                      : RM == kRowsIntId ? (const void *)(cur + J.el_row) : (const void *)(cur + kElV);
+  const void *src_s = RM == kRowsRes    ? (const void *)(ks + base)
+                      : RM == kRowsMask ? (const void *)vbuf
+                                        : RM == kRowsIntId ? (const void *)(cur + J.el_row) : (const void *)(cur + kElV);
   const void *src_g = cb.recs + (size_t)i * J.rec_elems + (RM == kRowsIntId ? J.el_row : kElV);
-  const bool staged = RM == kRowsMask || J.stage_full;
+  const bool staged = RM == kRowsRes || RM == kRowsMask || J.stage_full;
   // (k, 0), (k, 1) row pairs; V rows form the second value by the short product
   // by b (p > 2^33, b*p < 2^63: mul_small)
   const bool paired = RPI == 1 && cb.pair_ok && (cur[kElNact] >> 32);
@@ -1035,11 +1074,10 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
   // A lane's further steps (T > 32): advance the multiplier once and go through
   // the rows again; in blocks of at most 64 tests a lane, after which the block's
   // suspects are settled.
-  uint64_t E = Glm;  // the lane's multiplier as stored, advanced by G^32 per step u
   GiantMul G;
   G.set(E, p, pinv);
   auto start = [&](uint32_t sl) {
-    return staged ? giant_start<RM>(src_s, J.row_c, sl) : giant_start<RM>(src_g, J.row_c, sl);
+    return staged ? giant_start<GM>(src_s, J.row_c, sl) : giant_start<GM>(src_g, J.row_c, sl);
   };
   uint32_t u = 0, at = 0, suspects = 0;  // step, the block's first pass, suspects so far
 #pragma unroll 1
@@ -1049,12 +1087,12 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
     // Separate calls for staged and global V keep each load's address
     // space known to the compiler.
     if (RM == kRowsV && paired && staged)
-      giant_test<RPI, RM, RPI == 1>(F, src_s, J.row_c, at, g1, nact, lane_row, G, np, pinv, hA, hB, J.base,
+      giant_test<RPI, GM, RPI == 1>(F, src_s, J.row_c, at, g1, n, lane_row, G, np, pinv, hA, hB, J.base,
                                     (uint32_t)cur[kElRcp]);
     else if (staged)
-      giant_test<RPI, RM>(F, src_s, J.row_c, at, g1, nact, lane_row, G, np, pinv, hA, hB);
+      giant_test<RPI, GM>(F, src_s, J.row_c, at, g1, n, lane_row, G, np, pinv, hA, hB);
     else
-      giant_test<RPI, RM>(F, src_g, J.row_c, at, g1, nact, lane_row, G, np, pinv, hA, hB);
+      giant_test<RPI, GM>(F, src_g, J.row_c, at, g1, n, lane_row, G, np, pinv, hA, hB);
     // Suspects: every lane forms the exact value and key of its next one, then
     // the warp takes them in turn: each lane scans its own tags (its two chains,
     // 16 bits of each value's key), and a tag match is settled by walking the
@@ -1064,7 +1102,7 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
     while (uint32_t any = __ballot_sync(0xffffffffu, bits != 0)) {
       const uint32_t bit = bits ? __ffsll((long long)bits) - 1 : 0;
       const uint32_t sl = (at + 2 * (bit & 31) + (bit >> 5)) * RPI + lane_row;
-      const bool mine = bits != 0 && sl < nact;
+      const bool mine = bits != 0 && sl < n;
       bits &= bits - 1;
       any = __ballot_sync(0xffffffffu, mine);
       suspects += __popc(any);
@@ -1080,8 +1118,8 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
       bool edge = false;
       if (mine) {
         const uint64_t v = start(sl);
-        y = giant_exact<RM>(v, G);
-        edge = exact_key<RM>(y, giant_key<RM>(v, G, RM == kRowsV ? G.w() : 0, np, pinv), p, pinv, f);
+        y = giant_exact<GM>(v, G);
+        edge = exact_key<GM>(y, giant_key<GM>(v, G, RM == kRowsV ? G.w() : 0, np, pinv), p, pinv, f);
       }
       const uint32_t both = __ballot_sync(0xffffffffu, edge);  // these could be stored under F + 1 too
 #pragma unroll 1
@@ -1106,6 +1144,8 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
               uint32_t row;
               if constexpr (RM == kRowsMask) {
                 row = nth_row(cur[kElV], slot);
+              } else if constexpr (RM == kRowsRes) {
+                row = rid[base + slot];
               } else {
                 const uint64_t pk = rec_el(J, cb, J.el_row + (slot >> 2), i);
                 row = (uint32_t)(pk >> (16 * (slot & 3))) & 0xffffu;
@@ -1121,16 +1161,31 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
     }
     at = g1;
     if (at < ngi) continue;
-    if (++u >= spl) break;
     at = 0;
-    E = shoup_mul(E, cur[kElGw], cur[kElGq], p);
+    if (++u < spl) {
+      E = shoup_mul(E, cur[kElGw], cur[kElGq], p);
+    } else if constexpr (RM == kRowsRes) {  // the next residue that has rows
+      u = 0;
+      do {
+        if (++r >= J.Q) return;
+        Er = shoup_mul(Er, cur[kElV], cur[kElV + 1], p);
+      } while (vbuf[r] == 0);
+      n = vbuf[r];
+      ngi = (n + RPI - 1) / RPI;
+      base = __ldg(J.row_base + r);
+      src_s = ks + base;
+      E = Er;
+    } else {
+      break;
+    }
     G.set(E, p, pinv);
   }
 }
 
 // Per-warp shared memory of the fast kernel:
 //   [filter, fwords x 4 B][tags, chain_len x 32 x 4 B][2 stages x stage_elems x 8 B]
-//   ([kMaskRows V x 4 B], row_mask only)
+//   ([kMaskRows V x 4 B], row_mask; [kResMax counts x 4 B][k and ids of the rows,
+//   row_slots x 6 B], by_res)
 // The stages hold a record's header and V (double-buffered with cp.async); each
 // lane's B^lane and G^(lane+1) entries are loaded into registers one prime ahead.
 // With row_mask the stage holds the header and the active-row mask, and the
@@ -1208,12 +1263,13 @@ bsgs_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
 // start-value form RM.  Per-warp shared memory, in fixed places whatever the
 // item:
 //   [2 stages x stage_max x 8 B]([kMaskRows V x 4 B], RM = kRowsMask)
-//   [the item's filter, fwords x 4 B, and tags, chain_len x 32 x 4 B]
+//   ([kResMax counts x 4 B][row_slots_max x 6 B], RM = kRowsRes)[the item's filter, fwords x 4 B, and tags, chain_len x 32 x 4 B]
 // The record of the warp's next prime (possibly another item's) is staged by
 // cp.async while the current one runs, as in bsgs_kernel.
 template <int TL, int RM>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, kWarpCtas)
-bsgs_batch_kernel(const BatchItem *__restrict__ items, uint32_t nitems, uint32_t warp_bytes, uint32_t stage_max) {
+bsgs_batch_kernel(const BatchItem *__restrict__ items, uint32_t nitems, uint32_t warp_bytes, uint32_t stage_max,
+                  uint32_t row_slots_max) {
   extern __shared__ uint4 smem4[];
   __shared__ uint32_t start[kBatchMaxItems + 1];  // prefix sums of the items' prime counts
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1232,7 +1288,7 @@ bsgs_batch_kernel(const BatchItem *__restrict__ items, uint32_t nitems, uint32_t
   uint8_t *base = reinterpret_cast<uint8_t *>(smem4) + (size_t)warp * warp_bytes;
   uint64_t *stage0 = reinterpret_cast<uint64_t *>(base);
   uint32_t *vbuf = reinterpret_cast<uint32_t *>(stage0 + 2 * stage_max);
-  uint32_t *fwords = vbuf + (RM == kRowsMask ? kMaskRows : 0);
+  uint32_t *fwords = vbuf + (RM == kRowsMask ? kMaskRows : RM == kRowsRes ? kResMax + row_slots_max * 6 / 4 : 0);
   const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
   const uint32_t first = blockIdx.x * kWarpsPerBlock + warp;
   // the item of global index g, from the item of an earlier (smaller) index
@@ -1291,7 +1347,7 @@ bsgs_batch_kernel(const BatchItem *__restrict__ items, uint32_t nitems, uint32_t
   if (lane == 0 && npaired && ck < nitems) atomicAdd(&items[ck].hb.stat[kStatPaired], (unsigned long long)npaired);
 }
 
-typedef void (*BatchFn)(const BatchItem *, uint32_t, uint32_t, uint32_t);
+typedef void (*BatchFn)(const BatchItem *, uint32_t, uint32_t, uint32_t, uint32_t);
 
 template <int RM>
 static BatchFn batch_fn_t(uint32_t tlanes) {
@@ -1320,11 +1376,12 @@ static BsgsFn bsgs_fn_t(uint32_t tlanes) {
 }
 
 static int row_mode(const JobDev &job) {
-  return job.row_mask ? kRowsMask : job.row_ids_only ? kRowsIntId : job.int_rows ? kRowsIntV : kRowsV;
+  return job.by_res ? kRowsRes : job.row_mask ? kRowsMask : job.row_ids_only ? kRowsIntId : job.int_rows ? kRowsIntV : kRowsV;
 }
 
 static BsgsFn bsgs_fn(const JobDev &job) {
   switch (row_mode(job)) {
+    case kRowsRes: return bsgs_fn_t<kRowsRes>(job.tlanes);
     case kRowsMask: return bsgs_fn_t<kRowsMask>(job.tlanes);
     case kRowsIntId: return bsgs_fn_t<kRowsIntId>(job.tlanes);
     case kRowsIntV: return bsgs_fn_t<kRowsIntV>(job.tlanes);
@@ -1667,12 +1724,13 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
         const uint32_t row = J.row_mask ? nth_row(rec_el(J, cb, J.el_v, i), slot)
                                         : (uint32_t)(rec_el(J, cb, J.el_row + (slot >> 2), i) >> (16 * (slot & 3))) &
                                               0xffffu;
-        // integer rows: the normal form of k*b^r*Z from Z's Montgomery form (the CTA
-        // layout, whose k*b^r may exceed 32 bits: k*Z, times b per residue step)
+        // integer rows: the normal form of k*b^r*Z from Z's Montgomery form (CTA layout
+        // and by_res, whose k*b^r may exceed 32 bits: k*Z, times b per residue step)
         uint64_t y;
-        if (WG > 1) {
+        if (WG > 1 || J.by_res) {
           y = montmul((uint64_t)__ldg(J.row_k + row), Gl, p, pinv);
-          const uint64_t bw = rec_el(J, cb, kElWoff + 2 * WG, i), bq = rec_el(J, cb, kElWoff + 2 * WG + 1, i);
+          constexpr uint32_t eb = WG > 1 ? kElWoff + 2 * WG : kElV;
+          const uint64_t bw = rec_el(J, cb, eb, i), bq = rec_el(J, cb, eb + 1, i);
 #pragma unroll 1
           for (uint32_t q = __ldg(J.row_r + row); q; q--) y = shoup_mul(y, bw, bq, p);
         } else {
@@ -1778,6 +1836,7 @@ cudaError_t launch_bsgs(const JobDev &job, const ChunkBufs &cb, const HitBufs &h
 
 static BatchFn batch_fn(const JobDev &rep) {
   switch (row_mode(rep)) {
+    case kRowsRes: return batch_fn_t<kRowsRes>(rep.tlanes);
     case kRowsMask: return batch_fn_t<kRowsMask>(rep.tlanes);
     case kRowsIntId: return batch_fn_t<kRowsIntId>(rep.tlanes);
     case kRowsIntV: return batch_fn_t<kRowsIntV>(rep.tlanes);
@@ -1792,10 +1851,11 @@ cudaError_t batch_configure(const JobDev &rep, uint32_t warp_bytes, int device, 
 }
 
 cudaError_t launch_bsgs_batch(const JobDev &rep, const BatchItem *items, uint32_t nitems, uint32_t stage_max,
-                              uint32_t warp_bytes, int grid, cudaStream_t st) {
+                              uint32_t row_slots_max, uint32_t warp_bytes, int grid, cudaStream_t st) {
   if (nitems == 0) return cudaSuccess;
   if (nitems > kBatchMaxItems) return cudaErrorInvalidValue;
-  batch_fn(rep)<<<grid, 32 * kWarpsPerBlock, kWarpsPerBlock * warp_bytes, st>>>(items, nitems, warp_bytes, stage_max);
+  batch_fn(rep)<<<grid, 32 * kWarpsPerBlock, kWarpsPerBlock * warp_bytes, st>>>(items, nitems, warp_bytes, stage_max,
+                                                                                       row_slots_max);
   return cudaGetLastError();
 }
 
