@@ -382,6 +382,9 @@ static int count_rows(const Seqs &s, uint32_t Q, bool datless) {
   return rows;
 }
 
+// Whether rows that are no 32-bit integers go by residue: every residue has rows to share a multiplier.
+static bool rows_by_residue(uint32_t Q, size_t nk, size_t rows) { return Q <= kResMax && nk >= 4 && rows <= 512; }
+
 // One point of the planner's search: the parameters that define a plan, and its modelled cost.
 struct PlanChoice {
   uint32_t Q = 0, T = 0, m = 0;
@@ -422,6 +425,16 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
   // A giant step (Shoup product + probe) costs about 1.4 baby steps (a short or
   // Shoup product + insert), measured on the benchmark job.
   constexpr double kGiantWeight = 1.4;
+  // Warp plans of few k, measured on jobs of one to fourteen (the weights above were
+  // fitted on more): each step after a lane's first advances the lane's multiplier and goes through the
+  // rows again (two baby steps beside the rows' own); a baby step by a b^Q above
+  // 2^31 is a full Shoup product (1.4); a row that is no 32-bit integer takes a
+  // full product per step (2.0), or by residue a multiplier each (2.2 a residue).
+  // One k over 2e6 exponents: Q = 26, T = 64 takes 3.3 ns per prime against 4.3 for
+  // Q = 2, T = 1024; four k over 8e5: Q = 2, T = 256 4.0 against 5.9 for Q = 8, T = 64.
+  const bool few = s.k.size() <= 16;
+  constexpr double kStepCost = 2.0, kShoupStep = 1.4, kResidueRow = 2.0, kResidueCost = 2.2;
+  constexpr double kCtaFew = 2.5;  // 14 k over 1.8e6 exponents: a CTA per prime takes 37 ns, a warp 15
   // Setup-kernel cost per (k, n mod Q) row, in the same units.
   constexpr double kRowCost = 0.18;
   // A step of the CTA kernel costs more than one of the warp kernel (block-wide
@@ -441,6 +454,8 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
       for (uint32_t e = 1; e < Q && c < (1ull << 32); e++) c *= s.base;
       ints_q = c < (1ull << 32);
     }
+    const bool short_q = Q * std::log2((double)s.base) < 31.0;  // b^Q as the short product's integer
+    const bool res_q = rows_by_residue(Q, s.k.size(), (size_t)rows);
     auto consider = [&](bool cta, uint64_t T, uint64_t m, uint32_t nb, uint32_t slog, double cost) {
       if (ranked) ranked->push_back(PlanChoice{Q, (uint32_t)T, (uint32_t)m, cta, cost, nb});
       if (force) {
@@ -490,7 +505,9 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
           const double fp = ER * (double)T * ((double)m / nb) / 65536.0;  // expected tag matches per prime
           // (a prime with more than kMatchCap matches takes the slow exact path)
           if (warps >= 4 && fp <= 2.0) {
-            const double cost = (std::ceil((double)m / 32.0) + kGiantWeight * std::ceil(ER / rpi) * spl +
+            const double cost = ((few && !short_q ? kShoupStep : 1.0) * std::ceil((double)m / 32.0) +
+                                 (few && !ints_q && !res_q ? kResidueRow : kGiantWeight) * std::ceil(ER / rpi) * spl +
+                                 kStepCost * (spl - 1) + (few && !ints_q && res_q ? kResidueCost * Q * spl : 0.0) +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
                                 std::sqrt(kFullWarps / warps);
             consider(false, T, m, 1u << blog, slog, cost);
@@ -522,7 +539,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
           if (m <= mcap && m < 65536 && m * T >= X && slog <= 17 && smem <= kCtaSmemMax && fp <= 16.0) {
             const double cost = ((double)m / 32.0 + kGiantWeight * kCtaWarps * std::ceil(ER / kCtaWarps) * spl +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
-                                std::sqrt(kFullWarps / kCtaWarps) * kCtaStepCost;
+                                std::sqrt(kFullWarps / kCtaWarps) * kCtaStepCost * (few ? kCtaFew : 1.0);
             consider(true, T, m, nbk, slog, cost);
           }
         }
@@ -766,7 +783,7 @@ static uint32_t plan_row_form(const Plan &pl, const Seqs &s, std::vector<uint32_
 
 // Rows of the warp layout handled by residue (JobDev::by_res).
 static bool row_by_res(const Plan &pl, uint32_t form, size_t nk) {
-  return form == kRowsV && !pl.cta && pl.Q <= kResMax && nk >= 4 && pl.nrows <= 512;
+  return form == kRowsV && !pl.cta && rows_by_residue(pl.Q, nk, pl.nrows);
 }
 
 // First element of the lane tables in a record (el_tab; a record has el_tab + 64
@@ -1657,7 +1674,7 @@ static int sieve_range_impl(rs_job *j, uint64_t p0, uint64_t p1, rs_factor *out,
         forms[c * P + q] = form.form;
         set_step(j->cb, form);
         if (ce) cudaEventRecord(ce[2 + 4 * q], j->st);
-        e = launch_setup(pt.dev, j->cb, j->st);
+        e = launch_setup(pt.dev, j->cb, (todo[c].b - todo[c].a) / 2 + 1, j->st);
         if (e == cudaSuccess) e = cudaMemsetAsync(j->cb.redo_count, 0, 8, j->st);
         if (ce) cudaEventRecord(ce[3 + 4 * q], j->st);
         if (e == cudaSuccess) e = launch_bsgs(pt.dev, j->cb, pt.hb, pt.bsgs_grid, j->st);
@@ -2174,7 +2191,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
       cudaMemcpyAsync(&h_counts[R.count0 + rd], j->cb.count, 4, cudaMemcpyDeviceToHost, s);
       ChunkBufs cb = j->cb;
       set_step(cb, R.forms[rd]);
-      launch_setup(R.pt->dev, cb, s);
+      launch_setup(R.pt->dev, cb, (c.b - c.a) / 2 + 1, s);
       cudaMemsetAsync(j->cb.redo_count, 0, 8, s);
       tot.launches += (j->nsp > j->nsp_small ? 2 : 1) + 1;
     }

@@ -225,7 +225,8 @@ cudaError_t launch_sieve(uint64_t lo, uint64_t hi, const uint32_t *sp, const uin
 uint32_t sieve_segments(uint64_t lo, uint64_t hi);
 cudaError_t launch_emit(uint64_t lo, uint64_t hi, const uint32_t *gbits, const uint32_t *seg, uint32_t cap, uint64_t *out,
                         uint32_t *out32, uint64_t *rcp, cudaStream_t st);
-cudaError_t launch_setup(const JobDev &job, const ChunkBufs &cb, cudaStream_t st);
+// odds: odd numbers of the chunk's window, a bound on its primes
+cudaError_t launch_setup(const JobDev &job, const ChunkBufs &cb, uint64_t odds, cudaStream_t st);
 cudaError_t launch_bsgs(const JobDev &job, const ChunkBufs &cb, const HitBufs &hb, int grid,
                         cudaStream_t st);
 cudaError_t launch_bsgs_exact(const JobDev &job, const ChunkBufs &cb, const HitBufs &hb, int grid,

@@ -32,6 +32,7 @@
 //   verify_kernel  direct k*b^n check of every hit (kernel_v0.24.6.cu:1649-1671).
 #include <cstdio>
 #include <type_traits>
+#include <algorithm>
 
 #include "rs_arith.cuh"
 #include "rs_internal.h"
@@ -64,24 +65,25 @@ __global__ void __launch_bounds__(256) sieve_large_kernel(uint64_t lo, uint64_t 
 
 // ORDERED: the segment's primes go back to gbits as bits and their number to
 // seg_count, for the ordered compaction below.
-template <bool ORDERED>
+// ODDS: odd numbers per segment; a window with few segments takes shorter ones.
+template <bool ORDERED, int ODDS>
 __global__ void __launch_bounds__(kSieveThreads)
 sieve_small_kernel(uint64_t lo, uint64_t hi, const uint32_t *__restrict__ sp, const uint64_t *__restrict__ sp_rcp,
                    uint32_t nsmall, uint32_t *gbits, uint64_t *__restrict__ out, uint32_t *__restrict__ count,
                    uint32_t cap, uint32_t *__restrict__ seg_count) {
-  __shared__ uint32_t bits[kSieveOdds / 32];
+  __shared__ uint32_t bits[ODDS / 32];
   __shared__ uint32_t warp_tot[kSieveThreads / 32];
   __shared__ uint32_t block_base;
-  const uint64_t base = lo + 2ull * (uint64_t)kSieveOdds * blockIdx.x;  // odd
+  const uint64_t base = lo + 2ull * (uint64_t)ODDS * blockIdx.x;  // odd
   if (base > hi) return;
   const uint64_t span = (hi - base) / 2 + 1;
-  const uint32_t nodd = span < (uint64_t)kSieveOdds ? (uint32_t)span : (uint32_t)kSieveOdds;
+  const uint32_t nodd = span < (uint64_t)ODDS ? (uint32_t)span : (uint32_t)ODDS;
   const uint64_t last = base + 2ull * (nodd - 1);
   const uint32_t tid = threadIdx.x;
   const uint32_t nwords = (nodd + 31) / 32;
-  uint32_t *gseg = gbits + (size_t)blockIdx.x * (kSieveOdds / 32);
+  uint32_t *gseg = gbits + (size_t)blockIdx.x * (ODDS / 32);
 
-  for (uint32_t w = tid; w < kSieveOdds / 32; w += kSieveThreads) bits[w] = w < nwords ? gseg[w] : 0u;
+  for (uint32_t w = tid; w < ODDS / 32; w += kSieveThreads) bits[w] = w < nwords ? gseg[w] : 0u;
   __syncthreads();
 
   // Smallest primes: the whole CTA strides over the multiples of one prime.
@@ -114,7 +116,7 @@ sieve_small_kernel(uint64_t lo, uint64_t hi, const uint32_t *__restrict__ sp, co
   __syncthreads();
 
   // Compaction: each thread owns a contiguous run of words.
-  constexpr uint32_t WPT = kSieveOdds / 32 / kSieveThreads;
+  constexpr uint32_t WPT = ODDS / 32 / kSieveThreads;
   uint32_t mine = 0;
   uint32_t wv[WPT];
 #pragma unroll
@@ -274,10 +276,17 @@ cudaError_t launch_sieve(uint64_t lo, uint64_t hi, const uint32_t *sp, const uin
     sieve_large_kernel<<<(nl + 255) / 256, 256, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, nsp, gbits, nodd);
   }
   if (!seg) {
-    sieve_small_kernel<false>
-        <<<blocks, kSieveThreads, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, gbits, out, count, cap, nullptr);
+    // Below two blocks an SM a window's time is one block's: segments a quarter as
+    // long (a 1e5-wide window at 1e13: 61 -> 37 us for both passes).
+    constexpr int kShort = kSieveOdds / 4;
+    if (blocks < 304)
+      sieve_small_kernel<false, kShort><<<(unsigned)((nodd + kShort - 1) / kShort), kSieveThreads, 0, st>>>(
+          lo, hi, sp, sp_rcp, nsmall, gbits, out, count, cap, nullptr);
+    else
+      sieve_small_kernel<false, kSieveOdds>
+          <<<blocks, kSieveThreads, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, gbits, out, count, cap, nullptr);
   } else {
-    sieve_small_kernel<true><<<blocks, kSieveThreads, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, gbits, nullptr, nullptr, 0, seg);
+    sieve_small_kernel<true, kSieveOdds><<<blocks, kSieveThreads, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, gbits, nullptr, nullptr, 0, seg);
     segment_scan_kernel<<<1, 1024, 0, st>>>(seg, blocks, count);
   }
   return cudaGetLastError();
@@ -642,8 +651,10 @@ cudaError_t launch_jacobi_tables(const uint32_t *kodd, const uint32_t *word_off,
   return cudaGetLastError();
 }
 
-cudaError_t launch_setup(const JobDev &job, const ChunkBufs &cb, cudaStream_t st) {
-  const unsigned blocks = (cb.cap + 127) / 128;
+cudaError_t launch_setup(const JobDev &job, const ChunkBufs &cb, uint64_t odds, cudaStream_t st) {
+  // (the chunk has at most `odds` primes: a narrow window launched 40,000 empty
+  // blocks for its buffer's capacity, 30 of the 45 us)
+  const unsigned blocks = (unsigned)((std::min<uint64_t>(cb.cap, odds) + 127) / 128);
   setup_kernel<<<blocks, 128, 0, st>>>(job, cb);
   return cudaGetLastError();
 }
@@ -1872,31 +1883,31 @@ cudaError_t launch_bsgs_exact(const JobDev &job, const ChunkBufs &cb, const HitB
 // Direct verification of every candidate hit.
 
 __global__ void verify_kernel(JobDev J, HitBufs hb) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t cnt = *hb.raw_count;
   const uint32_t n = cnt < hb.cap ? cnt : hb.cap;
-  if (i >= n) return;
-  const Hit h = hb.raw[i];
-  const uint64_t p = h.p;
-  Mont M;
-  M.p = p;
-  M.pinv = mont_pinv(p);
-  uint64_t one, r2;
-  mont_consts(p, M.pinv, one, r2);
-  const uint64_t bmod = p > J.base ? (uint64_t)J.base : (uint64_t)J.base % p;
-  const uint64_t bm = montmul(bmod, r2, M);
-  const uint64_t x = mont_pow(bm, h.n, one, M);
-  const uint64_t km = montmul((uint64_t)h.k, r2, M);
-  const uint64_t y = montmul(montmul(x, km, M), 1, M);  // k*b^n mod p, normal form
-  const uint64_t want = J.sign < 0 ? 1 : p - 1;
-  if (y == want) {
-    const uint32_t idx = atomicAdd(hb.fac_count, 1u);
-    if (idx < hb.cap) hb.fac[idx] = h;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Hit h = hb.raw[i];
+    const uint64_t p = h.p;
+    Mont M;
+    M.p = p;
+    M.pinv = mont_pinv(p);
+    uint64_t one, r2;
+    mont_consts(p, M.pinv, one, r2);
+    const uint64_t bmod = p > J.base ? (uint64_t)J.base : (uint64_t)J.base % p;
+    const uint64_t bm = montmul(bmod, r2, M);
+    const uint64_t x = mont_pow(bm, h.n, one, M);
+    const uint64_t km = montmul((uint64_t)h.k, r2, M);
+    const uint64_t y = montmul(montmul(x, km, M), 1, M);  // k*b^n mod p, normal form
+    const uint64_t want = J.sign < 0 ? 1 : p - 1;
+    if (y == want) {
+      const uint32_t idx = atomicAdd(hb.fac_count, 1u);
+      if (idx < hb.cap) hb.fac[idx] = h;
+    }
   }
 }
 
 cudaError_t launch_verify(const JobDev &job, const HitBufs &hb, cudaStream_t st) {
-  const unsigned blocks = (hb.cap + 255) / 256;
+  const unsigned blocks = std::min(608u, (hb.cap + 255) / 256);
   verify_kernel<<<blocks, 256, 0, st>>>(job, hb);
   return cudaGetLastError();
 }
