@@ -36,20 +36,23 @@ constexpr uint32_t kNoTable = 0xffffffffu;  // no quadratic-character table for 
 //   6,7 B in normal form and its Shoup constant (the chain step),
 //   8,9 B^(32W*chain_len) likewise (chain t -> chain t+32W), 10,11 G^32 likewise,
 //   W > 1 only: 12.. B^(32w*chain_len) for w < W likewise (pairs; warp w's offset),
-//   then b likewise,
+//   then b likewise (by_res: 12,13 b likewise),
 //   el_v.. V[max_act] (giant-step start per active row), el_row.. row ids (u16,
-//   4 per element), el_tab.. B^(lane*chain_len) (32 elements, the chain starts
+//   4 per element), el_tab.. lambda*B^(lane*chain_len) (32 elements, the chain starts
 //   of warp 0), el_tab+32.. G^(lane % tlanes + 1) (32 elements).
-// Residues are in Montgomery form unless marked normal.
+// Residues are in Montgomery form unless marked normal.  Baby steps and giant
+// values carry the factor lambda = 2^64 mod p (in the chain starts, and in V or
+// Z): the filter's keys are fractions y/p, and 1, B, B^2, ... of a large p
+// would all have keys near zero.
 //
 // Integer rows (JobDev::int_rows, every row's k*b^r below 2^32): the giant value
 // of row (k, r) at step s is c*Z_s with the integer c = k*b^r and
 // Z_s = +-B^e0 * G^s (the sign of k*b^n+-1 folded in).  Then V[] holds the
-// integers c, and el_tab+32.. holds Z_(lane % tlanes + 1) times 2^128 mod p
-// instead of G^(lane % tlanes + 1) times 2^64: the kernels' normal-form
-// multiplier from_mont(entry) is then Z's Montgomery form, so Shoup's product
-// c*from_mont(entry), and equally montmul(c, entry), is the Montgomery form of
-// the giant value, as V*G^s is in the general layout.  With row_ids_only the
+// integers c, and el_tab+32.. holds Z_(lane % tlanes + 1) in Montgomery form, whose
+// product by -p^-1 mod 2^64 is Z's 64-bit fraction and Shoup constant: c times
+// it is a giant step's key, and c*Z (exact values) comes in normal form.  CTA
+// records, and by_res records of the warp layout, treat every row as the
+// integer k with the multiplier Z*b^r, so their rows always are integers.  With row_ids_only the
 // record has no V at all (el_row == el_v) and the kernels read c from row_c by
 // the row id; this halves the setup kernel's scattered stores for jobs whose V
 // would not be staged whole anyway.  With row_mask (integer rows, a warp per
@@ -63,8 +66,8 @@ constexpr uint32_t kElWoff = 12;   // warp offsets (W > 1)
 constexpr uint32_t kElV = 12;      // V in the warp-per-prime layout (W == 1)
 constexpr uint32_t kStepShoup = 0, kStepSmall = 1, kStepHigh = 2;  // ChunkBufs::small_step
 // Giant-step start values of the fast kernels (template argument): V in
-// Montgomery form, the integers k*b^r in V, k*b^r read by row id, or k*b^r of
-// the rows of an active-row mask.
+// Montgomery form, the integers k*b^r in V, k*b^r read by row id, k*b^r of the
+// rows of an active-row mask, or the integers k by residue.
 constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3, kRowsRes = 4;
 constexpr uint32_t kResMax = 8;    // residues (Q) of a by_res job at most
 constexpr uint32_t kMaskRows = 64;  // rows a row_mask record can describe

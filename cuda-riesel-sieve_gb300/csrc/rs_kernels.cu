@@ -4,7 +4,8 @@
 //                  segmented Eratosthenes over odd numbers: primes >= 65536
 //                  once per window into an L2-resident bitmap, smaller ones
 //                  per 2^15-odd segment in shared memory, then compaction; the
-//                  primes of a p-window go straight into HBM.  Replaces the
+//                  primes of a p-window go straight into HBM (in ascending order
+//                  by segment_scan_kernel and segment_emit_kernel).  Replaces the
 //                  host prime generator generateGPUPrimes
 //                  (kernel_v0.24.6.cu:1838-1987), but is complete (every
 //                  composite removed) where the reference leaves composites
@@ -17,18 +18,17 @@
 //                  integer rows (every k*b^r < 2^32) B^e0 moves into the lane
 //                  table and a start value is the integer k*b^r itself.
 //   bsgs_kernel    one prime per warp: baby steps B^j (j < m) in 64 chains of
-//                  consecutive exponents into a shared-memory table of 16-bit
-//                  tags, then giant steps for every active row, 32 lanes per
-//                  prime (kernel_v0.24.6.cu:365-620 is the per-thread,
-//                  global-memory original).  Candidate hits are checked
-//                  against the row bitmap on the device and appended with one
-//                  atomic each.
+//                  consecutive exponents into a shared-memory membership filter
+//                  keyed by 64-bit fractions, then giant steps for every active
+//                  row, 32 lanes per prime (kernel_v0.24.6.cu:365-620 is the
+//                  per-thread, global-memory original).  Candidate hits are
+//                  checked against the row bitmap on the device and appended with
+//                  one atomic each.
 //   bsgs_cta_kernel  the same with a CTA of 16 warps per prime and one large
-//                  table, for jobs with many k or wide n ranges.  Both are
-//                  instantiated per form of the start values (RM: per-prime
-//                  residues, integers in the record, integers by row id).
-//   bsgs_exact_kernel  the rare primes whose tag matches overflow the fast
-//                  path's list, with an exact (tag, j) table.
+//                  filter, for jobs with many k or wide n ranges; its tag matches
+//                  are settled by settle_kernel.
+//   bsgs_exact_kernel  the rare primes with too many suspects, with an exact
+//                  (tag, j) table.
 //   verify_kernel  direct k*b^n check of every hit (kernel_v0.24.6.cu:1649-1671).
 #include <cstdio>
 #include <type_traits>
@@ -277,7 +277,7 @@ cudaError_t launch_sieve(uint64_t lo, uint64_t hi, const uint32_t *sp, const uin
   }
   if (!seg) {
     // Below two blocks an SM a window's time is one block's: segments a quarter as
-    // long (a 1e5-wide window at 1e13: 61 -> 37 us for both passes).
+    // long (a 1e5-wide window at 1e13: 61 -> 56 us for both passes).
     constexpr int kShort = kSieveOdds / 4;
     if (blocks < 304)
       sieve_small_kernel<false, kShort><<<(unsigned)((nodd + kShort - 1) / kShort), kSieveThreads, 0, st>>>(
@@ -652,8 +652,8 @@ cudaError_t launch_jacobi_tables(const uint32_t *kodd, const uint32_t *word_off,
 }
 
 cudaError_t launch_setup(const JobDev &job, const ChunkBufs &cb, uint64_t odds, cudaStream_t st) {
-  // (the chunk has at most `odds` primes: a narrow window launched 40,000 empty
-  // blocks for its buffer's capacity, 30 of the 45 us)
+  // (the chunk has at most `odds` primes: a narrow window need not launch a block
+  // for every 128 primes its buffer could hold)
   const unsigned blocks = (unsigned)((std::min<uint64_t>(cb.cap, odds) + 127) / 128);
   setup_kernel<<<blocks, 128, 0, st>>>(job, cb);
   return cudaGetLastError();
@@ -762,6 +762,9 @@ struct LazyShort {
 // buckets), and a probe is one 4-byte load instead of a 16-byte one, which
 // random addresses cost more than twice the shared-memory wavefronts.
 // The patterns are the best of a random search for few false positives.
+// Fewer bits a key make a step cheaper and the suspects dearer: two single bits
+// measured 2.47 ns per prime against 2.38 for three on the benchmark job; two
+// rotated patterns replaced both.
 //
 // What bounds the kernel is the integer pipes: a 32x32 high or wide product takes
 // four cycles of a scheduler's multiply pipe, a low one two, an add, shift or
@@ -1664,7 +1667,7 @@ __global__ void __launch_bounds__(128) settle_kernel(JobDev J, ChunkBufs cb, Hit
 }
 
 // The exact path: a table of (tag << jbits) | j entries with linear probing per
-// prime, for the primes whose tag matches overflowed the fast path's list.  WG
+// prime, for the primes with too many suspects for the fast path.  WG
 // warps share a prime (1 for warp-per-prime jobs, kCtaWarps for CTA jobs) with
 // the same chain layout as the fast kernels.
 template <int WG>

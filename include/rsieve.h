@@ -48,9 +48,10 @@ typedef struct rs_job rs_job;
 /* rs_options.baby_step: the product by B = b^Q that advances a baby-step chain. */
 #define RS_BABY_AUTO 0   /* the cheapest valid form below */
 #define RS_BABY_SHOUP 1  /* Shoup's product by a full-size constant: valid for every prime */
-#define RS_BABY_SHORT 2  /* the short product by the integer b^Q: p > 2^33 and b^Q * p < 2^63 */
-#define RS_BABY_HIGH 3   /* Shoup's product by a 32-bit constant: b^Q * 2^32 < p, CTA-per-prime
-                            layout only (the warp layout then takes RS_BABY_SHOUP) */
+#define RS_BABY_SHORT 2  /* the short product by the integer b^Q < 2^32, with a shift chosen for the launch's
+                            range of p: up to about 2^62, and well above b^Q */
+#define RS_BABY_HIGH 3   /* the short product with the 32-bit constant b^Q * 2^64 / p: p above b^Q * 2^32 and up to
+                            about 2^62, CTA-per-prime layout only (elsewhere as RS_BABY_AUTO) */
 
 /* rs_options.char_tables: the quadratic character (k/p) of every k is read
  * from a bit table of (a/k') over a in [0, k'), k' the odd part of k, when the
@@ -108,12 +109,13 @@ typedef struct {
   uint32_t x_range;      /* floor(nmax/Q) - floor(nmin/Q) + 1 */
   uint32_t baby_steps;   /* m */
   uint32_t giant_steps;  /* T (per row) */
-  uint32_t table_slots;  /* shared-memory hash slots per prime */
+  uint32_t table_slots;  /* shared-memory table size the plan was priced with, 16-bit slots per prime */
   uint32_t primes_per_launch;
   double work_per_prime; /* algorithmic montmuls per prime: 2*sqrt(E[R]*X) */
   uint64_t upload_bytes; /* host->device bytes copied when the job was created */
   uint32_t warps_per_prime; /* 1: a warp per prime; 16: a CTA per prime (large tables) */
-  uint32_t row_form;     /* giant-step start values: 0 per-prime residues, 1 the integers
+  uint32_t row_form;     /* giant-step rows: 0 some k*b^r is 2^32 or more (per-prime residues, or the
+                            integer k with a multiplier per residue class), 1 the integers
                             k*b^r (all < 2^32) in the records, 2 k*b^r read by row id,
                             3 k*b^r of the rows of a per-prime active-row mask (at most
                             64 rows, a warp per prime) */
@@ -139,8 +141,8 @@ typedef struct {
   uint64_t d2h_bytes;    /* device->host bytes the call copied */
   uint64_t primes_by_step[3]; /* primes whose baby steps used RS_BABY_SHOUP, _SHORT, _HIGH
                             (index = form - 1) */
-  uint64_t paired_primes; /* primes whose active rows came in (k, 0), (k, 1) pairs, the
-                            second giant value of each pair formed by the short product by b */
+  uint64_t paired_primes; /* primes whose active rows came in (k, 0), (k, 1) pairs (start values
+                            that are residues form the second value by the short product by b) */
   uint64_t exact_primes; /* primes finished by the exact (tag, j) table path */
 } rs_stats;
 
