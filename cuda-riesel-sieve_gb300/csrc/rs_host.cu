@@ -522,10 +522,9 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
         // V staging: the integers k*b^r read by row id (two bytes a row) when a lane takes
         // two or more giant steps, else eight bytes a row (the row form of plan_row_form)
         const double vbytes = (ints_q && T >= 64 ? 2.0 : 8.0) * (rows + 2) + 16.0;
-        // buckets: a power of two with at most ~2 entries each, or, when that table does
+        // table size, in the units the plan reports (the filter takes what the shared
+        // memory leaves): a power of two of at most ~2 baby steps a unit, or, when that does
         // not fit the shared memory, the smallest multiple of 64 with at most ~2 each.
-        // (Tables at ~3 entries a bucket measured slower on the wide job, 183-216 against
-        // 174 ns per prime: more full buckets and more false tag matches.)
         const uint32_t blog = std::max<uint32_t>(4, ilog2_ceil((m + 1) / 2));
         const uint32_t nb_opts[2] = {1u << blog, (uint32_t)std::max<uint64_t>(64, ((m + 1) / 2 + 63) / 64 * 64)};
         for (int o = 0; o < 2; o++) {
@@ -535,7 +534,6 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
           if (o == 1 && (nbk >= nb_opts[0] || nbk > 65536 || 20.0 * nb_opts[0] + vbytes + 16.0 * (kCtaMatchCap + 1) <= kCtaSmemMax))
             continue;
           const double fp = ER * (double)T * ((double)m / nb) / 65536.0;
-          // (m < 2^16: a bucket's insert count is the low half of its count word)
           if (m <= mcap && m < 65536 && m * T >= X && slog <= 17 && smem <= kCtaSmemMax && fp <= 16.0) {
             const double cost = ((double)m / 32.0 + kGiantWeight * kCtaWarps * std::ceil(ER / kCtaWarps) * spl +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
@@ -714,7 +712,8 @@ struct rs_job {
   void *d_chunk = nullptr;
   uint32_t *h_counts = nullptr;  // pinned, one slot per chunk + 2
   size_t h_counts_cap = 0;
-  uint32_t chunk_cap = 0;
+  uint32_t chunk_cap = 0;        // primes the chunk buffers hold
+  uint32_t launch_cap = 0;       // primes per launch at most (rs_job_info.primes_per_launch)
   uint32_t chunk_rec_elems = 0;  // record elements the chunk buffers were sized for
   uint64_t chunk_exact_bytes = 0;  // exact-kernel scratch they hold
   bool has_cta() const {
@@ -1332,7 +1331,25 @@ static void set_chunk_cap(rs_job *j) {
   }
   cap = std::max<uint64_t>(cap, 4096);
   cap = std::min<uint64_t>(cap, 1u << 23);
-  j->cb.cap = (uint32_t)cap;
+  j->launch_cap = (uint32_t)cap;
+}
+
+// Primes per launch for one call's range: a window that fits one launch of 2^21
+// primes gets buffers for itself, one of up to four launches a quarter each.
+// Mapping and unmapping the 3 GB of full-size buffers took 7 of the 25 ms of a
+// one-shot run over 2e8 at 1e13 and 2 of the 2.9 ms of a job's first narrow call.
+// (-b/-t fix the launch size, so they keep it.)
+static uint32_t call_cap(const rs_job *j, uint64_t lo, uint64_t hi) {
+  if (j->opt.block_scale > 0 || j->opt.thread_scale > 0) return j->launch_cap;
+  const double need = 1.35 * primes_estimate(lo, hi) + 4096.0, one = 1 << 21;
+  const double cap = need <= one ? need : std::max(one, need / 4);
+  return cap < (double)j->launch_cap ? (uint32_t)cap : j->launch_cap;
+}
+// Buffers for the range; what an earlier call left may be larger.
+static int ensure_call_buffers(rs_job *j, uint64_t lo, uint64_t hi) {
+  const int rc = ensure_chunk_buffers(j, call_cap(j, lo, hi));
+  if (!rc) j->cb.cap = std::min(j->chunk_cap, j->launch_cap);
+  return rc;
 }
 
 // Upload and configure one planned part.
@@ -1483,7 +1500,7 @@ int rs_job_info_get(const rs_job *j, rs_job_info *info) {
   info->baby_steps = pl.m;
   info->giant_steps = pl.T;
   info->table_slots = (uint32_t)kBucket * pl.nbuckets;
-  info->primes_per_launch = j->cb.cap;
+  info->primes_per_launch = j->launch_cap;
   info->work_per_prime = pl.work_per_prime;
   info->warps_per_prime = pl.cta ? kCtaWarps : 1;
   info->row_form = plan_row_form(pl, p0.seqs, nullptr);
@@ -1595,7 +1612,7 @@ static int sieve_range_impl(rs_job *j, uint64_t p0, uint64_t p1, rs_factor *out,
   CUDA_TRY(cudaSetDevice(j->device));
   int rc = ensure_sieving_primes(j, hi, &st.h2d_bytes);
   if (rc) return rc;
-  rc = ensure_chunk_buffers(j, j->cb.cap);
+  rc = ensure_call_buffers(j, lo, hi);
   if (rc) return rc;
   const size_t P = j->parts.size();
   for (auto &pt : j->parts) {
@@ -2032,7 +2049,7 @@ extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
   for (Run &r : runs) {
     rs_job *j = r.j;
     int rc = ensure_sieving_primes(j, r.hi, &tot.h2d_bytes);
-    if (!rc) rc = ensure_chunk_buffers(j, j->cb.cap);
+    if (!rc) rc = ensure_call_buffers(j, r.lo, r.hi);
     if (!rc && !r.pt->d_hits) rc = ensure_hit_buffers(j, *r.pt, 1u << 20);
     if (!rc) rc = build_char_tables(j, *r.pt, primes_estimate(r.lo, r.hi), false);
     if (rc) return rc;
