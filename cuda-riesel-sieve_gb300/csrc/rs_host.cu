@@ -825,32 +825,75 @@ static double primes_estimate(uint64_t a, uint64_t b) {
   return (double)(b - a + 1) / std::log((double)std::max<uint64_t>(b, 16));
 }
 
-// Build the character tables of a part that pay for themselves: every table
-// when `all`, else those whose k' is at most the primes the part has sieved,
-// counting `primes_more` (the estimate of the range about to be sieved) -- a
-// table costs one Jacobi symbol per entry, and saves one per prime sieved.
-// The per-k table offsets on the device (and the base's, in the part's
-// JobDev) follow, on the job's stream, ahead of the setup launches.
+// Build the character tables of a part that pay for themselves (every table when
+// `all`), for the primes the part has sieved, counting `primes_more` (the
+// estimate of the range about to be sieved).  A table saves kCharSave a prime (1000
+// k at 2^50: setup 24.1 ns per prime without tables, 11.4 with all).  From squares
+// it costs kSquareEntry an entry and segment of k', the longest CTA
+// kSquareChain an entry, and kSquareCall a call (1000 tables of k' up to 10^7:
+// 3.1 ms); by the Jacobi symbol of each entry kJacobiEntry (76 ms).  So
+// tables from squares come when half of what they save covers their entries and all
+// of it the launch; else those of k' at most the primes are built by symbols, which
+// also take less time for one or two large k'.  The per-k table offsets on the
+// device (and the base's, in the part's JobDev) follow, on the job's stream, ahead
+// of the setup launches.
+constexpr double kCharSave = 12.8e-6, kSquareEntry = 0.14e-6, kSquareChain = 21e-6, kSquareCall = 20.0;  // us
+constexpr double kJacobiEntry = 14e-6, kJacobiCall = 15.0;
 static int build_char_tables(rs_job *j, Part &pt, double primes_more, bool all) {
   if (pt.tab_k.empty()) return RS_OK;
   pt.primes_seen += primes_more;
-  std::vector<uint32_t> sel, first;
+  const double save = kCharSave * pt.primes_seen;
+  std::vector<uint32_t> sel, square, first;
   uint64_t words = 0;
-  for (size_t t = 0; t < pt.tab_k.size(); t++)
-    if (!pt.tab_built[t] && (all || (double)pt.tab_k[t] <= pt.primes_seen)) {
-      sel.push_back((uint32_t)t);
-      first.push_back((uint32_t)words);
-      words += (pt.tab_k[t] + 31) / 32;
+  double sq_net = 0.0, sq_max = 0.0, sel_net = 0.0;
+  for (size_t t = 0; t < pt.tab_k.size(); t++) {
+    if (pt.tab_built[t]) continue;
+    const double k = pt.tab_k[t], sq = kSquareEntry * k * (1.0 + std::floor(k / kSquareSeg));
+    if (pt.tab_k[t] <= kSquareMaxK && (all || sq <= 0.5 * save)) {
+      square.push_back((uint32_t)t);
+      sq_net += (all ? 0.0 : save) - sq;
+      sq_max = std::max(sq_max, kSquareChain * k - sq);
     }
-  if (sel.empty()) return RS_OK;
+    if (all || k <= pt.primes_seen) {
+      sel.push_back((uint32_t)t);
+      sel_net += (all ? 0.0 : save) - kJacobiEntry * k;
+    }
+  }
+  sq_net -= sq_max + kSquareCall;
+  if (!sel.empty()) sel_net -= kJacobiCall;
+  if (sq_net > sel_net) {  // the rest of the selection, if any, by symbols
+    sel.erase(std::remove_if(sel.begin(), sel.end(), [&](uint32_t t) { return pt.tab_k[t] <= kSquareMaxK; }), sel.end());
+  } else {
+    square.clear();
+  }
+  if (sel.empty() && square.empty()) return RS_OK;
+  // (the largest first: theirs are the longest CTAs)
+  std::sort(square.begin(), square.end(), [&](uint32_t x, uint32_t y) { return pt.tab_k[x] > pt.tab_k[y]; });
+  for (uint32_t t : sel) {
+    first.push_back((uint32_t)words);
+    words += (pt.tab_k[t] + 31) / 32;
+  }
+  std::vector<uint32_t> seg, seg_w0;  // segments of the tables from squares
+  for (uint32_t t : square)
+    for (uint32_t w = 0; w < (pt.tab_k[t] + 31) / 32; w += kSquareSeg / 32) {
+      seg.push_back(t);
+      seg_w0.push_back(w);
+    }
   std::vector<uint32_t> args(sel);
   args.insert(args.end(), first.begin(), first.end());
+  args.insert(args.end(), seg.begin(), seg.end());
+  args.insert(args.end(), seg_w0.begin(), seg_w0.end());
   uint32_t *d_args = nullptr;
   CUDA_TRY(cudaMallocAsync((void **)&d_args, args.size() * 4, j->st));
   cudaError_t e = cudaMemcpyAsync(d_args, args.data(), args.size() * 4, cudaMemcpyHostToDevice, j->st);
   if (e == cudaSuccess)
     e = launch_jacobi_tables(pt.d_tab_k, pt.d_tab_off, d_args, d_args + sel.size(), (uint32_t)sel.size(),
                              (uint32_t)words, pt.d_jac_bits, j->st);
+  if (e == cudaSuccess && !square.empty())
+    e = launch_square_tables(pt.d_tab_k, pt.d_tab_off, d_args + 2 * sel.size(),
+                             d_args + 2 * sel.size() + seg.size(), (uint32_t)seg.size(), pt.tab_k[square[0]],
+                             pt.d_jac_bits, j->st);
+  sel.insert(sel.end(), square.begin(), square.end());
   cudaFreeAsync(d_args, j->st);
   if (e != cudaSuccess) return fail(RS_ERR_CUDA, "character tables: %s", cudaGetErrorString(e));
   for (uint32_t t : sel) pt.tab_built[t] = 1;

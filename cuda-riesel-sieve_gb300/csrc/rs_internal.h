@@ -253,6 +253,12 @@ cudaError_t launch_bsgs_batch(const JobDev &rep, const BatchItem *items, uint32_
 cudaError_t launch_jacobi_tables(const uint32_t *kodd, const uint32_t *word_off, const uint32_t *sel,
                                  const uint32_t *first, uint32_t nsel, uint32_t total_words, uint32_t *bits,
                                  cudaStream_t st);
+// The same tables from squares mod the primes of k' <= kSquareMaxK, a CTA for
+// each segment of kSquareSeg bits: table sel[i] from word w0[i] on.  kmax is the
+// largest k' of the selection.
+constexpr uint32_t kSquareSeg = 1760000, kSquareMaxK = 1u << 25;
+cudaError_t launch_square_tables(const uint32_t *kodd, const uint32_t *word_off, const uint32_t *sel,
+                                 const uint32_t *w0, uint32_t nseg, uint32_t kmax, uint32_t *bits, cudaStream_t st);
 // Record an error for rs_last_error() and return code (rs_host.cu).
 int set_error(int code, const char *fmt, ...);
 

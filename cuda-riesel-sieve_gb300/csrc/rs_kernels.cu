@@ -618,7 +618,8 @@ __global__ void __launch_bounds__(128) setup_kernel(JobDev J, ChunkBufs cb) {
 // Quadratic-character tables: word w of the table of odd k' holds bit t =
 // ((32*w + t) / k') == +1 (Jacobi symbol), for 32*w + t < k'.  One launch
 // builds the tables sel[0..nsel) of the job's list (odd parts kodd[], word
-// offsets word_off[]); thread g writes word g - first[i] of table sel[i], where
+// offsets word_off[]), for k' too large for square_table_kernel and for
+// selections too small for it; thread g writes word g - first[i] of table sel[i], where
 // first[] are the running word counts of the selected tables.
 __global__ void jacobi_table_kernel(const uint32_t *kodd, const uint32_t *word_off, const uint32_t *sel,
                                     const uint32_t *first, uint32_t nsel, uint32_t total_words, uint32_t *bits) {
@@ -642,12 +643,100 @@ __global__ void jacobi_table_kernel(const uint32_t *kodd, const uint32_t *word_o
   bits[word_off[t] + w] = out;
 }
 
+// The same tables from squares: (a/k') is the product of (a/q) over the primes q
+// that divide k' to an odd power, and the residues mod q are the squares 1, 4,
+// 9, ..., two additions and a shared-memory bit apiece, against a binary-gcd loop
+// of some twenty rounds an entry above.  A CTA makes the words from w0[] on of its
+// table, at most kSquareSeg bits; a q with more residues than that goes through all its
+// squares for each segment and keeps the ones there.
+//   [residues mod q from `base` on as bits, 32 more than the segment or q (periodic)]
+// XOR of their complements, 32 entries at a time, gives the table; entries with
+// a common factor stay 0.
+// Bound by the integer pipes (eight instructions a square): 1000 tables of k' up to
+// 10^7 take 3.1 ms, by symbols 76; a table's longest CTA about 21 ps an entry.
+__global__ void __launch_bounds__(1024, 1) square_table_kernel(const uint32_t *kodd, const uint32_t *word_off,
+                                                               const uint32_t *sel, const uint32_t *w0s,
+                                                               uint32_t *bits) {
+  extern __shared__ uint32_t res[];
+  __shared__ uint32_t next, primes[10];
+  const uint32_t tid = threadIdx.x, NT = blockDim.x;
+  const uint32_t t = sel[blockIdx.x], k = kodd[t], w0 = w0s[blockIdx.x];
+  const uint32_t w1 = min(w0 + kSquareSeg / 32, (k + 31) / 32);
+  uint32_t *out = bits + word_off[t];
+  for (uint32_t w = w0 + tid; w < w1; w += NT) out[w] = 0xffffffffu;
+  uint32_t n = k, from = 3, np = 0;  // what is left of k', whose prime factors are all >= from
+  while (n > 1) {
+    if (tid == 0) next = n;
+    __syncthreads();
+    for (uint32_t d = from + 2 * tid; d * d <= n; d += 2 * NT)
+      if (n % d == 0) {
+        atomicMin(&next, d);
+        break;
+      }
+    __syncthreads();
+    const uint32_t q = next;
+    bool odd = false;
+    do {
+      n /= q;
+      odd = !odd;
+    } while (n % q == 0);
+    from = q + 2;
+    if (tid == 0) primes[np] = q;
+    np++;
+    if (odd) {
+      const bool whole = q <= kSquareSeg;
+      const uint32_t base = whole ? 0 : (uint32_t)((uint64_t)w0 * 32 % q);
+      const uint32_t span = (whole ? q : 32 * (w1 - w0)) + 32;  // bits kept, at most kSquareSeg + 32
+      for (uint32_t w = tid; w < (span + 31) / 32; w += NT) res[w] = 0;
+      __syncthreads();
+      // x = tid + 1 + i*NT: x^2 - base mod q by its differences
+      const uint32_t half = (q - 1) / 2, x0 = tid + 1;
+      if (x0 <= half) {
+        const uint32_t d2 = (uint32_t)(2ull * NT * NT % q);
+        uint32_t y = (uint32_t)(((uint64_t)x0 * x0 + q - base) % q), c = (uint32_t)((2ull * x0 + NT) * NT % q);
+        for (uint32_t x = x0; x <= half; x += NT) {
+          for (uint32_t e = y; e < span; e += q) atomicOr(&res[e >> 5], 1u << (e & 31));
+          y += c;
+          y = min(y, y - q);
+          c += d2;
+          c = min(c, c - q);
+        }
+      }
+      __syncthreads();
+      for (uint32_t w = w0 + tid; w < w1; w += NT) {
+        const uint32_t off = whole ? 32 * w % q : 32 * (w - w0), i = off >> 5;
+        out[w] ^= ~__funnelshift_r(res[i], res[i + 1], off);
+      }
+    }
+    __syncthreads();
+  }
+  for (uint32_t w = w0 + tid; w < w1; w += NT) {
+    uint32_t clear = 32 * w + 32 > k ? ~((1u << (k & 31)) - 1) : 0;
+    for (uint32_t i = 0; i < np; i++) {
+      const uint32_t q = primes[i], off = 32 * w % q;
+      for (uint32_t b = off ? q - off : 0; b < 32; b += q) clear |= 1u << b;
+    }
+    out[w] &= ~clear;
+  }
+}
+
 cudaError_t launch_jacobi_tables(const uint32_t *kodd, const uint32_t *word_off, const uint32_t *sel,
                                  const uint32_t *first, uint32_t nsel, uint32_t total_words, uint32_t *bits,
                                  cudaStream_t st) {
   if (total_words == 0 || nsel == 0) return cudaSuccess;
   jacobi_table_kernel<<<(total_words + 255) / 256, 256, 0, st>>>(kodd, word_off, sel, first, nsel, total_words,
                                                                  bits);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_square_tables(const uint32_t *kodd, const uint32_t *word_off, const uint32_t *sel,
+                                 const uint32_t *w0, uint32_t nseg, uint32_t kmax, uint32_t *bits, cudaStream_t st) {
+  if (nseg == 0) return cudaSuccess;
+  const uint32_t smem = std::min(kmax, kSquareSeg) / 32 * 4 + 12;
+  const cudaError_t e = cudaFuncSetAttribute((const void *)square_table_kernel,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSquareSeg / 32 * 4 + 12);
+  if (e != cudaSuccess) return e;
+  square_table_kernel<<<nseg, 1024, smem, st>>>(kodd, word_off, sel, w0, bits);
   return cudaGetLastError();
 }
 

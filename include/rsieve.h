@@ -55,11 +55,11 @@ typedef struct rs_job rs_job;
 
 /* rs_options.char_tables: the quadratic character (k/p) of every k is read
  * from a bit table of (a/k') over a in [0, k'), k' the odd part of k, when the
- * table exists, else computed (a Jacobi symbol per prime and k).  A table costs
- * one Jacobi symbol per entry to build on the device, so it pays once the job
- * has sieved more primes than k'. */
+ * table exists, else computed (a Jacobi symbol per prime and k).  A table is
+ * built on the device, a few percent of a Jacobi symbol an entry, or for one or
+ * two large k' a symbol an entry. */
 #define RS_TABLES_AUTO 0    /* build each table when the primes the job has sieved, with
-                               those of the range about to be sieved, reach its k' */
+                               the call's range counted, pay for it */
 #define RS_TABLES_ALWAYS 1  /* build every table when the job is created */
 #define RS_TABLES_NEVER 2   /* no tables: compute every character */
 
