@@ -927,6 +927,22 @@ static uint32_t warp_filter(uint32_t m, uint32_t fixed, uint32_t static_smem, ui
 }
 static uint32_t filter_shift(uint32_t words) { return std::max(11u, std::min(16u, 27 - ilog2_ceil(words))); }
 
+// Whether two CTAs of the CTA kernel share an SM: their filters must then keep
+// two words a baby step, and more with the probes of a prime, whose false
+// positives grow.  Two CTAs hide each other's barriers and one-warp passes: 467 k,
+// m = 7168, T = 64 takes 47.1 ns per prime against 52.5 with one; 78 k, m = 5120
+// 22.2 against 27.4; 106 k, m = 11264 (2.05 words) 31.4 against 35.0.  With
+// 128,000 probes (1000 k, m = 8192, T = 128, 2.7 words) 138 against 133, and
+// at 1.5 words (467 k, m = 14336) 61 against 55.
+static bool cta_pair(uint32_t m, uint64_t fixed, uint32_t row_slots, double probes) {
+  const double words = std::min(3.5, ((double)kCtaPairSmem - (double)(fixed + 4ull * row_slots)) / 4.0 / m);
+  return words >= 2.0 && probes <= 8192.0 * words * words;
+}
+// Bytes of a CTA beside its filter and its rows' k: tags, row ids, suspects and keys, counts.
+static uint64_t cta_fixed(uint32_t m, uint32_t row_slots, uint32_t Q) {
+  return align_up(2ull * m + 2ull * row_slots + 20ull * kCtaMatchCap + 4ull * Q + 16, 16);
+}
+
 static int upload_part(rs_job *j, Part &pt) {
   const Plan &pl = pt.plan;
   const Seqs &s = pt.seqs;
@@ -1119,15 +1135,17 @@ static int upload_part(rs_job *j, Part &pt) {
     d.stage_full = 0;
     d.stage_elems = d.el_v;
   }
-  d.ctab_smem = 0;
+  d.cta_pair = d.ctab_smem = 0;
   if (d.cta_warps > 1) {
     // bytes per CTA: tags, the rows' ids and (when 1.5 filter words a baby step
     // still fit) their k, suspects and keys, counts; the filter takes the rest up
     // to 3.5 words a baby step
-    const uint64_t fixed = align_up(2ull * pl.m + 2ull * row_slots + 20ull * kCtaMatchCap + 4ull * pl.Q + 16, 16);
-    d.ctab_smem = fixed + 4ull * row_slots + 6ull * pl.m <= kCtaSmemMax ? 1u : 0u;
+    const uint64_t fixed = cta_fixed(pl.m, row_slots, pl.Q);
+    d.cta_pair = cta_pair(pl.m, fixed, row_slots, pl.nrows * ((pl.Q & 1) ? 0.75 : 0.5) * pl.T) ? 1u : 0u;
+    const uint64_t smem_max = d.cta_pair ? kCtaPairSmem : kCtaSmemMax;
+    d.ctab_smem = fixed + 4ull * row_slots + 6ull * pl.m <= smem_max ? 1u : 0u;
     const uint64_t used = fixed + (d.ctab_smem ? 4ull * row_slots : 0);
-    const uint64_t left = used < kCtaSmemMax ? (kCtaSmemMax - used) / 16 * 4 : 0;
+    const uint64_t left = used < smem_max ? (smem_max - used) / 16 * 4 : 0;
     d.fwords = (uint32_t)std::min<uint64_t>({left, 65532, std::max<uint64_t>(1024, (7ull * pl.m / 2 + 3) & ~3ull)});
     if (d.fwords < 256) return fail(RS_ERR_INVALID, "a CTA plan's rows leave no shared memory for its filter");
     d.fshift = filter_shift(d.fwords);

@@ -86,6 +86,8 @@ struct __align__(16) KInfo {
 // Shared memory of the warp-per-prime kernels: an SM's, what a CTA reserves, its
 // allocation granule, and the CTAs of four warps that registers allow on an SM.
 constexpr uint32_t kSmemPerSm = 233472, kSmemReserved = 1024, kSmemGranule = 1024, kWarpCtas = 5;
+// Bytes of each of two CTAs of the CTA kernel on an SM.
+constexpr uint32_t kCtaPairSmem = (kSmemPerSm / 2 - kSmemReserved) / kSmemGranule * kSmemGranule;
 // Bytes a warp needs beside its filter: tags, two record stages, V of a row mask or the residues' row lists.
 inline uint32_t warp_kernel_fixed(uint32_t chain_len, uint32_t stage_elems, bool row_mask, bool by_res,
                                   uint32_t row_slots) {
@@ -135,6 +137,7 @@ struct JobDev {
   uint32_t warp_smem;    // shared-memory bytes per warp (bsgs_kernel) or per CTA (bsgs_cta_kernel)
   uint32_t exact_log2;   // slots of the exact kernel's table = 1 << exact_log2
   uint32_t exact_global; // that table exceeds shared memory: it lives in ChunkBufs::exact_tab
+  uint32_t cta_pair;     // CTA kernel: shared memory for two CTAs per SM
   uint32_t ctab_smem;    // CTA kernel: the k of the active rows are kept in shared memory beside their ids
   // device arrays
   const uint32_t *row_r;     // [nrows] n mod Q of each row
