@@ -393,6 +393,22 @@ struct PlanChoice {
   uint32_t nb = 0;  // table size, as Plan::nbuckets
 };
 
+// Whether two CTAs of the CTA kernel share an SM: their filters must then keep
+// two words a baby step, and more with the probes of a prime, whose false
+// positives grow.  Two CTAs hide each other's barriers and one-warp passes: 467 k,
+// m = 7168, T = 64 takes 47.1 ns per prime against 52.5 with one; 78 k, m = 5120
+// 22.2 against 27.4; 106 k, m = 11264 (2.05 words) 31.4 against 35.0.  With
+// 128,000 probes (1000 k, m = 8192, T = 128, 2.7 words) 138 against 133, and
+// at 1.5 words (467 k, m = 14336) 61 against 55.
+static bool cta_pair(uint32_t m, uint64_t fixed, uint32_t row_slots, double probes) {
+  const double words = std::min(3.5, ((double)kCtaPairSmem - (double)(fixed + 4ull * row_slots)) / 4.0 / m);
+  return words >= 2.0 && probes <= 8192.0 * words * words;
+}
+// Bytes of a CTA beside its filter and its rows' k: tags, row ids, suspects and keys, counts.
+static uint64_t cta_fixed(uint32_t m, uint32_t row_slots, uint32_t Q) {
+  return align_up(2ull * m + 2ull * row_slots + 20ull * kCtaMatchCap + 4ull * Q + 16, 16);
+}
+
 // Plan a job.  With `force`, take exactly that choice (it must be feasible);
 // with `ranked`, also return every feasible choice, cheapest first.
 static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_bitmap = true,
@@ -440,7 +456,51 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
   // A step of the CTA kernel costs more than one of the warp kernel (block-wide
   // barriers, per-prime tag-match passes); fitted with rs_job_autotune on mixed jobs.
   constexpr double kCtaStepCost = 1.25;
+  // The CTA plans among themselves, in ns per prime: measured on jobs of 78 to 1000 k
+  // at 15 plans, to about 12%, with two CTAs per SM and with one.  The
+  // cost above weighs the cheapest against the warp plans, but takes T = 32, m =
+  // 14336 for 467 k (55.0 ns) before T = 64, m = 7168 (47.1).
+  struct CtaPlan {
+    uint32_t Q;
+    int rows;
+    uint32_t X;
+    double ER;
+    uint64_t T, m;
+    uint32_t nb, slog;
+    double cost, ns;
+  };
+  std::vector<CtaPlan> cta_plans;
+  auto cta_ns = [](uint32_t m, double ER, int rows, uint32_t Q, uint64_t T) {
+    const uint32_t slots = (uint32_t)rows + 4 * Q + 8;
+    const bool two = cta_pair(m, cta_fixed(m, slots, Q), slots, ER * (double)T);
+    const double giants = ER * (double)T / 32.0;
+    return (two ? 12.0 + 1.3 * m / 1024.0 + 0.0255 * giants : 10.7 + 2.26 * m / 1024.0 + 0.028 * giants) + 0.01 * rows;
+  };
   double best = 1e300;
+  auto consider = [&](uint32_t Q, int rows, uint32_t X, double ER, bool cta, uint64_t T, uint64_t m, uint32_t nb,
+                      uint32_t slog, double cost) {
+    if (ranked) ranked->push_back(PlanChoice{Q, (uint32_t)T, (uint32_t)m, cta, cost, nb});
+    if (force) {
+      if (force->Q != Q || force->T != T || force->m != m || force->cta != cta || force->nb != nb) return;
+      cost = -1.0;  // the forced choice wins
+    }
+    if (cost < best) {
+      best = cost;
+      pl.Q = Q;
+      pl.nrows = (uint32_t)rows;
+      pl.X = X;
+      pl.m = (uint32_t)m;
+      pl.T = (uint32_t)T;
+      pl.tlanes = (uint32_t)std::min<uint64_t>(T, 32);
+      pl.rows_per_it = 32 / pl.tlanes;
+      pl.steps_per_lane = (uint32_t)std::max<uint64_t>(1, T / 32);
+      pl.table_log2 = slog;
+      pl.nbuckets = nb;
+      pl.cta = cta;
+      pl.cost = cost;
+      pl.work_per_prime = 2.0 * std::sqrt(ER * (double)X);
+    }
+  };
   for (uint32_t Q : Qs) {
     const uint32_t X = nmax / Q - nmin / Q + 1;
     const int rows = count_rows(s, Q, datless);
@@ -456,29 +516,6 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
     }
     const bool short_q = Q * std::log2((double)s.base) < 31.0;  // b^Q as the short product's integer
     const bool res_q = rows_by_residue(Q, s.k.size(), (size_t)rows);
-    auto consider = [&](bool cta, uint64_t T, uint64_t m, uint32_t nb, uint32_t slog, double cost) {
-      if (ranked) ranked->push_back(PlanChoice{Q, (uint32_t)T, (uint32_t)m, cta, cost, nb});
-      if (force) {
-        if (force->Q != Q || force->T != T || force->m != m || force->cta != cta || force->nb != nb) return;
-        cost = -1.0;  // the forced choice wins
-      }
-      if (cost < best) {
-        best = cost;
-        pl.Q = Q;
-        pl.nrows = (uint32_t)rows;
-        pl.X = X;
-        pl.m = (uint32_t)m;
-        pl.T = (uint32_t)T;
-        pl.tlanes = (uint32_t)std::min<uint64_t>(T, 32);
-        pl.rows_per_it = 32 / pl.tlanes;
-        pl.steps_per_lane = (uint32_t)std::max<uint64_t>(1, T / 32);
-        pl.table_log2 = slog;
-        pl.nbuckets = nb;
-        pl.cta = cta;
-        pl.cost = cost;
-        pl.work_per_prime = 2.0 * std::sqrt(ER * (double)X);
-      }
-    };
     for (uint32_t tl = 0; tl <= 20; tl++) {
       const uint64_t T = (uint64_t)1 << tl;
       const uint64_t m0 = (X + T - 1) / T;
@@ -510,7 +547,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
                                  kStepCost * (spl - 1) + (few && !ints_q && res_q ? kResidueCost * Q * spl : 0.0) +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
                                 std::sqrt(kFullWarps / warps);
-            consider(false, T, m, 1u << blog, slog, cost);
+            consider(Q, rows, X, ER, false, T, m, 1u << blog, slog, cost);
           }
         }
       }
@@ -538,12 +575,19 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
             const double cost = ((double)m / 32.0 + kGiantWeight * kCtaWarps * std::ceil(ER / kCtaWarps) * spl +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
                                 std::sqrt(kFullWarps / kCtaWarps) * kCtaStepCost * (few ? kCtaFew : 1.0);
-            consider(true, T, m, nbk, slog, cost);
+            cta_plans.push_back({Q, rows, X, ER, T, m, nbk, slog, cost, cta_ns((uint32_t)m, ER, rows, Q, T)});
           }
         }
       }
     }
   }
+  double cta_cost = 1e300, cta_min = 1e300;
+  for (const CtaPlan &c : cta_plans) {
+    cta_cost = std::min(cta_cost, c.cost);
+    cta_min = std::min(cta_min, c.ns);
+  }
+  for (const CtaPlan &c : cta_plans)
+    consider(c.Q, c.rows, c.X, c.ER, true, c.T, c.m, c.nb, c.slog, cta_cost * c.ns / cta_min);
   if (ranked)
     std::sort(ranked->begin(), ranked->end(), [](const PlanChoice &a, const PlanChoice &b) { return a.cost < b.cost; });
   if (pl.Q == 0) return fail(RS_ERR_INVALID, "no feasible plan (n range too wide for the -m limit)");
@@ -926,22 +970,6 @@ static uint32_t warp_filter(uint32_t m, uint32_t fixed, uint32_t static_smem, ui
   return words > 2048 && words < 2200 ? 2048 : words;
 }
 static uint32_t filter_shift(uint32_t words) { return std::max(11u, std::min(16u, 27 - ilog2_ceil(words))); }
-
-// Whether two CTAs of the CTA kernel share an SM: their filters must then keep
-// two words a baby step, and more with the probes of a prime, whose false
-// positives grow.  Two CTAs hide each other's barriers and one-warp passes: 467 k,
-// m = 7168, T = 64 takes 47.1 ns per prime against 52.5 with one; 78 k, m = 5120
-// 22.2 against 27.4; 106 k, m = 11264 (2.05 words) 31.4 against 35.0.  With
-// 128,000 probes (1000 k, m = 8192, T = 128, 2.7 words) 138 against 133, and
-// at 1.5 words (467 k, m = 14336) 61 against 55.
-static bool cta_pair(uint32_t m, uint64_t fixed, uint32_t row_slots, double probes) {
-  const double words = std::min(3.5, ((double)kCtaPairSmem - (double)(fixed + 4ull * row_slots)) / 4.0 / m);
-  return words >= 2.0 && probes <= 8192.0 * words * words;
-}
-// Bytes of a CTA beside its filter and its rows' k: tags, row ids, suspects and keys, counts.
-static uint64_t cta_fixed(uint32_t m, uint32_t row_slots, uint32_t Q) {
-  return align_up(2ull * m + 2ull * row_slots + 20ull * kCtaMatchCap + 4ull * Q + 16, 16);
-}
 
 static int upload_part(rs_job *j, Part &pt) {
   const Plan &pl = pt.plan;
