@@ -404,9 +404,15 @@ static bool cta_pair(uint32_t m, uint64_t fixed, uint32_t row_slots, double prob
   const double words = std::min(3.5, ((double)kCtaPairSmem - (double)(fixed + 4ull * row_slots)) / 4.0 / m);
   return words >= 2.0 && probes <= 8192.0 * words * words;
 }
+// Suspects a CTA has room for: twice what the fullest filters leave of a prime's
+// probes.  (Sixty-four, the room of the jobs with up to 80,000 probes, sent every
+// prime of 8000 k with 512,000 to the exact path.)
+static uint32_t cta_match_cap(double probes) {
+  return std::max<uint32_t>(kCtaMatchCap, ((uint32_t)std::min(1024.0, 8e-4 * probes) + 3) & ~3u);
+}
 // Bytes of a CTA beside its filter and its rows' k: tags, row ids, suspects and keys, counts.
-static uint64_t cta_fixed(uint32_t m, uint32_t row_slots, uint32_t Q) {
-  return align_up(2ull * m + 2ull * row_slots + 20ull * kCtaMatchCap + 4ull * Q + 16, 16);
+static uint64_t cta_fixed(uint32_t m, uint32_t row_slots, uint32_t Q, double probes) {
+  return align_up(2ull * m + 2ull * row_slots + 20ull * cta_match_cap(probes) + 4ull * Q + 16, 16);
 }
 
 // Plan a job.  With `force`, take exactly that choice (it must be feasible);
@@ -472,7 +478,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
   std::vector<CtaPlan> cta_plans;
   auto cta_ns = [](uint32_t m, double ER, int rows, uint32_t Q, uint64_t T) {
     const uint32_t slots = (uint32_t)rows + 4 * Q + 8;
-    const bool two = cta_pair(m, cta_fixed(m, slots, Q), slots, ER * (double)T);
+    const bool two = cta_pair(m, cta_fixed(m, slots, Q, ER * (double)T), slots, ER * (double)T);
     const double giants = ER * (double)T / 32.0;
     return (two ? 12.0 + 1.3 * m / 1024.0 + 0.0255 * giants : 10.7 + 2.26 * m / 1024.0 + 0.028 * giants) + 0.01 * rows;
   };
@@ -1163,13 +1169,15 @@ static int upload_part(rs_job *j, Part &pt) {
     d.stage_full = 0;
     d.stage_elems = d.el_v;
   }
-  d.cta_pair = d.ctab_smem = 0;
+  d.match_cap = d.cta_pair = d.ctab_smem = 0;
   if (d.cta_warps > 1) {
     // bytes per CTA: tags, the rows' ids and (when 1.5 filter words a baby step
     // still fit) their k, suspects and keys, counts; the filter takes the rest up
     // to 3.5 words a baby step
-    const uint64_t fixed = cta_fixed(pl.m, row_slots, pl.Q);
-    d.cta_pair = cta_pair(pl.m, fixed, row_slots, pl.nrows * ((pl.Q & 1) ? 0.75 : 0.5) * pl.T) ? 1u : 0u;
+    const double probes = pl.nrows * ((pl.Q & 1) ? 0.75 : 0.5) * pl.T;
+    const uint64_t fixed = cta_fixed(pl.m, row_slots, pl.Q, probes);
+    d.match_cap = cta_match_cap(probes);
+    d.cta_pair = cta_pair(pl.m, fixed, row_slots, probes) ? 1u : 0u;
     const uint64_t smem_max = d.cta_pair ? kCtaPairSmem : kCtaSmemMax;
     d.ctab_smem = fixed + 4ull * row_slots + 6ull * pl.m <= smem_max ? 1u : 0u;
     const uint64_t used = fixed + (d.ctab_smem ? 4ull * row_slots : 0);
@@ -1315,8 +1323,24 @@ static int ensure_gbits(rs_job *j, uint64_t words) {
   return RS_OK;
 }
 
+// Room for tag matches per prime of a chunk: a suspect has one for every 65536
+// baby steps, and match_cap is twice a prime's suspects.  (With eight a prime for
+// every job, 4000 k at m = 16384 sent all primes to the exact path.)
+static uint32_t cand_room(uint32_t match_cap, uint32_t m) {
+  const uint32_t room = (uint32_t)(1.25 * match_cap * m / 65536.0);
+  return match_cap > (uint32_t)kCtaMatchCap ? std::max(kCandPerPrime, room) : kCandPerPrime;
+}
+static uint32_t cand_per_prime(const rs_job *j) {
+  uint32_t n = 0;
+  for (auto &pt : j->parts)
+    if (pt->dev.cta_warps > 1) {
+      n = std::max(n, cand_room(pt->dev.match_cap, pt->dev.m));
+    }
+  return n;
+}
+
 static size_t chunk_bytes_per_prime(const rs_job *j) {
-  return 8 + 4 + 8 * (size_t)j->max_rec_elems() + (j->has_cta() ? kCandPerPrime * sizeof(Candidate) : 0);
+  return 8 + 4 + 8 * (size_t)j->max_rec_elems() + cand_per_prime(j) * sizeof(Candidate);
 }
 
 static uint64_t exact_scratch_bytes(const rs_job *j) {
@@ -1328,7 +1352,7 @@ static uint64_t exact_scratch_bytes(const rs_job *j) {
 static int ensure_chunk_buffers(rs_job *j, uint32_t cap) {
   const uint32_t rec = j->max_rec_elems();
   const uint64_t xs = exact_scratch_bytes(j);
-  const uint32_t ncand = j->has_cta() ? (uint32_t)std::min<uint64_t>((uint64_t)cap * kCandPerPrime, 1u << 30) : 0;
+  const uint32_t ncand = (uint32_t)std::min<uint64_t>((uint64_t)cap * cand_per_prime(j), 1u << 30);
   if (j->d_chunk && j->chunk_cap >= cap && j->chunk_rec_elems >= rec && j->chunk_exact_bytes >= xs && j->cb.cand_cap >= ncand)
     return RS_OK;
   if (j->d_chunk) cudaFreeAsync(j->d_chunk, j->st);
@@ -2701,8 +2725,7 @@ int rs::job_footprint(const char *text, size_t len, const rs_options &opt, JobFo
   std::vector<Seqs> groups = split_parts(std::move(all));
   *fp = JobFootprint{};
   fp->parts = (uint32_t)groups.size();
-  uint32_t rec = 0;
-  bool cta = false;
+  uint32_t rec = 0, cand = 0;
   for (Seqs &g : groups) {
     normalise(g);
     Plan pl;
@@ -2710,9 +2733,10 @@ int rs::job_footprint(const char *text, size_t len, const rs_options &opt, JobFo
     if (rc) return rc;
     fp->arrays += part_array_bytes(pl, g, opt.datless != 0);
     rec = std::max(rec, record_el_tab(pl, plan_row_form(pl, g, nullptr), g.k.size()) + 64);
-    cta = cta || pl.cta;
+    if (pl.cta)
+      cand = std::max(cand, cand_room(cta_match_cap(pl.nrows * ((pl.Q & 1) ? 0.75 : 0.5) * pl.T), pl.m));
   }
-  fp->per_prime = 8 + 4 + 8 * (uint64_t)rec + (cta ? kCandPerPrime * sizeof(Candidate) : 0);
+  fp->per_prime = 8 + 4 + 8 * (uint64_t)rec + cand * sizeof(Candidate);
   return RS_OK;
 }
 

@@ -11,7 +11,9 @@
 namespace rs {
 
 constexpr int kBucket = 8;          // 16-bit table slots in the planner's unit of table size
-constexpr int kMatchCap = 64;       // warp kernel: a prime with more suspects takes the exact path
+// Warp kernel: a prime with more suspects takes the exact path (at 64, 5000 k over 2e4
+// exponents sent a fifth of the primes there: 612 ns per prime, now 355).
+constexpr int kMatchCap = 256;
 // BSGS exact path (rare primes): 32-bit entries (tag << jbits) | j, linear probing.
 // j <= m-1 <= 2^jbits - 2, so a real entry is never all ones.
 constexpr uint32_t kEmpty = 0xffffffffu;
@@ -73,7 +75,7 @@ constexpr uint32_t kResMax = 8;    // residues (Q) of a by_res job at most
 constexpr uint32_t kMaskRows = 64;  // rows a row_mask record can describe
 constexpr int kCtaWarps = 16;      // warps sharing one prime in the CTA-per-prime kernel
 constexpr uint32_t kCtaSmemMax = 232448;  // shared memory a CTA may opt into (227 KB)
-constexpr int kCtaMatchCap = 64;   // suspects per prime there; a prime with more takes the exact path
+constexpr int kCtaMatchCap = 64;   // suspects per prime there, at least (JobDev::match_cap)
 
 // Per-k data of the setup kernel's row loop, 32 bytes: odd part of k, its 2-adic
 // valuation, the offset of its character table (kNoTable if none), k, its first
@@ -137,6 +139,7 @@ struct JobDev {
   uint32_t warp_smem;    // shared-memory bytes per warp (bsgs_kernel) or per CTA (bsgs_cta_kernel)
   uint32_t exact_log2;   // slots of the exact kernel's table = 1 << exact_log2
   uint32_t exact_global; // that table exceeds shared memory: it lives in ChunkBufs::exact_tab
+  uint32_t match_cap;    // CTA kernel: suspects a prime may have; one with more takes the exact path
   uint32_t cta_pair;     // CTA kernel: shared memory for two CTAs per SM
   uint32_t ctab_smem;    // CTA kernel: the k of the active rows are kept in shared memory beside their ids
   // device arrays
@@ -172,7 +175,7 @@ struct Candidate {
   uint64_t y;
   uint32_t i, row, s, thread;
 };
-constexpr uint32_t kCandPerPrime = 8;  // room per prime of a chunk (about 3 are used on the wide job)
+constexpr uint32_t kCandPerPrime = 8;  // room per prime of a chunk, at least (about 3 are used with 1000 k)
 
 // Buffers of one chunk of primes.
 struct ChunkBufs {

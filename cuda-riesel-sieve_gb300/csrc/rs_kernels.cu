@@ -1502,7 +1502,7 @@ int bsgs_smem_bytes(const JobDev &job) {
 // multiplied by the lane's Z*b^r for one or two steps u (G0, G1).  Suspects are
 // listed as they are found.
 template <bool KS, bool TWO>
-__device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint32_t *keys, uint32_t *count,
+__device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint32_t *keys, uint32_t *count, uint32_t cap,
                                            const uint32_t *ks, const uint16_t *rid, const uint32_t *__restrict__ row_k,
                                            uint32_t n, uint32_t warp, const GiantMul &G0, const GiantMul &G1,
                                            uint32_t s0) {
@@ -1535,7 +1535,7 @@ __device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint
         // (edge: a baby step may be stored under the next key)
         const uint32_t idx = atomicAdd(count, edge ? 2u : 1u);
         for (uint32_t e = 0; e <= (uint32_t)edge; e++)
-          if (idx + e < (uint32_t)kCtaMatchCap) {
+          if (idx + e < cap) {
             list[idx + e] = Match{y, rid[sl], s0 + (i & 4 ? 32 : 0)};
             keys[idx + e] = f + e;
           }
@@ -1553,7 +1553,7 @@ __device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint
 // that every row is the integer k.  Shared memory:
 //   [filter, fwords x 4 B][tags, 32W x chain_len x 4 B][k of the active rows,
 //   row_slots x 4 B (when it fits: KS)][their row ids, row_slots x 2 B]
-//   [kCtaMatchCap suspects][their keys][rows per residue, Q x 4 B][count, 16 B]
+//   [match_cap suspects][their keys][rows per residue, Q x 4 B][count, 16 B]
 // What bounds it is the integer pipes, as the warp kernel, at four warps a
 // scheduler.  On the wide job (1000 k, T = 64) it takes 103 ns per prime against 156
 // with buckets of eight 16-bit tags, counts and signatures: giant steps 49 (one
@@ -1573,8 +1573,8 @@ __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J
   uint32_t *ks = tags + T * CL;
   uint16_t *rid = reinterpret_cast<uint16_t *>(ks + (KS ? J.row_slots : 0));
   Match *list = reinterpret_cast<Match *>(rid + J.row_slots);
-  uint32_t *keys = reinterpret_cast<uint32_t *>(list + kCtaMatchCap);
-  uint32_t *nrow = keys + kCtaMatchCap;
+  uint32_t *keys = reinterpret_cast<uint32_t *>(list + J.match_cap);
+  uint32_t *nrow = keys + J.match_cap;
   uint32_t *count = nrow + J.Q;
   Filter<3> F;
   F.w = fwords;
@@ -1675,10 +1675,10 @@ __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J
             if (u + 1 < spl) {
               E = shoup_mul(E, Gw, Gq, p);
               G1.set(E, p, pinv);
-              cta_giants<KS, true>(F, list, keys, count, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
+              cta_giants<KS, true>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
               if (u + 2 < spl) E = shoup_mul(E, Gw, Gq, p);
             } else {
-              cta_giants<KS, false>(F, list, keys, count, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
+              cta_giants<KS, false>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
             }
           }
         }
@@ -1692,7 +1692,7 @@ __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J
     // a prime on the wide job, nearly all false) go to settle_kernel: a thread that
     // walked its chains here kept the whole CTA waiting, 17 of 117 ns per prime.
     const uint32_t mc = *count;
-    if (mc > (uint32_t)kCtaMatchCap) {
+    if (mc > J.match_cap) {
       if (tid == 0) {
         const uint32_t r = atomicAdd(cb.redo_count, 1u);
         if (r < cb.cap) cb.redo[r] = i;
