@@ -1,0 +1,31 @@
+"""The warp kernel's giant steps at the edges of a block of 64 passes, against
+the oracle.  With an odd Q every row is active for the primes with (b/p) = -1,
+so a job of n sequences at Q = 1 makes exactly n passes a step."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _set(f):
+    return [(int(x["p"]), int(x["k"]), int(x["n"])) for x in f]
+
+
+def _check(rs, oracle_mod, base, sign, ks, nmin, width, p0, p1, **opts):
+    """The factors of a datless job on [p0, p1], equal to the oracle's; the job's plan and counters."""
+    nl = [np.array([nmin, nmin + width - 1], dtype=np.uint32) for _ in ks]
+    with rs.Job(base=base, sign=sign, ks=ks, nlists=nl, datless=1, **opts) as job:
+        got, st = job.sieve(p0, p1)
+        info = dict(job.info)
+    want, npr = oracle_mod.Job.from_arrays(base, sign, ks, nl).sieve(p0, p1, datless=True)
+    assert st["primes"] == npr
+    assert _set(got) == _set(want)
+    return info, st, len(want)
+
+
+@pytest.mark.parametrize("passes", [63, 64, 65, 66, 67, 68, 128, 129])
+def test_pass_block_edges(rs, oracle_mod, passes):
+    ks = [3 + 2 * i for i in range(passes)]
+    info, st, n = _check(rs, oracle_mod, 7, -1, ks, 1000, 20000, 10**6, 10**6 + 20000, Q=1, hash_m=8)
+    assert (info["rows"], info["warps_per_prime"]) == (passes, 1) and info["giant_steps"] >= 32
+    assert n > 100
