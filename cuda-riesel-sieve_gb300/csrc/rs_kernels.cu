@@ -1555,7 +1555,7 @@ __device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint
 // that every row is the integer k.  Shared memory:
 //   [filter, fwords x 4 B][tags, 32W x chain_len x 4 B][k of the active rows,
 //   row_slots x 4 B (when it fits: KS)][their row ids, row_slots x 2 B]
-//   [match_cap suspects][their keys][rows per residue, Q x 4 B][count, 16 B]
+//   [match_cap suspects][their keys][rows per residue, Q x 4 B][count, redo flag, 16 B]
 // What bounds it is the integer pipes, as the warp kernel, at four warps a
 // scheduler.  On the wide job (1000 k, T = 64) it takes 103 ns per prime against 156
 // with buckets of eight 16-bit tags, counts and signatures: giant steps 49 (one
@@ -1624,7 +1624,7 @@ __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J
     const uint4 z4 = make_uint4(0, 0, 0, 0);
 #pragma unroll 4
     for (uint32_t q = tid; q < J.fwords / 4; q += T) smem4[q] = z4;
-    for (uint32_t q = tid; q <= J.Q; q += T) nrow[q] = 0;  // and count
+    for (uint32_t q = tid; q < J.Q + 2; q += T) nrow[q] = 0;  // and count and the redo flag
     __syncthreads();
     // the active rows into their residues' lists (in any order): x the k, y the residue's first slot and r
     auto place = [&](bool on, uint32_t id, uint2 kr) {
@@ -1724,7 +1724,7 @@ __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J
         const uint32_t idx = atomicAdd(cb.redo_count + 1, 1u);
         if (idx < cb.cand_cap) {
           cb.cand[idx] = Candidate{mt.y, i, mt.row, mt.s, tid};
-        } else {  // no room: the exact path takes the prime
+        } else if (atomicExch(count + 1, 1u) == 0) {  // no room: the exact path takes the prime, once
           const uint32_t r = atomicAdd(cb.redo_count, 1u);
           if (r < cb.cap) cb.redo[r] = i;
         }
