@@ -193,7 +193,7 @@ struct ChunkBufs {
   // same with step_shift = 32) or kStepShoup (Shoup's product by a full-size constant).
   uint32_t small_step;
   uint32_t step_shift;
-  uint32_t pair_ok;     // mul_small by the base is valid for every prime of the chunk
+  uint32_t pair_ok;     // mul_small by the base is valid for every prime of the chunk (and small_step is not kStepShoup)
 };
 
 struct HitBufs {
@@ -204,7 +204,9 @@ struct HitBufs {
   uint32_t cap;
   unsigned long long *stat;  // [kStatCount] counters of one rs_sieve_range call, zeroed at its start
 };
-constexpr int kStatPaired = 0;  // primes whose giant loop took the (k, 0), (k, 1) row-pair path
+// Primes whose active rows come in (k, 0), (k, 1) pairs, in launches where the
+// product of a pair is valid (ChunkBufs::pair_ok).  V rows use that product.
+constexpr int kStatPaired = 0;
 constexpr int kStatExact = 1;   // primes finished by the exact kernel
 constexpr int kStatCount = 2;
 

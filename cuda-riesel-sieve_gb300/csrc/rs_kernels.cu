@@ -1076,8 +1076,8 @@ __device__ __forceinline__ void giant_test(const Filter<2> &F, const void *src, 
 // resolution of the suspects.  cur is the prime's staged record (header, and V
 // or the row mask; nact != 0), Bl and Glm the lane's two table entries, c_lo /
 // c_hi (row_mask) the lane's row constants, tags the lane's column of the tag
-// list; npaired counts the primes that took the row-pair path.  Shared by the
-// single-job kernel and the multi-job kernel below.
+// list; npaired counts the primes whose rows come in pairs (kStatPaired).  Shared
+// by the single-job kernel and the multi-job kernel below.
 template <int TL, int RM>
 __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb, const HitBufs &hb, uint32_t *fwords,
                                            uint32_t nw, uint32_t *tags, uint32_t *vbuf,
@@ -1172,10 +1172,11 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
                                         : RM == kRowsIntId ? (const void *)(cur + J.el_row) : (const void *)(cur + kElV);
   const void *src_g = cb.recs + (size_t)i * J.rec_elems + (RM == kRowsIntId ? J.el_row : kElV);
   const bool staged = RM == kRowsRes || RM == kRowsMask || J.stage_full;
-  // (k, 0), (k, 1) row pairs; V rows form the second value by the short product
-  // by b (p > 2^33, b*p < 2^63: mul_small)
-  const bool paired = RPI == 1 && cb.pair_ok && (cur[kElNact] >> 32);
-  npaired += paired && staged && spl == 1;
+  // (k, 0), (k, 1) row pairs.  V rows form the second value by the short product
+  // by b (p > 2^33, b*p < 2^63: mul_small); integer rows, whose key costs less than
+  // that, take each row by itself and are counted only.
+  const bool paired = RPI == 1 && cb.pair_ok && staged && (cur[kElNact] >> 32);
+  npaired += paired;
   // A lane's further steps (T > 32): advance the multiplier once and go through
   // the rows again; in blocks of at most 64 tests a lane, after which the block's
   // suspects are settled.
@@ -1191,7 +1192,7 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
     uint32_t hA = 0, hB = 0;
     // Separate calls for staged and global V keep each load's address
     // space known to the compiler.
-    if (RM == kRowsV && paired && staged)
+    if (RM == kRowsV && paired)
       giant_test<RPI, GM, RPI == 1>(F, src_s, J.row_c, at, g1, n, lane_row, G, np, pinv, hA, hB, J.base,
                                     (uint32_t)cur[kElRcp]);
     else if (staged)
@@ -1320,7 +1321,7 @@ bsgs_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
   const uint64_t *ltab = cb.recs + J.el_tab + lane;  // this lane's B^lane; G^(lane+1) 32 further
 
   uint64_t nBl = 0, nGl = 0;
-  uint32_t npaired = 0;  // primes of this warp that took the row-pair path
+  uint32_t npaired = 0;  // primes of this warp whose rows come in pairs
   uint32_t c_lo = 0, c_hi = 0;  // row_mask: k*b^r of rows lane and lane + 32
   if constexpr (RM == kRowsMask) {
     c_lo = lane < J.nrows ? __ldg(J.row_c + lane) : 0u;

@@ -141,8 +141,11 @@ typedef struct {
   uint64_t d2h_bytes;    /* device->host bytes the call copied */
   uint64_t primes_by_step[3]; /* primes whose baby steps used RS_BABY_SHOUP, _SHORT, _HIGH
                             (index = form - 1) */
-  uint64_t paired_primes; /* primes whose active rows came in (k, 0), (k, 1) pairs (start values
-                            that are residues form the second value by the short product by b) */
+  uint64_t paired_primes; /* primes whose active rows came in (k, 0), (k, 1) pairs: Q = 2, every k with
+                            both residues, (b/p) = 1, a warp per prime with 32 giant steps or more,
+                            baby steps by RS_BABY_SHORT, p > 2^33 and b*p < 2^63.  A fact about the rows: row_form 0
+                            with fewer than four k forms the second value of a pair by the short
+                            product by b, the other forms take each row by itself */
   uint64_t exact_primes; /* primes finished by the exact (tag, j) table path */
 } rs_stats;
 

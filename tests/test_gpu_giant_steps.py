@@ -1,6 +1,10 @@
-"""The warp kernel's giant steps at the edges of a block of 64 passes, against
-the oracle.  With an odd Q every row is active for the primes with (b/p) = -1,
-so a job of n sequences at Q = 1 makes exactly n passes a step."""
+"""The warp kernel's giant steps against the oracle: at the edges of a block of
+64 passes, and on the row-pair product.
+
+With an odd Q every row is active for the primes with (b/p) = -1, so a job of n
+sequences at Q = 1 makes exactly n passes a step.  Rows that are residues (some
+k*b >= 2^32, fewer than four k) at Q = 2 come in pairs (k, 0), (k, 1) for the
+primes with (b/p) = 1, and the second value of a pair is a product by b."""
 import numpy as np
 import pytest
 
@@ -29,3 +33,12 @@ def test_pass_block_edges(rs, oracle_mod, passes):
     info, st, n = _check(rs, oracle_mod, 7, -1, ks, 1000, 20000, 10**6, 10**6 + 20000, Q=1, hash_m=8)
     assert (info["rows"], info["warps_per_prime"]) == (passes, 1) and info["giant_steps"] >= 32
     assert n > 100
+
+
+@pytest.mark.parametrize("nk,width,T", [(3, 20000, 32), (2, 200000, 128), (1, 70000, 128)])
+def test_row_pair_product(rs, oracle_mod, nk, width, T):
+    p0 = 2**33 + 1
+    info, st, n = _check(rs, oracle_mod, 745, -1, [9000001 + 2 * i for i in range(nk)], 1000, width, p0, p0 + 3 * 10**7, Q=2)
+    assert (info["row_form"], info["warps_per_prime"], info["giant_steps"]) == (0, 1, T)
+    assert n >= 3
+    assert st["primes"] // 8 < st["paired_primes"] < st["primes"]
