@@ -764,6 +764,7 @@ struct rs_job {
   size_t h_counts_cap = 0;
   uint32_t chunk_cap = 0;        // primes the chunk buffers hold
   uint32_t launch_cap = 0;       // primes per launch at most (rs_job_info.primes_per_launch)
+  uint32_t split_calls = 0;      // calls run in more launches than larger buffers would take (call_cap)
   uint32_t chunk_rec_elems = 0;  // record elements the chunk buffers were sized for
   uint64_t chunk_exact_bytes = 0;  // exact-kernel scratch they hold
   bool has_cta() const {
@@ -1447,16 +1448,29 @@ static void set_chunk_cap(rs_job *j) {
   j->launch_cap = (uint32_t)cap;
 }
 
-// Primes per launch for one call's range: a window that fits one launch of 2^21
-// primes gets buffers for itself, one of up to four launches a quarter each.
-// Mapping and unmapping the 3 GB of full-size buffers took 7 of the 25 ms of a
-// one-shot run over 2e8 at 1e13 and 2 of the 2.9 ms of a job's first narrow call.
+// Primes the chunk buffers should hold for one call's range.  A job's first call:
+// a window that fits one launch of 2^21 primes gets buffers for itself, one of up
+// to four launches a quarter each.  Mapping and unmapping the 3 GB of full-size
+// buffers took 7 of the 25 ms of a one-shot run over 2e8 at 1e13 and 2 of the 2.9
+// ms of a job's first narrow call.  Later calls: buffers that are too small grow
+// by half at least, so that a job whose windows grow maps them a few times, and a
+// job that goes on to split its windows gets buffers for a whole one, at the
+// eighth such call: a window of 1e8 at 1e13 takes 8.95 ms in three launches and
+// 8.72 in one, whose buffers cost 2.3 ms more to map.
 // (-b/-t fix the launch size, so they keep it.)
-static uint32_t call_cap(const rs_job *j, uint64_t lo, uint64_t hi) {
+static uint32_t call_cap(rs_job *j, uint64_t lo, uint64_t hi) {
+  constexpr uint32_t kSplitCalls = 8;
   if (j->opt.block_scale > 0 || j->opt.thread_scale > 0) return j->launch_cap;
-  const double need = 1.35 * primes_estimate(lo, hi) + 4096.0, one = 1 << 21;
-  const double cap = need <= one ? need : std::max(one, need / 4);
-  return cap < (double)j->launch_cap ? (uint32_t)cap : j->launch_cap;
+  const uint64_t need = (uint64_t)(1.35 * primes_estimate(lo, hi)) + 4096, one = 1 << 21;
+  const uint64_t have = j->d_chunk ? std::min(j->chunk_cap, j->launch_cap) : 0;
+  uint64_t cap = need <= one ? need : std::max(one, need / 4);
+  if (have && cap > have) {
+    cap = std::max(cap, have + have / 2);
+  } else if (have && need > have && have < j->launch_cap && ++j->split_calls >= kSplitCalls) {
+    j->split_calls = 0;
+    cap = need;
+  }
+  return (uint32_t)std::min<uint64_t>(cap, j->launch_cap);
 }
 // Buffers for the range; what an earlier call left may be larger.
 static int ensure_call_buffers(rs_job *j, uint64_t lo, uint64_t hi) {
