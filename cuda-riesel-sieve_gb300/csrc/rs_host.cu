@@ -767,11 +767,6 @@ struct rs_job {
   uint32_t split_calls = 0;      // calls run in more launches than larger buffers would take (call_cap)
   uint32_t chunk_rec_elems = 0;  // record elements the chunk buffers were sized for
   uint64_t chunk_exact_bytes = 0;  // exact-kernel scratch they hold
-  bool has_cta() const {
-    for (auto &pt : parts)
-      if (pt->dev.cta_warps > 1) return true;
-    return false;
-  }
   uint32_t max_rec_elems() const {
     uint32_t r = 0;
     for (auto &pt : parts) r = std::max(r, pt->dev.rec_elems);
@@ -1180,6 +1175,7 @@ static int upload_part(rs_job *j, Part &pt) {
     d.match_cap = cta_match_cap(probes);
     d.cta_pair = cta_pair(pl.m, fixed, row_slots, probes) ? 1u : 0u;
     const uint64_t smem_max = d.cta_pair ? kCtaPairSmem : kCtaSmemMax;
+    // (always with cta_pair, which asks for 8 bytes of filter a baby step beside them)
     d.ctab_smem = fixed + 4ull * row_slots + 6ull * pl.m <= smem_max ? 1u : 0u;
     const uint64_t used = fixed + (d.ctab_smem ? 4ull * row_slots : 0);
     const uint64_t left = used < smem_max ? (smem_max - used) / 16 * 4 : 0;

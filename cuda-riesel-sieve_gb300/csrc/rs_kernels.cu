@@ -1905,7 +1905,7 @@ static cudaError_t configure_one(const void *fn, int smem, int threads, int devi
 static int bsgs_threads(const JobDev &job) { return job.cta_warps > 1 ? 32 * kCtaWarps : 32 * kWarpsPerBlock; }
 
 static BsgsFn bsgs_cta_fn(const JobDev &job) {
-  if (job.cta_pair) return job.ctab_smem ? bsgs_cta_kernel<true, 2> : bsgs_cta_kernel<false, 2>;
+  if (job.cta_pair) return bsgs_cta_kernel<true, 2>;  // (cta_pair leaves room for the rows' k)
   return job.ctab_smem ? bsgs_cta_kernel<true, 1> : bsgs_cta_kernel<false, 1>;
 }
 
