@@ -1150,6 +1150,11 @@ static int upload_part(rs_job *j, Part &pt) {
   d.int_rows = pl.cta || d.by_res || form != kRowsV ? 1u : 0u;
   d.row_ids_only = pl.cta || d.by_res || form == kRowsIntId ? 1u : 0u;  // no V in the record
   d.row_mask = !pl.cta && form == kRowsMask ? 1u : 0u;      // neither V nor row ids: an active-row mask
+  // V rows of the warp layout: up to 6 rows over four or more steps a lane, or 12
+  // over 8, go through their steps one by one.  Of the time with a multiplier per
+  // step that is 0.68 for 4 rows at T = 1024, 0.93 for 6 rows at T = 128 and 0.79 at T =
+  // 512, 0.91 for 12 rows there; 9 rows at T = 128 took 1.09, 18 rows at T = 256 1.09.
+  d.few_rows = !pl.cta && !d.int_rows && (pl.T >= 256 ? pl.nrows <= 12 : pl.T >= 128 && pl.nrows <= 6) ? 1u : 0u;
   d.el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : d.by_res ? kElV + 2 : kElV;
   if (d.row_mask) {
     d.el_row = d.el_v;
@@ -2122,10 +2127,7 @@ static uint32_t batch_item_words(uint32_t warp_bytes, uint32_t stage_max, uint32
 }
 
 // Kernel variant of a warp-per-prime part: items of one multi-job launch share it.
-static uint32_t batch_variant(const JobDev &d) {
-  const uint32_t rm = d.by_res ? kRowsRes : d.row_mask ? kRowsMask : d.row_ids_only ? kRowsIntId : d.int_rows ? kRowsIntV : kRowsV;
-  return d.tlanes * 8 + rm;
-}
+static uint32_t batch_variant(const JobDev &d) { return d.tlanes * 8 + (uint32_t)row_mode(d); }
 
 extern "C" int rs_batch_run(rs_batch *B, rs_stats *stats) {
   if (!B) return fail(RS_ERR_INVALID, "rs_batch_run: NULL batch");

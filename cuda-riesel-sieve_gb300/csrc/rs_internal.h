@@ -69,8 +69,8 @@ constexpr uint32_t kElV = 12;      // V in the warp-per-prime layout (W == 1)
 constexpr uint32_t kStepShoup = 0, kStepSmall = 1, kStepHigh = 2;  // ChunkBufs::small_step
 // Giant-step start values of the fast kernels (template argument): V in
 // Montgomery form, the integers k*b^r in V, k*b^r read by row id, k*b^r of the
-// rows of an active-row mask, or the integers k by residue.
-constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3, kRowsRes = 4;
+// rows of an active-row mask, the integers k by residue, or V of few rows (JobDev::few_rows).
+constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3, kRowsRes = 4, kRowsFew = 5;
 constexpr uint32_t kResMax = 8;    // residues (Q) of a by_res job at most
 constexpr uint32_t kMaskRows = 64;  // rows a row_mask record can describe
 constexpr int kCtaWarps = 16;      // warps sharing one prime in the CTA-per-prime kernel
@@ -115,6 +115,7 @@ struct JobDev {
   uint32_t row_ids_only; // integer rows whose records keep no V: the kernels read k*b^r by row id
   uint32_t row_mask;     // integer rows whose records keep only a mask of the active rows (see above)
   uint32_t by_res;       // warp layout, k*b^r too large for integer rows: the rows are the integers k, one list per residue
+  uint32_t few_rows;     // V rows, so few for their steps that the kernel advances their values and not a multiplier
   uint32_t T;            // giant steps per row
   uint32_t tlanes;       // min(T, 32): lanes sharing one row
   uint32_t rows_per_it;  // 32 / tlanes
@@ -162,6 +163,16 @@ struct JobDev {
   uint64_t b_rcp;
   uint32_t b_jac;
 };
+
+// Kernel variant of a job's warp layout.
+inline int row_mode(const JobDev &d) {
+  return d.by_res         ? kRowsRes
+         : d.row_mask     ? kRowsMask
+         : d.row_ids_only ? kRowsIntId
+         : d.int_rows     ? kRowsIntV
+         : d.few_rows     ? kRowsFew
+                          : kRowsV;
+}
 
 struct Hit {
   uint64_t p;

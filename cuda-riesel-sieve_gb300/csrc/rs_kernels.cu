@@ -1154,7 +1154,9 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
 
   // Giant steps: lane (lane_row, lane_t) takes row slots g*RPI + lane_row for
   // two consecutive passes g at a time, giant indices s = lane_t + 1 + 32u.
-  constexpr int GM = RM == kRowsRes ? kRowsMask : RM;  // the lists hold integers, as a mask's
+  // the form of the start values: by residue the lists hold integers, as a mask's
+  constexpr int GM = RM == kRowsRes ? kRowsMask : RM == kRowsFew ? kRowsV : RM;
+  constexpr bool V = GM == kRowsV;
   uint32_t n = nact;  // the rows gone through: all active ones, or those of residue r
   uint32_t r = 0, base = 0;
   uint64_t E = Glm;  // the lane's multiplier as stored, advanced by G^32 per step u
@@ -1174,22 +1176,59 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
   const bool staged = RM == kRowsRes || RM == kRowsMask || J.stage_full;
   // (k, 0), (k, 1) row pairs.  V rows form the second value by the short product
   // by b (p > 2^33, b*p < 2^63: mul_small); integer rows, whose key costs less than
-  // that, take each row by itself and are counted only.
+  // that, and few V rows of many steps take each row by itself and are counted only.
   const bool paired = RPI == 1 && cb.pair_ok && staged && (cur[kElNact] >> 32);
   npaired += paired;
   // A lane's further steps (T > 32): advance the multiplier once and go through
   // the rows again; in blocks of at most 64 tests a lane, after which the block's
-  // suspects are settled.
+  // suspects are settled.  Few V rows (kRowsFew): advance two rows' values by G^32, in
+  // unreduced form, through their steps.  A multiplier costs a product and its w,
+  // as much as a row, which pays with more rows, four to a loop.
   GiantMul G;
   G.set(E, p, pinv);
   auto start = [&](uint32_t sl) {
     return staged ? giant_start<GM>(src_s, J.row_c, sl) : giant_start<GM>(src_g, J.row_c, sl);
   };
   uint32_t u = 0, at = 0, suspects = 0;  // step, the block's first pass, suspects so far
+  const uint32_t per = min(spl, 32u);    // kRowsFew: steps of a row in a block (both powers of two)
+  uint64_t ya = 0, yb = 0;               // ... the two rows' values
 #pragma unroll 1
   while (true) {
-    const uint32_t g1 = min(ngi, at + 64);
+    const uint32_t g1 = min(ngi, at + 64), u0 = u, at0 = at;
     uint32_t hA = 0, hB = 0;
+    if constexpr (RM == kRowsFew) {
+      const LazyShoup by_g{cur[kElGw], cur[kElGq], np};
+      uint32_t sh = 0;
+#pragma unroll 1
+      do {
+        if (u == 0) {
+          const LazyShoup first{G.w(), G.wq, np};
+          ya = first(start(at));
+          if (at + 1 < n) yb = first(start(at + 1));
+        } else {
+          ya = by_g(ya);
+          yb = by_g(yb);
+        }
+        auto steps = [&](auto both) {
+          constexpr bool BOTH = decltype(both)::value;
+#pragma unroll 1
+          for (const uint32_t end = sh + per;;) {
+            if (F.test((uint32_t)(frac64(ya, pinv) >> 32))) hA |= 1u << sh;
+            if (BOTH && F.test((uint32_t)(frac64(yb, pinv) >> 32))) hB |= 1u << sh;
+            if (++sh == end) break;
+            ya = by_g(ya);
+            if (BOTH) yb = by_g(yb);
+          }
+        };
+        if (at + 1 < n) steps(std::true_type{});
+        else steps(std::false_type{});
+        u += per;
+        if (u == spl) {
+          u = 0;
+          at += 2;
+        }
+      } while (sh < 32 && at < n);
+    } else
     // Separate calls for staged and global V keep each load's address
     // space known to the compiler.
     if (RM == kRowsV && paired)
@@ -1207,7 +1246,19 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
 #pragma unroll 1
     while (uint32_t any = __ballot_sync(0xffffffffu, bits != 0)) {
       const uint32_t bit = bits ? __ffsll((long long)bits) - 1 : 0;
-      const uint32_t sl = (at + 2 * (bit & 31) + (bit >> 5)) * RPI + lane_row;
+      uint32_t sl = (at + 2 * (bit & 31) + (bit >> 5)) * RPI + lane_row, su = 0;
+      GiantMul M = G;
+      if constexpr (RM == kRowsFew) {  // the multiplier of step su, by powers of G^32
+        sl = at0 + 2 * ((bit & 31) / per) + (bit >> 5);
+        su = u0 + (bit & 31) % per;
+        uint64_t e = Glm, q = cur[kElGs];
+#pragma unroll 1
+        for (uint32_t x = su; x; x >>= 1) {
+          if (x & 1) e = montmul(e, q, p, pinv);
+          q = montmul(q, q, p, pinv);
+        }
+        M.set(e, p, pinv);
+      }
       const bool mine = bits != 0 && sl < n;
       bits &= bits - 1;
       any = __ballot_sync(0xffffffffu, mine);
@@ -1224,8 +1275,8 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
       bool edge = false;
       if (mine) {
         const uint64_t v = start(sl);
-        y = giant_exact<GM>(v, G);
-        edge = exact_key<GM>(y, giant_key<GM>(v, G, RM == kRowsV ? G.w() : 0, np, pinv), p, pinv, f);
+        y = giant_exact<GM>(v, M);
+        edge = exact_key<GM>(y, giant_key<GM>(v, M, V ? M.w() : 0, np, pinv), p, pinv, f);
       }
       const uint32_t both = __ballot_sync(0xffffffffu, edge);  // these could be stored under F + 1 too
 #pragma unroll 1
@@ -1240,13 +1291,14 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
           if (!__any_sync(0xffffffffu, zero_half(z))) continue;
           const uint64_t ys = __shfl_sync(0xffffffffu, y, src);
           const uint32_t slot = __shfl_sync(0xffffffffu, sl, src);
-          uint64_t va = RM == kRowsV ? Bl : from_mont(Bl, p, pinv);
-          uint64_t vb = RM == kRowsV ? Blb : from_mont(Blb, p, pinv);
+          const uint32_t step = RM == kRowsFew ? __shfl_sync(0xffffffffu, su, src) : u;
+          uint64_t va = V ? Bl : from_mont(Bl, p, pinv);
+          uint64_t vb = V ? Blb : from_mont(Blb, p, pinv);
 #pragma unroll 1
           for (uint32_t t = 0; t < CL; t++) {
             const bool ma = va == ys && t < na, mb = vb == ys && t < nb;
             if (ma || mb) {
-              const uint32_t s = ((uint32_t)src & (TL - 1)) + 1 + 32 * u;
+              const uint32_t s = ((uint32_t)src & (TL - 1)) + 1 + 32 * step;
               uint32_t row;
               if constexpr (RM == kRowsMask) {
                 row = nth_row(cur[kElV], slot);
@@ -1264,6 +1316,10 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
           }
         }
       }
+    }
+    if constexpr (RM == kRowsFew) {
+      if (at < n) continue;
+      return;
     }
     at = g1;
     if (at < ngi) continue;
@@ -1481,12 +1537,9 @@ static BsgsFn bsgs_fn_t(uint32_t tlanes) {
   }
 }
 
-static int row_mode(const JobDev &job) {
-  return job.by_res ? kRowsRes : job.row_mask ? kRowsMask : job.row_ids_only ? kRowsIntId : job.int_rows ? kRowsIntV : kRowsV;
-}
-
 static BsgsFn bsgs_fn(const JobDev &job) {
   switch (row_mode(job)) {
+    case kRowsFew: return bsgs_kernel<32, kRowsFew>;
     case kRowsRes: return bsgs_fn_t<kRowsRes>(job.tlanes);
     case kRowsMask: return bsgs_fn_t<kRowsMask>(job.tlanes);
     case kRowsIntId: return bsgs_fn_t<kRowsIntId>(job.tlanes);
@@ -1944,6 +1997,7 @@ cudaError_t launch_bsgs(const JobDev &job, const ChunkBufs &cb, const HitBufs &h
 
 static BatchFn batch_fn(const JobDev &rep) {
   switch (row_mode(rep)) {
+    case kRowsFew: return bsgs_batch_kernel<32, kRowsFew>;
     case kRowsRes: return batch_fn_t<kRowsRes>(rep.tlanes);
     case kRowsMask: return batch_fn_t<kRowsMask>(rep.tlanes);
     case kRowsIntId: return batch_fn_t<kRowsIntId>(rep.tlanes);

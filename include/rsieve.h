@@ -143,9 +143,9 @@ typedef struct {
                             (index = form - 1) */
   uint64_t paired_primes; /* primes whose active rows came in (k, 0), (k, 1) pairs: Q = 2, every k with
                             both residues, (b/p) = 1, a warp per prime with 32 giant steps or more,
-                            baby steps by RS_BABY_SHORT, p > 2^33 and b*p < 2^63.  A fact about the rows: row_form 0
-                            with fewer than four k forms the second value of a pair by the short
-                            product by b, the other forms take each row by itself */
+                            baby steps by RS_BABY_SHORT, p > 2^33 and b*p < 2^63.  A fact about the
+                            rows: only rows held as residues, of few k and with few giant steps,
+                            have the second value of a pair formed by the short product by b */
   uint64_t exact_primes; /* primes finished by the exact (tag, j) table path */
 } rs_stats;
 
