@@ -276,10 +276,14 @@ cudaError_t launch_sieve(uint64_t lo, uint64_t hi, const uint32_t *sp, const uin
     sieve_large_kernel<<<(nl + 255) / 256, 256, 0, st>>>(lo, hi, sp, sp_rcp, nsmall, nsp, gbits, nodd);
   }
   if (!seg) {
-    // Below two blocks an SM a window's time is one block's: segments a quarter as
-    // long (a 1e5-wide window at 1e13: 61 -> 56 us for both passes).
+    // While the blocks of segments a quarter as long are two an SM at most, a
+    // window's time is one block's, and such segments are faster: both passes take 61
+    // -> 56 us at 1e13 for a window of 1e5, 80 -> 69 for one of 4e6 (61 segments), 82 ->
+    // 81 at 92 segments.  With more of them each block's walk over the small primes
+    // counts: 83 -> 92 us at 122 segments, 105 -> 155 at 290.
     constexpr int kShort = kSieveOdds / 4;
-    if (blocks < 304)
+    constexpr uint32_t kShortMax = 2 * 152 / 4;  // GB300's SMs
+    if (blocks <= kShortMax)
       sieve_small_kernel<false, kShort><<<(unsigned)((nodd + kShort - 1) / kShort), kSieveThreads, 0, st>>>(
           lo, hi, sp, sp_rcp, nsmall, gbits, out, count, cap, nullptr);
     else
