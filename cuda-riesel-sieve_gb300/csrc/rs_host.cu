@@ -382,7 +382,8 @@ static int count_rows(const Seqs &s, uint32_t Q, bool datless) {
   return rows;
 }
 
-// Whether rows that are no 32-bit integers go by residue: every residue has rows to share a multiplier.
+// Whether the planner prices rows that are no 32-bit integers by residue (row_by_res
+// decides): every residue has rows to share a multiplier.
 static bool rows_by_residue(uint32_t Q, size_t nk, size_t rows) { return Q <= kResMax && nk >= 4 && rows <= 512; }
 
 // One point of the planner's search: the parameters that define a plan, and its modelled cost.
@@ -826,9 +827,18 @@ static uint32_t plan_row_form(const Plan &pl, const Seqs &s, std::vector<uint32_
   return ids ? kRowsIntId : kRowsIntV;
 }
 
-// Rows of the warp layout handled by residue (JobDev::by_res).
+// Rows of the warp layout handled by residue (JobDev::by_res): where a residue's
+// multiplier is shared by enough active rows a row slot, or V would not be staged.
+// Time of V rows over time by residue (search and setup; b = 745, forced Q, 2e4 to 4e6
+// exponents), by `shared`: Q = 3 to 7 0.75 to 0.97 up to 2, 0.87 to 1.1 at 2.5 to 3.5,
+// 1.0 to 1.3 from 5 on; Q = 2 0.88 to 0.98 at 2, 0.96 to 1.09 at 2.5; Q = 8 0.66 to 0.92 up to
+// 4, 1.03 to 1.09 from 5 (T = 16) or 7 on.  With T below 8, where a row's V product in the setup kernel
+// weighs more, 1.05 to 1.12 at 2.25 and 0.85 to 1.0 up to 1.5.
 static bool row_by_res(const Plan &pl, uint32_t form, size_t nk) {
-  return form == kRowsV && !pl.cta && rows_by_residue(pl.Q, nk, pl.nrows);
+  if (form != kRowsV || pl.cta || !rows_by_residue(pl.Q, nk, pl.nrows)) return false;
+  const double shared = nk * ((pl.Q & 1) ? 0.75 : 0.5) * pl.tlanes / 32.0;
+  const double least = (pl.Q == 8 ? 4.2 : 2.2) * std::sqrt(std::min(1.0, pl.tlanes / 8.0));
+  return shared >= least || kElV + pl.nrows > kStageElems;
 }
 
 // First element of the lane tables in a record (el_tab; a record has el_tab + 64
@@ -1165,9 +1175,9 @@ static int upload_part(rs_job *j, Part &pt) {
   }
   d.rec_elems = d.el_tab + 64;
   // the warp kernel's staged part of a record: header + V (header + row ids
-  // without V, header + mask with row_mask) when it fits 2 KB; else the header alone
+  // without V, header + mask with row_mask) when it fits kStageElems; else the header alone
   const uint32_t staged = d.row_ids_only || d.row_mask ? d.el_tab : d.el_row;
-  if (staged * 8 <= 2048) {
+  if (staged <= kStageElems) {
     d.stage_full = 1;
     d.stage_elems = staged;
   } else {

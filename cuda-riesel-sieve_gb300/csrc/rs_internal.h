@@ -73,6 +73,7 @@ constexpr uint32_t kStepShoup = 0, kStepSmall = 1, kStepHigh = 2;  // ChunkBufs:
 constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3, kRowsRes = 4, kRowsFew = 5;
 constexpr uint32_t kResMax = 8;    // residues (Q) of a by_res job at most
 constexpr uint32_t kMaskRows = 64;  // rows a row_mask record can describe
+constexpr uint32_t kStageElems = 256;  // record elements the warp kernel stages at most (2 KB)
 constexpr int kCtaWarps = 16;      // warps sharing one prime in the CTA-per-prime kernel
 constexpr uint32_t kCtaSmemMax = 232448;  // shared memory a CTA may opt into (227 KB)
 constexpr int kCtaMatchCap = 64;   // suspects per prime there, at least (JobDev::match_cap)
