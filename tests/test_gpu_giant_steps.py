@@ -53,7 +53,7 @@ def test_row_pair_product(rs, oracle_mod, nk, width, T):
 def test_few_rows_many_steps(rs, oracle_mod, nk, Q, sign, width, hash_m, T):
     ks = [9000001 + 2 * i for i in range(nk)]
     found = 0
-    for p0, window in ((10**6, 3 * 10**4), (2**33 + 1, 2 * 10**6), (2**62 + 1, 3 * 10**4)):
+    for p0, window in ((10**6, 3 * 10**4), (2**33 + 1, 2 * 10**6), (2**47 + 1, 10**5)):
         info, st, n = _check(rs, oracle_mod, 745, sign, ks, 1000, width, p0, p0 + window, Q=Q, hash_m=hash_m)
         assert (info["row_form"], info["warps_per_prime"], info["giant_steps"]) == (0, 1, T)
         assert info["rows"] <= 12 and st["exact_primes"] <= st["primes"] // 50

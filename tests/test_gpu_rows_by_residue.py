@@ -21,7 +21,7 @@ def test_line_of_rows_by_residue(rs, oracle_mod, nk, Q, sign, width, T):
     with rs.Job(base=745, sign=sign, ks=ks, nlists=nl, datless=1, Q=Q) as job:
         info = job.info
         assert (info["row_form"], info["warps_per_prime"], info["giant_steps"]) == (0, 1, T)
-        for p0, window in ((10**6, 2 * 10**4), (2**33 + 1, 10**6), (2**61 + 1, 3 * 10**4)):
+        for p0, window in ((10**6, 2 * 10**4), (2**33 + 1, 10**6), (2**47 + 1, 10**5)):
             got, st = job.sieve(p0, p0 + window)
             want, npr = oj.sieve(p0, p0 + window, datless=True)
             key = lambda f: [(int(x["p"]), int(x["k"]), int(x["n"])) for x in f]  # noqa: E731
