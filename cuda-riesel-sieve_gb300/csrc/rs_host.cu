@@ -2656,16 +2656,27 @@ extern "C" int rs_gpu_primes(uint64_t lo, uint64_t hi, uint64_t *out, size_t cap
   // the primes as bits with their prefix sums per segment, then in order: no sort
   const uint64_t words = sieve_bitmap_words(lo, hi);
   const uint32_t segs = sieve_segments(lo, hi);
-  DeviceScratch bits(tmp.st, words * 4 + segs * 4ull + 4);
-  CUDA_TRY(bits.err);
-  uint32_t *d_bits = (uint32_t *)bits.ptr, *d_seg = d_bits + words, *d_cnt = d_seg + segs;
+  // A small window's primes come back with their number, in one copy and one wait
+  // (1e4 wide at 1e13: 0.253 ms with two, 0.239 in one); a larger one's after it.
+  const uint64_t room = odds <= 8192 ? odds : 0;
+  DeviceScratch scratch(tmp.st, room * 8 + 4 + segs * 4ull + words * 4);
+  CUDA_TRY(scratch.err);
+  uint64_t *d_small = (uint64_t *)scratch.ptr;
+  uint32_t *d_cnt = (uint32_t *)(d_small + room), *d_seg = d_cnt + 1, *d_bits = d_seg + segs;
   CUDA_TRY(launch_sieve(lo, hi, tmp.d_sp, tmp.d_sp_rcp, tmp.nsp, tmp.nsp_small, d_bits, nullptr, d_cnt, 0, tmp.st, d_seg));
-  uint32_t n = 0;
-  CUDA_TRY(cudaMemcpyAsync(&n, d_cnt, 4, cudaMemcpyDeviceToHost, tmp.st));
+  if (room) CUDA_TRY(launch_emit(lo, hi, d_bits, d_seg, (uint32_t)room, d_small, nullptr, nullptr, tmp.st));
+  std::vector<uint64_t> got(room + 1, 0);
+  CUDA_TRY(cudaMemcpyAsync(got.data(), d_small, room * 8 + 4, cudaMemcpyDeviceToHost, tmp.st));
   CUDA_TRY(cudaStreamSynchronize(tmp.st));
+  uint32_t n = 0;
+  memcpy(&n, got.data() + room, 4);
   *count = n;
   if (n > cap) return fail(RS_ERR_CAPACITY, "%u primes, buffer holds %zu", n, cap);
   if (n == 0) return RS_OK;
+  if (room) {
+    memcpy(out, got.data(), (size_t)n * 8);
+    return RS_OK;
+  }
   DeviceScratch d_out(tmp.st, (size_t)n * 8);
   CUDA_TRY(d_out.err);
   CUDA_TRY(launch_emit(lo, hi, d_bits, d_seg, n, (uint64_t *)d_out.ptr, nullptr, nullptr, tmp.st));
