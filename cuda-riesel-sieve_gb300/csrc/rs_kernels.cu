@@ -1820,12 +1820,17 @@ __global__ void __launch_bounds__(128) settle_kernel(JobDev J, ChunkBufs cb, Hit
 // prime, for the primes with too many suspects for the fast path.  WG
 // warps share a prime (1 for warp-per-prime jobs, kCtaWarps for CTA jobs) with
 // the same chain layout as the fast kernels.
+// The smallest primes come here, and among them those modulo which B has a small
+// order d: their baby steps are d values over and over.  The table holds the first
+// d, and a match stands for j, j + d, ...; all m of them made runs of m/d
+// entries in one place of the table, which each insert and probe walked.
 template <int WG>
 __global__ void __launch_bounds__(WG == 1 ? 32 * kWarpsPerBlock : 32 * WG, 1)
 bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
   extern __shared__ uint4 smem4[];
   constexpr uint32_t G = 32 * WG;                           // threads per prime
   constexpr uint32_t NG = WG == 1 ? kWarpsPerBlock : 1;     // primes per block
+  __shared__ uint32_t order;  // WG > 1
   const uint32_t grp = threadIdx.x / G, gt = threadIdx.x % G, wig = gt >> 5, lane = threadIdx.x & 31;
   const uint32_t S = 1u << J.exact_log2;
   const uint32_t tmask = S - 1;
@@ -1855,18 +1860,42 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
     if (WG == 1) __syncwarp();
     else __syncthreads();
     for (uint32_t q = gt; q < S; q += G) tab[q] = kEmpty;
+    if (WG > 1 && gt == 0) order = J.m;
     if (WG == 1) __syncwarp();
     else __syncthreads();
     // the thread's two baby chains, j = (gt + G*c)*chain_len + t
     uint64_t Bl = rec_el(J, cb, J.el_tab + lane, i);
     if (WG > 1 && wig) Bl = shoup_mul(Bl, rec_el(J, cb, kElWoff + 2 * wig, i), rec_el(J, cb, kElWoff + 2 * wig + 1, i), p);
+    const uint64_t Blb = shoup_mul(Bl, rec_el(J, cb, kElOfw, i), rec_el(J, cb, kElOfq, i), p);
+    // the first j at which the values repeat the one of j = 0, or m
+    uint32_t d = J.m;
+    {
+      const uint64_t v0 = rec_el(J, cb, J.el_tab, i);
+#pragma unroll 1
+      for (uint32_t c = 0; c < 2; c++) {
+        const uint32_t j0 = (gt + G * c) * J.chain_len;
+        uint64_t v = c ? Blb : Bl;
+#pragma unroll 1
+        for (uint32_t j = j0; j < d && j < j0 + J.chain_len; j++) {
+          if (v == v0 && j) d = j;
+          v = shoup_mul(v, Stw, Stq, p);
+        }
+      }
+      if (WG == 1) {
+        d = __reduce_min_sync(0xffffffffu, d);
+      } else {
+        if (d < J.m) atomicMin(&order, d);
+        __syncthreads();
+        d = order;
+      }
+    }
 #pragma unroll 1
     for (uint32_t c = 0; c < 2; c++) {
       const uint32_t j0 = (gt + G * c) * J.chain_len;
-      uint64_t v = c ? shoup_mul(Bl, rec_el(J, cb, kElOfw, i), rec_el(J, cb, kElOfq, i), p) : Bl;
+      uint64_t v = c ? Blb : Bl;
       if (J.int_rows) v = from_mont(v, p, pinv);  // giant values (below) come in normal form
 #pragma unroll 1
-      for (uint32_t j = j0; j < J.m && j < j0 + J.chain_len; j++) {
+      for (uint32_t j = j0; j < d && j < j0 + J.chain_len; j++) {
         uint32_t h = (uint32_t)v & tmask;
         const uint32_t e = ((((uint32_t)(v >> tl)) & tagmask) << jbits) | j;
 #pragma unroll 1
@@ -1910,7 +1939,8 @@ bsgs_exact_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
           for (uint32_t q = 0; q < S; q++) {
             const uint32_t e = tab[h];
             if (e == kEmpty) break;
-            if ((e >> jbits) == tag) record_hit(J, hb, p, row, s, e & jmask);
+            if ((e >> jbits) == tag)
+              for (uint32_t j = e & jmask; j < J.m; j += d) record_hit(J, hb, p, row, s, j);
             h = (h + 1) & tmask;
           }
           if (u + 1 < J.steps_per_lane) {
