@@ -1717,6 +1717,10 @@ static std::vector<Chunk> plan_chunks(uint64_t lo, uint64_t hi, uint32_t C) {
   std::vector<Chunk> todo;
   uint64_t a = lo;
   while (a <= hi) {
+    if (1.3 * primes_estimate(a, hi) <= (double)C) {  // (exceeds the number of primes from 3 on, too)
+      todo.push_back({a, hi});
+      break;
+    }
     const double la = std::log((double)a);
     double w = la > 3.0 ? 0.8 * (double)C * (la - 1.2) : 1.6 * (double)C;
     if (w < 64) w = 64;

@@ -36,3 +36,15 @@ def test_growing_windows(rs, oracle_mod):
     want, npr = oj.sieve(p0, p0 + 5 * 10**6 - 1, datless=True)
     assert st["primes"] == npr and _set(got) == _set(want) and len(want) > 20
     assert _set(again) == {x for x in _set(want) if x[0] < p0 + 4 * 10**5}
+
+
+@pytest.mark.parametrize("hi", [1000, 20000, 10**5, 3 * 10**6])
+def test_window_from_three_in_one_launch(rs, oracle_mod, hi):
+    """A window that its buffers hold is one launch, where primes are densest too."""
+    import rsieve.synth as S
+
+    b, s, ks, nl = S.plain_job(1)
+    with rs.Job(base=b, sign=s, ks=ks[:3], nlists=nl[:3]) as job:
+        got, st = job.sieve(3, hi)
+    want, npr = oracle_mod.Job.from_arrays(b, s, ks[:3], nl[:3]).sieve(3, hi)
+    assert st["bsgs_launches"] == 1 and st["primes"] == npr and _set(got) == _set(want)
