@@ -1206,6 +1206,12 @@ static int upload_part(rs_job *j, Part &pt) {
     for (uint32_t k : s.k) kmax = std::max<uint64_t>(kmax, k);
     d.edge_lim = (uint32_t)std::min<uint64_t>(0xffffffffu, ((kmax + 1) >> (d.fshift - 10)) + 1);
   } else {  // bytes per warp: the filter takes what the shared memory leaves (warp_filter)
+    // Suspects: twice and more the false ones that the fullest filters leave (2.5e-3 of the
+    // probes), or 64: the smallest primes match at every step, and a true suspect
+    // is a walk along the chains by one warp.  With 256 for every job, 50000 numbers at
+    // 1e6 for one k took 0.53 ms against 0.31, 3 to 1000 for 22 k 0.85 against 0.64.
+    const double probes = pl.nrows * ((pl.Q & 1) ? 0.75 : 0.5) * pl.T;
+    d.match_cap = (uint32_t)std::min<double>(kMatchCap, std::max(64.0, 6.4e-3 * probes));
     const uint32_t fixed = warp_kernel_fixed(d.chain_len, d.stage_elems, d.row_mask != 0, d.by_res != 0, d.row_slots);
     d.fwords = warp_filter(pl.m, fixed, 0, pt.ctas);
     d.warp_smem = 4 * d.fwords + fixed;

@@ -11,8 +11,9 @@
 namespace rs {
 
 constexpr int kBucket = 8;          // 16-bit table slots in the planner's unit of table size
-// Warp kernel: a prime with more suspects takes the exact path (at 64, 5000 k over 2e4
-// exponents sent a fifth of the primes there: 612 ns per prime, now 355).
+// Warp kernel: suspects a prime may have at most (JobDev::match_cap; at 64 for all jobs,
+// 5000 k over 2e4 exponents sent a fifth of the primes to the exact path: 612 ns per
+// prime, with 256 355).
 constexpr int kMatchCap = 256;
 // BSGS exact path (rare primes): 32-bit entries (tag << jbits) | j, linear probing.
 // j <= m-1 <= 2^jbits - 2, so a real entry is never all ones.
@@ -141,7 +142,7 @@ struct JobDev {
   uint32_t warp_smem;    // shared-memory bytes per warp (bsgs_kernel) or per CTA (bsgs_cta_kernel)
   uint32_t exact_log2;   // slots of the exact kernel's table = 1 << exact_log2
   uint32_t exact_global; // that table exceeds shared memory: it lives in ChunkBufs::exact_tab
-  uint32_t match_cap;    // CTA kernel: suspects a prime may have; one with more takes the exact path
+  uint32_t match_cap;    // suspects a prime may have; one with more takes the exact path
   uint32_t cta_pair;     // CTA kernel: shared memory for two CTAs per SM
   uint32_t ctab_smem;    // CTA kernel: the k of the active rows are kept in shared memory beside their ids
   // device arrays

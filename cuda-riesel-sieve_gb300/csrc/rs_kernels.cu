@@ -1267,7 +1267,7 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
       bits &= bits - 1;
       any = __ballot_sync(0xffffffffu, mine);
       suspects += __popc(any);
-      if (suspects > (uint32_t)kMatchCap) {  // the exact path takes the prime
+      if (suspects > J.match_cap) {  // the exact path takes the prime
         if (lane == 0) {
           const uint32_t r = atomicAdd(cb.redo_count, 1u);
           if (r < cb.cap) cb.redo[r] = i;

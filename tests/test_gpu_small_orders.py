@@ -43,3 +43,20 @@ def test_small_orders(rs, oracle_mod, nk, width, hash_m, m, order):
     key = lambda f: [(int(x["p"]), int(x["k"]), int(x["n"])) for x in f]  # noqa: E731
     assert st["primes"] == npr and st["exact_primes"] > 0
     assert key(got) == key(want) and p in {x[0] for x in key(want)}
+
+
+def test_smallest_primes(rs, oracle_mod):
+    """Primes with more than 64 suspects take the exact path in a job of few probes:
+    a prime below m matches at each of its some 170 giant steps."""
+    rng = np.random.default_rng(22)
+    ks = [1000003 + 2 * i for i in range(22)]
+    nl = [np.unique(np.concatenate([[10**6, 10**6 + 70000], rng.integers(10**6, 10**6 + 70001, 3)])).astype(np.uint32)
+          for _ in ks]
+    with rs.Job(base=745, sign=-1, ks=ks, nlists=nl) as job:
+        info = job.info
+        got, st = job.sieve(3, 1000)
+    assert info["warps_per_prime"] == 1 and info["baby_steps"] > 400 and 300 < info["rows"] * info["giant_steps"] < 600
+    want, npr = oracle_mod.Job.from_arrays(745, -1, ks, nl).sieve(3, 1000)
+    key = lambda f: [(int(x["p"]), int(x["k"]), int(x["n"])) for x in f]  # noqa: E731
+    assert st["primes"] == npr and key(got) == key(want) and len(want) > 50
+    assert npr // 4 < st["exact_primes"] <= npr
