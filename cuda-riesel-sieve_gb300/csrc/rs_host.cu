@@ -533,7 +533,10 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
       // (a product plus a table operation), the table clear, the per-prime
       // setup kernel (grows with the rows), the expected tag-match
       // resolution (one pass over the baby steps), and a penalty for fewer
-      // resident warps when the tables are large.
+      // resident warps when the tables are large.  Tables, their bytes and their
+      // false matches (fp) are those of the hash tables before the filter, on which
+      // the weights of more than 16 k were fitted; a plan they admit has room for
+      // its filter (at least 1.25 words a baby step in the warp layout, 1.5 in a CTA).
       {  // warp per prime: whole chains of 64 when that stays within the cap
         uint64_t m = m0;
         if (m > 64 && ((m + 63) & ~63ull) <= mcap) m = (m + 63) & ~63ull;
@@ -541,13 +544,12 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
         if (m <= mcap && m * T >= X && slog <= kMaxTableLog2) {
           const uint32_t blog = std::max<uint32_t>(4, ilog2_ceil((2 * m + kBucket - 1) / kBucket));
           const double nb = (double)(1u << blog);
-          // the kernel's shared memory per warp and per CTA (128-byte granules, 1 KB reserved)
+          // shared memory per warp and per CTA (128-byte granules, 1 KB reserved)
           const uint64_t stage = kElV + ((rows + 1) & ~1u);
           const uint64_t wsm = align_up((20u << blog) + 16 * (stage * 8 <= 2048 ? stage : kElV) + 256, 16);
           const double cta_bytes = (double)align_up(4 * wsm, 128) + 1024.0;
           const double warps = std::min(kFullWarps, 4.0 * std::floor(kSmemPerSm / cta_bytes));
           const double fp = ER * (double)T * ((double)m / nb) / 65536.0;  // expected tag matches per prime
-          // (a prime with more than kMatchCap matches takes the slow exact path)
           if (warps >= 4 && fp <= 2.0) {
             const double cost = ((few && !short_q ? kShoupStep : 1.0) * std::ceil((double)m / 32.0) +
                                  (few && !ints_q && !res_q ? kResidueRow : kGiantWeight) * std::ceil(ER / rpi) * spl +

@@ -261,9 +261,9 @@ int bsgs_exact_smem_bytes(const JobDev &job);
 uint64_t bsgs_exact_scratch_bytes(const JobDev &job, int exact_grid);
 cudaError_t bsgs_configure(const JobDev &job, int device, int *grid_out, int *exact_grid_out);
 // Multi-job launch over `nitems` items in device memory that share rep's kernel
-// variant (rep: any of them); stage_max and row_slots_max are the largest over the items, and
-// warp_bytes holds every item's warp_kernel_bytes with that stage.
-// batch_configure gives the grid.
+// variant (rep: any of them); stage_max and row_slots_max are the largest over the
+// items, and warp_bytes is a warp's shared memory (warp_kernel_share), in which
+// every item's filter fits beside that stage.  batch_configure gives the grid.
 cudaError_t batch_configure(const JobDev &rep, uint32_t warp_bytes, int device, int *grid_out);
 cudaError_t launch_bsgs_batch(const JobDev &rep, const BatchItem *items, uint32_t nitems, uint32_t stage_max,
                               uint32_t row_slots_max, uint32_t warp_bytes, int grid, cudaStream_t st);

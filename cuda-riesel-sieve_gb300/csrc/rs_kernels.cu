@@ -1089,7 +1089,6 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
                                            uint64_t Glm, uint32_t lane, uint32_t c_lo, uint32_t c_hi,
                                            uint32_t &npaired) {
   constexpr uint32_t RPI = 32 / TL;  // row slots per lane-group pass
-  const uint32_t lane_t = lane & (TL - 1);
   const uint32_t lane_row = lane / TL;
   const uint32_t spl = TL == 32 ? J.steps_per_lane : 1;
   if constexpr (RM == kRowsMask) {  // V from the active-row mask
@@ -1156,8 +1155,8 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
   else baby(LazyShort{J.bq_small, (uint32_t)(Stq >> (32 - cb.step_shift)), cb.step_shift, np});
   __syncwarp();
 
-  // Giant steps: lane (lane_row, lane_t) takes row slots g*RPI + lane_row for
-  // two consecutive passes g at a time, giant indices s = lane_t + 1 + 32u.
+  // Giant steps: a lane takes row slots g*RPI + lane_row for two consecutive
+  // passes g at a time, giant indices s = lane % TL + 1 + 32u.
   // the form of the start values: by residue the lists hold integers, as a mask's
   constexpr int GM = RM == kRowsRes ? kRowsMask : RM == kRowsFew ? kRowsV : RM;
   constexpr bool V = GM == kRowsV;
@@ -1359,11 +1358,11 @@ __device__ __forceinline__ void bsgs_prime(const JobDev &J, const ChunkBufs &cb,
 // own buffer from the constants of rows lane and lane + 32 that each lane keeps
 // in registers.
 //
-// Each lane runs two independent product chains in both phases (baby steps
-// j = lane + 64t and j = lane + 32 + 64t; giant steps on two row slots at a
-// time) so that consecutive dependent Shoup products overlap.
+// Each lane runs two independent chains in both phases (baby steps j = lane*c + t
+// and j = (lane + 32)*c + t, c the chain length; giant steps on two row slots
+// at a time), so that dependent products overlap.
 // TL = giant steps handled side by side per row (min(T, 32)); RM = the form
-// of the giant-step start values (kRowsV, kRowsIntV, kRowsIntId).
+// of the giant-step start values (kRowsV to kRowsFew).
 template <int TL, int RM>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, 4)
 bsgs_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
@@ -1641,8 +1640,7 @@ __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J
   F.sh1 = J.fshift;
   F.mul = J.fwords << J.fshift;
   const uint32_t total = *cb.count;
-  const uint32_t n = total < cb.cap ? total : cb.cap;
-  const uint32_t ja0 = tid * CL, jb0 = (tid + T) * CL;  // the thread's chains; m == 2*T*CL
+  const uint32_t n = total < cb.cap ? total : cb.cap;  // (the thread's chains begin at tid*CL and (tid + T)*CL; m == 2*T*CL)
 
   // What a prime needs first is loaded during the giant steps of the one before
   // it: its header and the thread's first two row ids with their k and slots.

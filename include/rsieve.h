@@ -109,16 +109,20 @@ typedef struct {
   uint32_t x_range;      /* floor(nmax/Q) - floor(nmin/Q) + 1 */
   uint32_t baby_steps;   /* m */
   uint32_t giant_steps;  /* T (per row) */
-  uint32_t table_slots;  /* shared-memory table size the plan was priced with, 16-bit slots per prime */
-  uint32_t primes_per_launch;
+  uint32_t table_slots;  /* table size the planner priced, in 16-bit slots per prime; the kernels keep a
+                            filter instead, of the bytes that the shared memory leaves them */
+  uint32_t primes_per_launch; /* at most (from -b/-t or mem_limit); a call's buffers may be smaller */
   double work_per_prime; /* algorithmic montmuls per prime: 2*sqrt(E[R]*X) */
   uint64_t upload_bytes; /* host->device bytes copied when the job was created */
   uint32_t warps_per_prime; /* 1: a warp per prime; 16: a CTA per prime (large tables) */
-  uint32_t row_form;     /* giant-step rows: 0 some k*b^r is 2^32 or more (per-prime residues, or the
-                            integer k with a multiplier per residue class), 1 the integers
-                            k*b^r (all < 2^32) in the records, 2 k*b^r read by row id,
-                            3 k*b^r of the rows of a per-prime active-row mask (at most
-                            64 rows, a warp per prime) */
+  uint32_t row_form;     /* giant-step rows of a warp per prime: 0 some k*b^r is 2^32 or more
+                            (per-prime residues, or the integer k with a multiplier per
+                            residue class), 1 the integers k*b^r (all < 2^32) in the
+                            records, 2 k*b^r read by row id, 3 k*b^r of the rows of a
+                            per-prime active-row mask (at most 64 rows).  A CTA per prime
+                            (16) always keeps row ids and the integer k; its 0 to 2 say
+                            only whether all k*b^r are below 2^32 and what the plan was
+                            priced with */
   uint32_t parts;        /* (base, sign) groups of the input, each planned and searched as
                             its own part over the same primes; the plan fields above
                             describe the first part, num_k and num_candidates count all */
