@@ -21,6 +21,7 @@ constexpr uint32_t kEmpty = 0xffffffffu;
 constexpr int kWarpsPerBlock = 4;   // BSGS kernels: one prime per warp
 constexpr int kSieveOdds = 1 << 15; // odd numbers per sieve segment (4 KB of bits)
 constexpr int kSieveThreads = 256;
+constexpr uint32_t kSms = 152;      // GB300's SMs
 constexpr uint32_t kNoTable = 0xffffffffu;  // no quadratic-character table for this k
 
 // Per-prime records, written by the setup kernel and read by the BSGS kernel:

@@ -282,7 +282,7 @@ cudaError_t launch_sieve(uint64_t lo, uint64_t hi, const uint32_t *sp, const uin
     // 81 at 92 segments.  With more of them each block's walk over the small primes
     // counts: 83 -> 92 us at 122 segments, 105 -> 155 at 290.
     constexpr int kShort = kSieveOdds / 4;
-    constexpr uint32_t kShortMax = 2 * 152 / 4;  // GB300's SMs
+    constexpr uint32_t kShortMax = 2 * kSms / 4;
     if (blocks <= kShortMax)
       sieve_small_kernel<false, kShort><<<(unsigned)((nodd + kShort - 1) / kShort), kSieveThreads, 0, st>>>(
           lo, hi, sp, sp_rcp, nsmall, gbits, out, count, cap, nullptr);
@@ -2088,7 +2088,7 @@ __global__ void verify_kernel(JobDev J, HitBufs hb) {
 }
 
 cudaError_t launch_verify(const JobDev &job, const HitBufs &hb, cudaStream_t st) {
-  const unsigned blocks = std::min(608u, (hb.cap + 255) / 256);
+  const unsigned blocks = std::min(4 * kSms, (hb.cap + 255) / 256);  // (grid-stride)
   verify_kernel<<<blocks, 256, 0, st>>>(job, hb);
   return cudaGetLastError();
 }

@@ -59,3 +59,19 @@ def test_few_rows_many_steps(rs, oracle_mod, nk, Q, sign, width, hash_m, T):
         assert info["rows"] <= 12 and st["exact_primes"] <= st["primes"] // 50
         found += n
     assert found > 100
+
+
+def test_few_rows_batched(rs):
+    """The same rows in one batched launch: each item's factors are those of its own run."""
+    specs = [(1, 3, 200000, 6), (3, 2, 40000, 6), (1, 9, 300000, 7), (3, 3, 20000, 0)]
+    jobs = [rs.Job(base=745, sign=-1, ks=[9000001 + 2 * i for i in range(nk)], datless=1, Q=Q, hash_m=hash_m,
+                   nlists=[np.array([1000, 1000 + width - 1], dtype=np.uint32)] * nk, mem_limit=1 << 28)
+            for nk, Q, width, hash_m in specs]
+    for p0, window in ((10**6, 3 * 10**4), (2**33 + 1, 2 * 10**6)):
+        want = [_set(j.sieve(p0, p0 + window)[0]) for j in jobs]
+        with rs.Batch() as batch:
+            items = [batch.add(j, p0, p0 + window) for j in jobs]
+            batch.run()
+            assert [_set(batch.result(i)[0]) for i in items] == want and all(map(len, want[:1]))
+    for j in jobs:
+        j.close()
