@@ -1062,15 +1062,17 @@ __device__ __forceinline__ void giant_test(const Filter<2> &F, const void *src, 
     hA |= ha << sh;
     hB |= hb << sh;
   }
-  uint32_t ha = 0, hb = 0;
-  if (g + 2 <= g1) {
-    pass(g, 1, two, ha, hb);
-    if (g + 2 < g1) pass(g + 2, 2, std::false_type{}, ha, hb);
-  } else if (g < g1) {
-    pass(g, 1, std::false_type{}, ha, hb);
+  if (g < g1) {  // (after 64 passes sh is 32, no shift count of a 32-bit word)
+    uint32_t ha = 0, hb = 0;
+    if (g + 2 <= g1) {
+      pass(g, 1, two, ha, hb);
+      if (g + 2 < g1) pass(g + 2, 2, std::false_type{}, ha, hb);
+    } else {
+      pass(g, 1, std::false_type{}, ha, hb);
+    }
+    hA |= ha << sh;
+    hB |= hb << sh;
   }
-  hA |= __funnelshift_lc(0, ha, sh);  // (sh is 32 after 64 passes, more than << may take)
-  hB |= __funnelshift_lc(0, hb, sh);
 }
 
 // The work of one prime in the warp-per-prime layout, the whole warp together:
