@@ -416,6 +416,37 @@ static uint64_t cta_fixed(uint32_t m, uint32_t row_slots, uint32_t Q, double pro
   return align_up(2ull * m + 2ull * row_slots + 20ull * cta_match_cap(probes) + 4ull * Q + 16, 16);
 }
 
+// How the 16 warps of the CTA kernel share the giant steps of residues with rows for
+// few of them (four rows a warp): warps a residue, residues side by side, and warps
+// for a residue's pairs of steps.  `work`: passes over four rows of the longest warp, a
+// pair's multipliers counted as half of one; the split with the least of it is taken,
+// where it saves kSplitPays against all warps at each residue, for the split
+// kernel's own start takes about 2 ns a prime (32 k, Q = 2, T = 128, which saves one, 23.6
+// against 21.9; 24 k, Q = 8, T = 32, which saves three, 25.6 against 27.0).
+struct CtaSplit {
+  uint32_t rows = 0, res = 0, steps = 0;  // rows 0: all warps at each residue
+  double work = 0.0;
+};
+static CtaSplit cta_split(uint32_t nrows, uint32_t Q, uint64_t T) {
+  constexpr double kSplitPays = 2.5;
+  auto pow2 = [](uint32_t x) { return 1u << ilog2_ceil(std::max(1u, x)); };
+  const double active = (double)nrows / Q * ((Q & 1) ? 0.75 : 0.5);
+  const uint32_t passes = std::max(1u, (uint32_t)std::ceil(active / 4.0)), pairs = (uint32_t)std::max<uint64_t>(1, T / 64);
+  CtaSplit best;
+  best.work = Q * pairs * (0.5 + (double)passes / kCtaWarps);
+  const double most = best.work - kSplitPays;
+  if (passes > kCtaWarps / 2) return best;
+  for (uint32_t rows = 1; rows < (uint32_t)kCtaWarps && rows <= pow2(passes); rows *= 2) {
+    CtaSplit s;
+    s.rows = rows;
+    s.res = std::min(kCtaWarps / rows, pow2(Q));
+    s.steps = std::min(kCtaWarps / (rows * s.res), pairs);
+    s.work = std::ceil((double)Q / s.res) * (0.5 * pairs + std::ceil((double)passes / rows) * std::ceil((double)pairs / s.steps));
+    if (s.work < std::min(most, best.work)) best = s;
+  }
+  return best;
+}
+
 // Plan a job.  With `force`, take exactly that choice (it must be feasible);
 // with `ranked`, also return every feasible choice, cheapest first.
 static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_bitmap = true,
@@ -457,7 +488,8 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
   // Q = 2, T = 1024; four k over 8e5: Q = 2, T = 256 4.0 against 5.9 for Q = 8, T = 64.
   const bool few = s.k.size() <= 16;
   constexpr double kStepCost = 2.0, kShoupStep = 1.4, kResidueRow = 2.0, kResidueCost = 2.2;
-  constexpr double kCtaFew = 2.5;  // 14 k over 1.8e6 exponents: a CTA per prime takes 37 ns, a warp 15
+  // A unit of theirs is 2.5 to 3.7e-2 ns; a CTA plan of few k is priced by its ns (cta_ns).
+  constexpr double kUnitFew = 0.028;
   // Setup-kernel cost per (k, n mod Q) row, in the same units.
   constexpr double kRowCost = 0.18;
   // A step of the CTA kernel costs more than one of the warp kernel (block-wide
@@ -477,11 +509,17 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
     double cost, ns;
   };
   std::vector<CtaPlan> cta_plans;
-  auto cta_ns = [](uint32_t m, double ER, int rows, uint32_t Q, uint64_t T) {
+  auto cta_ns = [few](uint32_t m, double ER, int rows, uint32_t Q, uint64_t T) {
     const uint32_t slots = (uint32_t)rows + 4 * Q + 8;
     const bool two = cta_pair(m, cta_fixed(m, slots, Q, ER * (double)T), slots, ER * (double)T);
     const double giants = ER * (double)T / 32.0;
-    return (two ? 12.0 + 1.3 * m / 1024.0 + 0.0255 * giants : 10.7 + 2.26 * m / 1024.0 + 0.028 * giants) + 0.01 * rows;
+    // few rows a residue (1 to 16 k over 4e6 to 2e8 exponents, to about 15%): 12 k, Q = 8, T =
+    // 128, m = 8192 42.2 ns (42.6 by this); two k, Q = 48, T = 128, m = 10240 53.8 (52.9)
+    const CtaSplit sp = cta_split((uint32_t)rows, Q, T);
+    if (few)
+      return sp.work + (two ? 17.0 + 2.2 * m / 1024.0 + 0.0255 * giants : 10.0 + 2.7 * m / 1024.0 + 0.028 * giants);
+    return (two ? 12.0 + 1.3 * m / 1024.0 + 0.0255 * giants : 10.7 + 2.26 * m / 1024.0 + 0.028 * giants) + 0.01 * rows +
+           (sp.rows ? sp.work + 2.0 : 0.0);
   };
   double best = 1e300;
   auto consider = [&](uint32_t Q, int rows, uint32_t X, double ER, bool cta, uint64_t T, uint64_t m, uint32_t nb,
@@ -583,7 +621,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
           if (m <= mcap && m < 65536 && m * T >= X && slog <= 17 && smem <= kCtaSmemMax && fp <= 16.0) {
             const double cost = ((double)m / 32.0 + kGiantWeight * kCtaWarps * std::ceil(ER / kCtaWarps) * spl +
                                  nb * 8 / 1024.0 + 3.7 + kRowCost * rows + std::min(1.0, fp) * (double)m / 32.0) *
-                                std::sqrt(kFullWarps / kCtaWarps) * kCtaStepCost * (few ? kCtaFew : 1.0);
+                                std::sqrt(kFullWarps / kCtaWarps) * kCtaStepCost;
             cta_plans.push_back({Q, rows, X, ER, T, m, nbk, slog, cost, cta_ns((uint32_t)m, ER, rows, Q, T)});
           }
         }
@@ -596,7 +634,7 @@ static int make_plan(const Seqs &s, const rs_options &opt, Plan &pl, bool with_b
     cta_min = std::min(cta_min, c.ns);
   }
   for (const CtaPlan &c : cta_plans)
-    consider(c.Q, c.rows, c.X, c.ER, true, c.T, c.m, c.nb, c.slog, cta_cost * c.ns / cta_min);
+    consider(c.Q, c.rows, c.X, c.ER, true, c.T, c.m, c.nb, c.slog, few ? c.ns / kUnitFew : cta_cost * c.ns / cta_min);
   if (ranked)
     std::sort(ranked->begin(), ranked->end(), [](const PlanChoice &a, const PlanChoice &b) { return a.cost < b.cost; });
   if (pl.Q == 0) return fail(RS_ERR_INVALID, "no feasible plan (n range too wide for the -m limit)");
@@ -1166,7 +1204,7 @@ static int upload_part(rs_job *j, Part &pt) {
   // over 8, go through their steps one by one.  Of the time with a multiplier per
   // step that is 0.68 for 4 rows at T = 1024, 0.93 for 6 rows at T = 128 and 0.79 at T =
   // 512, 0.91 for 12 rows there; 9 rows at T = 128 took 1.09, 18 rows at T = 256 1.09.
-  d.few_rows = !pl.cta && !d.int_rows && (pl.T >= 256 ? pl.nrows <= 12 : pl.T >= 128 && pl.nrows <= 6) ? 1u : 0u;
+  d.split = !pl.cta && !d.int_rows && (pl.T >= 256 ? pl.nrows <= 12 : pl.T >= 128 && pl.nrows <= 6) ? 1u : 0u;
   d.el_v = pl.cta ? kElWoff + 2 * kCtaWarps + 2 : d.by_res ? kElV + 2 : kElV;
   if (d.row_mask) {
     d.el_row = d.el_v;
@@ -1204,6 +1242,8 @@ static int upload_part(rs_job *j, Part &pt) {
     if (d.fwords < 256) return fail(RS_ERR_INVALID, "a CTA plan's rows leave no shared memory for its filter");
     d.fshift = filter_shift(d.fwords);
     d.warp_smem = (uint32_t)(4ull * d.fwords + used);
+    const CtaSplit sp = cta_split(pl.nrows, pl.Q, pl.T);
+    d.split = sp.rows | sp.res << 8 | sp.steps << 16;
     uint64_t kmax = 0;
     for (uint32_t k : s.k) kmax = std::max<uint64_t>(kmax, k);
     d.edge_lim = (uint32_t)std::min<uint64_t>(0xffffffffu, ((kmax + 1) >> (d.fshift - 10)) + 1);

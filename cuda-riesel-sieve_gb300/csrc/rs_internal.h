@@ -71,7 +71,7 @@ constexpr uint32_t kElV = 12;      // V in the warp-per-prime layout (W == 1)
 constexpr uint32_t kStepShoup = 0, kStepSmall = 1, kStepHigh = 2;  // ChunkBufs::small_step
 // Giant-step start values of the fast kernels (template argument): V in
 // Montgomery form, the integers k*b^r in V, k*b^r read by row id, k*b^r of the
-// rows of an active-row mask, the integers k by residue, or V of few rows (JobDev::few_rows).
+// rows of an active-row mask, the integers k by residue, or V of few rows (JobDev::split).
 constexpr int kRowsV = 0, kRowsIntV = 1, kRowsIntId = 2, kRowsMask = 3, kRowsRes = 4, kRowsFew = 5;
 constexpr uint32_t kResMax = 8;    // residues (Q) of a by_res job at most
 constexpr uint32_t kMaskRows = 64;  // rows a row_mask record can describe
@@ -164,9 +164,13 @@ struct JobDev {
   uint32_t b_odd, b_e2;
   uint64_t b_rcp;
   uint32_t b_jac;
-  uint32_t few_rows;     // V rows, so few for their steps that the kernel advances their values and not a
-                         // multiplier (here at the end: among the constants above it moves what the CTA
-                         // kernel loads together, 1.3% of the 1000-k job)
+  // Warp layout: not 0 for V rows so few for their steps that the kernel advances their
+  // values and not a multiplier.  CTA layout: not 0 where residues have rows for few of
+  // the 16 warps; then warps that share a residue's rows | residues side by side << 8 | warps
+  // that share a residue's steps << 16, powers of two, their product up to 16.  (Last, for a
+  // field among the constants above changes what the CTA kernel loads together: 199.7 ms for 197.0
+  // of the 1000-k job.)
+  uint32_t split;
 };
 
 // Kernel variant of a job's warp layout.
@@ -175,7 +179,7 @@ inline int row_mode(const JobDev &d) {
          : d.row_mask     ? kRowsMask
          : d.row_ids_only ? kRowsIntId
          : d.int_rows     ? kRowsIntV
-         : d.few_rows     ? kRowsFew
+         : d.split        ? kRowsFew
                           : kRowsV;
 }
 

@@ -1556,17 +1556,17 @@ int bsgs_smem_bytes(const JobDev &job) {
   return job.cta_warps > 1 ? (int)job.warp_smem : kWarpsPerBlock * (int)job.warp_smem;
 }
 
-// Giant steps of the CTA kernel for one residue r: warp w takes groups w, w + W,
-// ... of four of the n active rows (ks: their k, or rid and the job's row_k),
+// Giant steps of the CTA kernel for one residue r: warp w of W takes groups w, w +
+// W, ... of four of the n active rows (ks: their k, or rid and the job's row_k),
 // multiplied by the lane's Z*b^r for one or two steps u (G0, G1).  Suspects are
 // listed as they are found.
-template <bool KS, bool TWO>
+template <bool KS, bool TWO, bool SPLIT>
 __device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint32_t *keys, uint32_t *count, uint32_t cap,
                                            const uint32_t *ks, const uint16_t *rid, const uint32_t *__restrict__ row_k,
-                                           uint32_t n, uint32_t warp, const GiantMul &G0, const GiantMul &G1,
-                                           uint32_t s0) {
+                                           uint32_t n, uint32_t warp, uint32_t warps, const GiantMul &G0,
+                                           const GiantMul &G1, uint32_t s0) {
 #pragma unroll 1
-  for (uint32_t g = 4 * warp; g < n; g += 4 * kCtaWarps) {
+  for (uint32_t g = 4 * warp; g < n; g += 4 * warps) {
     uint32_t c[4];
     if (KS) {
       const uint4 v = *reinterpret_cast<const uint4 *>(ks + g);
@@ -1576,11 +1576,16 @@ __device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint
       for (uint32_t i = 0; i < 4; i++) c[i] = __ldg(row_k + rid[min(g + i, n - 1)]);
     }
     uint32_t hit = 0;
+    auto rows = [&](auto count) {
 #pragma unroll
-    for (uint32_t i = 0; i < 4; i++) {
-      if (F.test(giant_key<kRowsIntV>(c[i], G0, 0, 0, 0))) hit |= 1u << i;
-      if (TWO && F.test(giant_key<kRowsIntV>(c[i], G1, 0, 0, 0))) hit |= 16u << i;
-    }
+      for (uint32_t i = 0; i < decltype(count)::value; i++) {
+        if (F.test(giant_key<kRowsIntV>(c[i], G0, 0, 0, 0))) hit |= 1u << i;
+        if (TWO && F.test(giant_key<kRowsIntV>(c[i], G1, 0, 0, 0))) hit |= 16u << i;
+      }
+    };
+    if (SPLIT && n - g == 1) rows(std::integral_constant<uint32_t, 1>{});
+    else if (SPLIT && n - g == 2) rows(std::integral_constant<uint32_t, 2>{});
+    else rows(std::integral_constant<uint32_t, 4>{});
     if (hit) {  // rare
 #pragma unroll 1
       for (uint32_t i = 0; i < 8; i++) {
@@ -1621,7 +1626,11 @@ __device__ __forceinline__ void cta_giants(const Filter<3> &F, Match *list, uint
 // clearing and row lists 17 (25 before the next prime's loads were moved
 // under the giant steps).  With shared memory for it two CTAs share an SM
 // (CTAS, at 64 registers a thread): 467 k at m = 7168, T = 64 take 47 ns against 52.5.
-template <bool KS, int CTAS>
+// SPLIT: residues with rows for few of the 16 warps (JobDev::split) are gone through
+// side by side, and a residue's steps by several warps in turn.  With all warps at one
+// residue most have no row and form its multipliers only: two k over 2e8 exponents (Q =
+// 48, T = 256, m = 16384) took 344 ns per prime, so split 92; twelve over 6e7 224, 92.
+template <bool KS, int CTAS, bool SPLIT>
 __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J, ChunkBufs cb, HitBufs hb) {
   extern __shared__ uint4 smem4[];
   constexpr uint32_t T = 32 * kCtaWarps;
@@ -1718,29 +1727,72 @@ __global__ void __launch_bounds__(32 * kCtaWarps, CTAS) bsgs_cta_kernel(JobDev J
       const uint64_t Gw = rec[kElGw], Gq = rec[kElGq];
       uint64_t Er = rec[J.el_tab + 32 + lane];
       if (i + gridDim.x < n) fetch(i + gridDim.x);
+      if constexpr (SPLIT) {
+        // The warp's place (slot) goes through residues slots apart, one of the pair r0,
+        // r0 + 1 and the other by turns: for even Q the active rows of few k are of one parity.
+        const uint32_t ws = J.split & 255, slots = J.split >> 8 & 255, wsteps = J.split >> 16;
+        const uint32_t slot = warp / (ws * wsteps), wr = warp % ws, wu = warp / ws % wsteps;
+        const uint32_t r0 = slots > 1 ? slot & ~1u : slot;
+        uint64_t pw = bw, pq = bq;  // b^slots and its Shoup constant, by squarings; b^r0 into Er
 #pragma unroll 1
-      for (uint32_t r = 0; r < J.Q; r++) {
-        const uint32_t nr = nrow[r];
-        if (nr) {
-          const uint32_t at = __ldg(J.row_base + r);
-          const uint32_t w = (warp + 5 * r) % kCtaWarps;  // uneven shares of several residues fall on different warps
-          uint64_t E = Er;
+        for (uint32_t x = r0, y = slots; y > 1; x >>= 1, y >>= 1) {
+          if (x & 1) Er = shoup_mul(Er, pw, pq, p);
+          const uint64_t sq = shoup_mul(pq * np, pw, pq, p);  // (pq * np is pw in Montgomery form)
+          pw = shoup_mul(pw, pw, pq, p);
+          pq = shoup_const(sq, pinv);
+        }
 #pragma unroll 1
-          for (uint32_t u = 0; u < spl; u += 2) {
-            GiantMul G0, G1;
-            G0.set(E, p, pinv);
-            G1 = G0;
-            if (u + 1 < spl) {
-              E = shoup_mul(E, Gw, Gq, p);
-              G1.set(E, p, pinv);
-              cta_giants<KS, true>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
-              if (u + 2 < spl) E = shoup_mul(E, Gw, Gq, p);
-            } else {
-              cta_giants<KS, false>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, w, G0, G1, lane + 1 + 32 * u);
+        for (uint32_t rb = r0, turn = slot; slot < slots && rb < J.Q; rb += slots, turn++) {
+          const uint32_t r = slots > 1 ? rb + (turn & 1) : rb;
+          const uint32_t nr = r < J.Q ? nrow[r] : 0;
+          if (nr) {
+            const uint32_t at = __ldg(J.row_base + r);
+            uint64_t E = r != rb ? shoup_mul(Er, bw, bq, p) : Er;
+#pragma unroll 1
+            for (uint32_t u = 0; u < spl; u += 2) {
+              const bool mine = (u >> 1) % wsteps == wu;
+              GiantMul G0, G1;
+              if (mine) G0.set(E, p, pinv);
+              G1 = G0;
+              if (u + 1 < spl) {
+                E = shoup_mul(E, Gw, Gq, p);
+                if (mine) {
+                  G1.set(E, p, pinv);
+                  cta_giants<KS, true, SPLIT>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, wr, ws, G0, G1, lane + 1 + 32 * u);
+                }
+                if (u + 2 < spl) E = shoup_mul(E, Gw, Gq, p);
+              } else if (mine) {
+                cta_giants<KS, false, SPLIT>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, wr, ws, G0, G1, lane + 1 + 32 * u);
+              }
             }
           }
+          Er = shoup_mul(Er, pw, pq, p);
         }
-        if (r + 1 < J.Q) Er = shoup_mul(Er, bw, bq, p);
+      } else {
+#pragma unroll 1
+        for (uint32_t r = 0; r < J.Q; r++) {
+          const uint32_t nr = nrow[r];
+          if (nr) {
+            const uint32_t at = __ldg(J.row_base + r);
+            const uint32_t w = (warp + 5 * r) % kCtaWarps;  // uneven shares of several residues fall on different warps
+            uint64_t E = Er;
+#pragma unroll 1
+            for (uint32_t u = 0; u < spl; u += 2) {
+              GiantMul G0, G1;
+              G0.set(E, p, pinv);
+              G1 = G0;
+              if (u + 1 < spl) {
+                E = shoup_mul(E, Gw, Gq, p);
+                G1.set(E, p, pinv);
+                cta_giants<KS, true, SPLIT>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, w, kCtaWarps, G0, G1, lane + 1 + 32 * u);
+                if (u + 2 < spl) E = shoup_mul(E, Gw, Gq, p);
+              } else {
+                cta_giants<KS, false, SPLIT>(F, list, keys, count, J.match_cap, ks + at, rid + at, J.row_k, nr, w, kCtaWarps, G0, G1, lane + 1 + 32 * u);
+              }
+            }
+          }
+          if (r + 1 < J.Q) Er = shoup_mul(Er, bw, bq, p);
+        }
       }
     }
     __syncthreads();
@@ -1990,8 +2042,13 @@ static cudaError_t configure_one(const void *fn, int smem, int threads, int devi
 static int bsgs_threads(const JobDev &job) { return job.cta_warps > 1 ? 32 * kCtaWarps : 32 * kWarpsPerBlock; }
 
 static BsgsFn bsgs_cta_fn(const JobDev &job) {
-  if (job.cta_pair) return bsgs_cta_kernel<true, 2>;  // (cta_pair leaves room for the rows' k)
-  return job.ctab_smem ? bsgs_cta_kernel<true, 1> : bsgs_cta_kernel<false, 1>;
+  // (cta_pair leaves room for the rows' k)
+  if (job.split) {
+    if (job.cta_pair) return bsgs_cta_kernel<true, 2, true>;
+    return job.ctab_smem ? bsgs_cta_kernel<true, 1, true> : bsgs_cta_kernel<false, 1, true>;
+  }
+  if (job.cta_pair) return bsgs_cta_kernel<true, 2, false>;
+  return job.ctab_smem ? bsgs_cta_kernel<true, 1, false> : bsgs_cta_kernel<false, 1, false>;
 }
 
 static const void *bsgs_fast_fn(const JobDev &job) {
