@@ -1062,7 +1062,9 @@ __device__ __forceinline__ void giant_test(const Filter<2> &F, const void *src, 
     hA |= ha << sh;
     hB |= hb << sh;
   }
-  if (g < g1) {  // (after 64 passes sh is 32, no shift count of a 32-bit word)
+  // (After 64 passes sh is 32, no shift count of a 32-bit word.  By a clamped shift in place of the
+  // guard one k takes 88.1 ms for 88.6, but 131 k 69.3 for 68.3, 32 k at T = 32 21.9 ns for 20.7.)
+  if (g < g1) {
     uint32_t ha = 0, hb = 0;
     if (g + 2 <= g1) {
       pass(g, 1, two, ha, hb);
